@@ -1,14 +1,16 @@
 // Plain tiled matrix product on the CUDA cores, any sizes:  C[M,N] (op)= A[M,K] * W[N,K]^T.
 //
-// This is the product of the true 32-bit path (float operands, float FMA, no tensor cores and
-// no reduced-precision mode), and the any-shape fallback of the bfloat16 path (bf16 operands
-// widened exactly, float accumulation).  The reference's scalar product has the same contract:
+// The entry point of the any-shape products: float operands (the true 32-bit path; float FMA, no tensor cores and no
+// reduced-precision mode) go to gemm_f32.cu, the kernel here is the fallback of the bfloat16 path (bf16 operands widened
+// exactly, float accumulation).  The reference's scalar product has the same contract:
 // C[m,n] = sum_k A[m,k] * W[n,k] with f32 accumulation (backend_bf16/src/kernels.rs:95-143).
 //
 // 64x64 output tile, 16-wide k slab, 256 threads, 4x4 outputs per thread.  Edges are guarded
 // element by element, so M, N and K need not be multiples of anything.
 #include "api.h"
 #include "common.cuh"
+
+int hb_gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K, int epi, void* stream);      // gemm_f32.cu
 
 #define TM 64
 #define TN 64
@@ -101,6 +103,7 @@ extern "C" int hb_gemm_simt(int dtype, const void* A, int lda, const void* W, in
                             int M, int N, int K, int epi, void* stream) {
   HB_REQUIRE(M > 0 && N > 0 && K > 0, "gemm: sizes must be positive (M=%d N=%d K=%d)", M, N, K);
   HB_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm: leading dimensions too small");
-  return dtype == HB_F32 ? gemm_simt_launch<float>(A, lda, W, ldw, C, ldc, M, N, K, epi, stream)
-                         : gemm_simt_launch<bf16>(A, lda, W, ldw, C, ldc, M, N, K, epi, stream);
+  HB_REQUIRE(epi == HB_EPI_STORE || epi == HB_EPI_STORE_F32 || epi == HB_EPI_RESIDUAL, "gemm: unknown epilogue %d", epi);
+  if (dtype == HB_F32) return hb_gemm_f32((const float*)A, lda, (const float*)W, ldw, (float*)C, ldc, M, N, K, epi, stream);
+  return gemm_simt_launch<bf16>(A, lda, W, ldw, C, ldc, M, N, K, epi, stream);
 }
