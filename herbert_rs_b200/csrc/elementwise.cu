@@ -41,11 +41,50 @@ __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict_
   }
 }
 
+// The same, 16 bytes of the table a thread: where hidden allows it and all rows start on 16 bytes.
+template <typename T>
+__global__ void __launch_bounds__(1024)
+embed_row_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ out, int copies, int hidden, int vocab, float scale,
+                 const T* __restrict__ pos_table, const int* __restrict__ positions, int n_positions) {
+  constexpr int E = 16 / (int)sizeof(T);
+  pdl_wait();
+  pdl_launch();
+  const int t = blockIdx.x;
+  const int id = ids[t], p = pos_table ? positions[t] : -1;
+  const bool known = id >= 0 && id < vocab, placed = known && p >= 0 && p < n_positions;
+  float* o = out + (size_t)t * copies * hidden;
+  for (int i = threadIdx.x * E; i < hidden; i += blockDim.x * E) {
+    uint4 a = make_uint4(0, 0, 0, 0), b = a;
+    if (known) a = *reinterpret_cast<const uint4*>(table + (size_t)id * hidden + i);
+    if (placed) b = *reinterpret_cast<const uint4*>(pos_table + (size_t)p * hidden + i);
+    const T* av = reinterpret_cast<const T*>(&a);
+    const T* bv = reinterpret_cast<const T*>(&b);
+    float v[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+      v[j] = known ? to_f32(av[j]) * scale : 0.0f;
+      if (placed) v[j] += to_f32(bv[j]);
+    }
+    for (int c = 0; c < copies; ++c)
+#pragma unroll
+      for (int j = 0; j < E; j += 4)
+        *reinterpret_cast<float4*>(o + (size_t)c * hidden + i + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  }
+}
+
 template <typename T>
 static int embed_launch(const void* table, const int* ids, float* out, int copies, int n_tokens, int hidden,
                         int vocab, float scale, const void* pos_table, const int* positions, int n_positions, void* stream) {
   HB_REQUIRE(n_tokens > 0 && hidden > 0 && vocab > 0 && copies > 0, "embed: sizes must be positive");
   HB_REQUIRE(pos_table == nullptr || (positions != nullptr && n_positions > 0), "embed: a position table needs positions");
+  constexpr int E = 16 / (int)sizeof(T);
+  if (hidden % E == 0 && (((uintptr_t)table | (uintptr_t)out | (uintptr_t)pos_table) & 15) == 0) {
+    const int need = ceil_div(hidden / E, 32) * 32;
+    hb_launch(embed_row_kernel<T>, dim3(n_tokens), dim3(need < 1024 ? need : 1024), 0, (cudaStream_t)stream, (const T*)table, ids, out, copies, hidden,
+              vocab, scale, (const T*)pos_table, positions, n_positions);
+    HB_CHECK_LAUNCH("embed");
+    return 0;
+  }
   int threads = hidden >= 1024 ? 256 : 128;
   hb_launch(embed_kernel<T>, dim3(n_tokens), dim3(threads), 0, (cudaStream_t)stream, (const T*)table, ids, out, copies, hidden, vocab, scale,
             (const T*)pos_table, positions, n_positions);

@@ -12,6 +12,7 @@
 //                            the token's id chooses from a table (the per-layer part of a second embedding)
 #include "api.h"
 #include "common.cuh"
+#include "row_norm.cuh"
 
 struct GatedJoinArgs {
   const float* y; int ldy;
@@ -61,11 +62,51 @@ __global__ void __launch_bounds__(256) gated_norm_residual_kernel(GatedJoinArgs 
   for (int i = threadIdx.x; i < D; i += blockDim.x) h[i] = from_f32<T>((row[i] * inv2) * a.w2[i]);
 }
 
+// The same with the row in registers (row_norm.cuh): where D is a multiple of 128 and all rows start on 16 bytes.
+template <typename T, int V>
+__global__ void __launch_bounds__(RN_MAX_THREADS) gated_norm_residual_row_kernel(GatedJoinArgs a) {
+  __shared__ float part[V * 16], part2[V * 16];
+  pdl_wait();
+  pdl_launch();
+  const int t = blockIdx.x, D = a.D;
+  RowRegs<V> v, x, w, z, zb, w2;
+  float* xr = a.x + (size_t)t * D;
+  rn_load(v, a.y + (size_t)t * a.ldy, D);
+  if (a.z) rn_load(z, a.z + (size_t)t * a.ldz, D);
+  if (a.zb) rn_load(zb, a.zb, D);
+  rn_load(x, xr, D);
+  rn_load(w, a.w, D);
+  if (a.w2) rn_load(w2, a.w2, D);
+  if (a.z) rn_each(v, [&](float f, int j, int c) { return f * (1.0f / (1.0f + expf(-(rn_at(z.v[j], c) + (a.zb ? rn_at(zb.v[j], c) : 0.0f))))); });
+  rn_parts(v, part, D, [](float f) { return f * f; });
+  const float inv = 1.0f / sqrtf(rn_sum(part, 0, D >> 7) / (float)D + a.eps);
+  rn_each(x, [&](float f, int j, int c) { return f + (rn_at(v.v[j], c) * inv) * rn_at(w.v[j], c); });
+  rn_store(xr, x, D);
+  if (a.h == nullptr) return;
+  T* h = (T*)a.h + (size_t)t * D;
+  if (a.w2 != nullptr) {
+    rn_parts(x, part2, D, [](float f) { return f * f; });
+    const float inv2 = 1.0f / sqrtf(rn_sum(part2, 0, D >> 7) / (float)D + a.eps2);
+    rn_each(x, [&](float f, int j, int c) { return (f * inv2) * rn_at(w2.v[j], c); });
+  }
+  rn_store(h, x, D);
+}
+
 extern "C" int hb_gated_norm_residual(int dtype, const float* y, int ldy, const float* z, int ldz, const float* zb,
                                       const float* w, float eps, float* x, const float* w2, float eps2, void* h,
                                       int n_rows, int D, void* stream) {
   HB_REQUIRE(n_rows > 0 && D > 0, "gated_norm_residual: sizes must be positive");
   HB_REQUIRE(z != nullptr || zb == nullptr, "gated_norm_residual: a gate's bias needs the gate");
+  if (rn_ok(D, (uintptr_t)y | (uintptr_t)ldy * 4 | (uintptr_t)z | (uintptr_t)(z ? ldz : 0) * 4 | (uintptr_t)zb | (uintptr_t)w | (uintptr_t)x | (uintptr_t)w2 | (uintptr_t)h)) {
+    const GatedJoinArgs g{y, ldy, z, ldz, zb, w, eps, x, w2, eps2, h, D};
+#define GJ_GO(V)                                                                                                                          \
+  if (dtype == HB_F32) hb_launch(gated_norm_residual_row_kernel<float, V>, dim3(n_rows), dim3(rn_threads(D)), 0, (cudaStream_t)stream, g); \
+  else hb_launch(gated_norm_residual_row_kernel<bf16, V>, dim3(n_rows), dim3(rn_threads(D)), 0, (cudaStream_t)stream, g)
+    RN_GO(D, GJ_GO);
+#undef GJ_GO
+    HB_CHECK_LAUNCH("gated_norm_residual");
+    return 0;
+  }
   const size_t smem = (size_t)D * sizeof(float);
   HB_REQUIRE(smem <= 160 * 1024, "gated_norm_residual: rows of %d numbers do not fit a block's shared memory", D);
   GatedJoinArgs a{y, ldy, z, ldz, zb, w, eps, x, w2, eps2, h, D};

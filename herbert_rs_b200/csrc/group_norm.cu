@@ -11,6 +11,7 @@
 //   hb_tanh_cap                x = cap * tanh(x / cap)                            (a cap on the logits)
 #include "api.h"
 #include "common.cuh"
+#include "row_norm.cuh"
 
 // One CTA per row; warps share the groups: a group of n = dim / groups numbers is summed by the warps that
 // hold its elements through shared memory (one float per group).
@@ -55,6 +56,52 @@ group_rmsnorm_kernel(const float* __restrict__ y, int ldy, const float* __restri
   }
 }
 
+// The same with the row in registers (row_norm.cuh): where groups are multiples of 128 columns and all rows start on 16 bytes.
+template <typename T, bool RESIDUAL, int V>
+__global__ void __launch_bounds__(RN_MAX_THREADS)
+group_rmsnorm_row_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ z, int ldz, float a, float b,
+                         const float* __restrict__ bias, const float* __restrict__ w, float* __restrict__ x, T* __restrict__ out,
+                         const int* __restrict__ rows, int dim, int groups, float eps) {
+  __shared__ float part[V * 16];
+  pdl_wait();
+  pdl_launch();
+  const int r = blockIdx.x;
+  RowRegs<V> v, u, wv, xv;
+  rn_load(v, y + (size_t)(rows ? rows[r] : r) * ldy, dim);
+  if (z) rn_load(u, z + (size_t)r * ldz, dim);
+  rn_load(wv, w, dim);
+  if (RESIDUAL) rn_load(xv, x + (size_t)r * dim, dim);
+  if (z) rn_each(v, [&](float f, int j, int c) { return a * f + b * rn_at(u.v[j], c); });
+  if (bias) {
+    rn_load(u, bias, dim);
+    rn_each(v, [&](float f, int j, int c) { return f + rn_at(u.v[j], c); });
+  }
+  rn_parts(v, part, dim, [](float f) { return f * f; });
+  const int n = dim / groups;
+  float inv[V];                                      // four neighbouring columns lie in one group
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    const int i = (j * blockDim.x + threadIdx.x) * 4, g = i < dim ? i / n : 0;
+    inv[j] = 1.0f / sqrtf(rn_sum(part, g * (n >> 7), n >> 7) / (float)n + eps);
+  }
+  rn_each(v, [&](float f, int j, int c) { return (f * inv[j]) * rn_at(wv.v[j], c) + (RESIDUAL ? rn_at(xv.v[j], c) : 0.0f); });
+  if (RESIDUAL) rn_store(x + (size_t)r * dim, v, dim);
+  if (!RESIDUAL || out) rn_store(out + (size_t)r * dim, v, dim);
+}
+
+template <bool RESIDUAL>
+static bool group_rmsnorm_rows(int dtype, const float* y, int ldy, const float* z, int ldz, float a, float b, const float* bias, const float* w,
+                               float* x, void* out, const int* rows, int n_rows, int dim, int groups, float eps, cudaStream_t s) {
+  if (!rn_ok(dim / groups, 0) || !rn_ok(dim, (uintptr_t)y | (uintptr_t)ldy * 4 | (uintptr_t)z | (uintptr_t)(z ? ldz : 0) * 4 | (uintptr_t)bias | (uintptr_t)w | (uintptr_t)x | (uintptr_t)out))
+    return false;
+#define GN_GO(V)                                                                                                                                              \
+  if (dtype == HB_F32) hb_launch(group_rmsnorm_row_kernel<float, RESIDUAL, V>, dim3(n_rows), dim3(rn_threads(dim)), 0, s, y, ldy, z, ldz, a, b, bias, w, x, (float*)out, rows, dim, groups, eps); \
+  else hb_launch(group_rmsnorm_row_kernel<bf16, RESIDUAL, V>, dim3(n_rows), dim3(rn_threads(dim)), 0, s, y, ldy, z, ldz, a, b, bias, w, x, (bf16*)out, rows, dim, groups, eps)
+  RN_GO(dim, GN_GO);
+#undef GN_GO
+  return true;
+}
+
 static int gn_threads(int dim) { return dim >= 2048 ? 256 : dim >= 512 ? 128 : 64; }
 
 extern "C" int hb_group_rmsnorm(int dtype, const float* x, const float* w, void* out, const int* rows, int n_rows, int dim,
@@ -62,6 +109,10 @@ extern "C" int hb_group_rmsnorm(int dtype, const float* x, const float* w, void*
   HB_REQUIRE(n_rows > 0 && dim > 0, "group_rmsnorm: sizes must be positive");
   HB_REQUIRE(groups >= 1 && groups <= GN_MAX_GROUPS && dim % groups == 0,
              "group_rmsnorm: %d groups must divide the width %d and be at most %d", groups, dim, GN_MAX_GROUPS);
+  if (group_rmsnorm_rows<false>(dtype, x, dim, nullptr, 0, 1.0f, 0.0f, nullptr, w, nullptr, out, rows, n_rows, dim, groups, eps, (cudaStream_t)stream)) {
+    HB_CHECK_LAUNCH("group_rmsnorm");
+    return 0;
+  }
   if (dtype == HB_F32)
     hb_launch(group_rmsnorm_kernel<float, false>, dim3(n_rows), dim3(gn_threads(dim)), 0, (cudaStream_t)stream, x, dim,
               (const float*)nullptr, 0, 1.0f, 0.0f, (const float*)nullptr, w, (float*)nullptr, (float*)out, rows, dim, groups, eps);
@@ -78,6 +129,10 @@ extern "C" int hb_group_rmsnorm_residual(int dtype, const float* y, int ldy, con
   HB_REQUIRE(n_rows > 0 && dim > 0, "group_rmsnorm_residual: sizes must be positive");
   HB_REQUIRE(groups >= 1 && groups <= GN_MAX_GROUPS && dim % groups == 0,
              "group_rmsnorm_residual: %d groups must divide the width %d and be at most %d", groups, dim, GN_MAX_GROUPS);
+  if (group_rmsnorm_rows<true>(dtype, y, ldy, z, ldz, a, b, bias, w, x, h, nullptr, n_rows, dim, groups, eps, (cudaStream_t)stream)) {
+    HB_CHECK_LAUNCH("group_rmsnorm_residual");
+    return 0;
+  }
   if (dtype == HB_F32)
     hb_launch(group_rmsnorm_kernel<float, true>, dim3(n_rows), dim3(gn_threads(dim)), 0, (cudaStream_t)stream, y, ldy, z, ldz, a, b,
               bias, w, x, (float*)h, (const int*)nullptr, dim, groups, eps);
