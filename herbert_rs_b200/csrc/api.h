@@ -166,6 +166,11 @@ int hb_moe_route(int dtype, const void* h, int ld, const void* w_router, int* id
 int hb_moe_experts(int dtype, const void* h, int ld, const void* up, const void* down, const int* ids, const
     float* weights, void* mid, float* y, int ldy, int n_tokens, int D, int F, int top, int act, int gated,
     float act_limit, int weigh_input, int accumulate, void* stream);
+int hb_moe_experts_few_ok(const void* h, int ld, const void* up, const void* down, const void* mid, int n_tokens, int top,
+    int E, int D, int F, int gated);
+int hb_moe_experts_few_bf16(const void* h, int ld, const void* up, const void* down, const int* ids, const float* weights,
+    void* mid, float* y, int ldy, int n_tokens, int D, int E, int F, int top, int act, int gated, float act_limit,
+    int weigh_input, int accumulate, void* stream);
 long long hb_moe_grouped_scratch_ints(int n_tokens, int E, int top);
 int hb_moe_experts_tc_rows(int n_tokens, int E, int top);
 int hb_moe_experts_tc_bf16(const void* h, int ld, const void* up, const void* down, const int* ids, const

@@ -21,6 +21,7 @@
 // wants: every weight row of a chosen expert is read once per token that chose it.
 #include "api.h"
 #include "common.cuh"
+#include "moe_act.cuh"
 
 #define MOE_WARPS 4
 #define MOE_ROUTE_WARPS 8
@@ -62,27 +63,9 @@ __device__ __forceinline__ float warp_dot(const bf16* a, const bf16* w, int n, i
   return warp_sum(dot);
 }
 
-// One block per token: its warps share the experts' dot products, the first warp then takes the
-// scores, the groups and the choice.
-template <typename T>
-__global__ void __launch_bounds__(MOE_ROUTE_WARPS * 32)
-moe_route_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr, int* __restrict__ ids, float* __restrict__ wts,
-                 int n_tokens, int D, int E, int top, int renorm, int sigmoid, int groups, int keep, int group_top,
-                 float wscale) {
-  extern __shared__ float sh[];  // [E] scores, [groups] group scores
-  pdl_wait();
-  pdl_launch();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x;
-  float* s = sh;
-  float* gs = sh + E;
-  const T* hr = h + (size_t)t * ld;
-  for (int e = warp; e < E; e += MOE_ROUTE_WARPS) {
-    const float dot = warp_dot(hr, wr + (size_t)e * D, D, lane);
-    if (lane == 0) s[e] = dot;
-  }
-  __syncthreads();
-  if (warp != 0) return;
+// The choice of one token by one warp, from its experts' dot products s [E] (overwritten); gs: [groups] floats.
+__device__ __forceinline__ void moe_choose(float* s, float* gs, int lane, int t, int* __restrict__ ids, float* __restrict__ wts, int E, int top,
+                                           int renorm, int sigmoid, int groups, int keep, int group_top, float wscale) {
   if (sigmoid) {
     for (int e = lane; e < E; e += 32) s[e] = 1.0f / (1.0f + expf(-s[e]));
   } else {
@@ -142,6 +125,107 @@ moe_route_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr, int*
     for (int r = 0; r < top; ++r) wts[(size_t)t * top + r] /= chosen_sum;
 }
 
+// Any sizes.  One block per token: its warps share the experts' dot products, the first warp then takes the choice.
+template <typename T>
+__global__ void __launch_bounds__(MOE_ROUTE_WARPS * 32)
+moe_route_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr, int* __restrict__ ids, float* __restrict__ wts,
+                 int n_tokens, int D, int E, int top, int renorm, int sigmoid, int groups, int keep, int group_top,
+                 float wscale) {
+  extern __shared__ float sh[];  // [E] scores, [groups] group scores
+  pdl_wait();
+  pdl_launch();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x;
+  float* s = sh;
+  float* gs = sh + E;
+  const T* hr = h + (size_t)t * ld;
+  for (int e = warp; e < E; e += MOE_ROUTE_WARPS) {
+    const float dot = warp_dot(hr, wr + (size_t)e * D, D, lane);
+    if (lane == 0) s[e] = dot;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  moe_choose(s, gs, lane, t, ids, wts, E, top, renorm, sigmoid, groups, keep, group_top, wscale);
+}
+
+// The same where rows are 16-byte pieces: a CTA of W warps takes TT tokens, whose inputs it keeps in shared memory, a warp two
+// experts at a time, so that a weight row is read once per TT tokens and an input piece is widened once per two experts.  The
+// 2 TT sums of the 32 lanes are added with halving exchanges; then a warp per token chooses.
+// Measured on a B200, 32 experts over 2,048 numbers, inside a step: 8 tokens 13 -> 7 us, 3,600 tokens 73 -> 38 us.
+__device__ __forceinline__ void moe_widen(const uint4& u, float* v, const float*) {
+  v[0] = __uint_as_float(u.x); v[1] = __uint_as_float(u.y); v[2] = __uint_as_float(u.z); v[3] = __uint_as_float(u.w);
+}
+__device__ __forceinline__ void moe_widen(const uint4& u, float* v, const bf16*) {
+  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = __bfloat1622float2(p[j]);
+    v[2 * j] = f.x;
+    v[2 * j + 1] = f.y;
+  }
+}
+template <typename T, int TT, int W>
+__global__ void __launch_bounds__(W * 32)
+moe_route_tile_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr, int* __restrict__ ids, float* __restrict__ wts,
+                      int n_tokens, int D, int E, int top, int renorm, int sigmoid, int groups, int keep, int group_top, float wscale) {
+  constexpr int VE = 16 / (int)sizeof(T), N = 2 * TT;
+  static_assert(TT <= W, "a warp per token chooses");
+  extern __shared__ __align__(16) unsigned char raw[];  // [TT][D] inputs, [TT][E] scores, [TT][groups] group scores
+  uint4* hs = reinterpret_cast<uint4*>(raw);
+  const int pieces = D / VE;
+  float* sc = reinterpret_cast<float*>(hs + (size_t)TT * pieces);
+  float* gs = sc + TT * E;
+  pdl_wait();
+  pdl_launch();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = blockIdx.x * TT;
+  const int nt = n_tokens - t0 < TT ? n_tokens - t0 : TT;
+  for (int tt = 0; tt < TT; ++tt)
+    for (int i = threadIdx.x; i < pieces; i += W * 32)
+      hs[tt * pieces + i] = reinterpret_cast<const uint4*>(h + (size_t)(t0 + (tt < nt ? tt : nt - 1)) * ld)[i];
+  __syncthreads();
+  for (int e0 = 2 * warp; e0 < E; e0 += 2 * W) {
+    const uint4* w0 = reinterpret_cast<const uint4*>(wr + (size_t)e0 * D);
+    const uint4* w1 = reinterpret_cast<const uint4*>(wr + (size_t)(e0 + 1 < E ? e0 + 1 : e0) * D);
+    float acc[N];                                       // [expert][token]
+#pragma unroll
+    for (int i = 0; i < N; ++i) acc[i] = 0.0f;
+#pragma unroll(TT == 1 ? 4 : 1)
+    for (int i = lane; i < pieces; i += 32) {
+      float a[VE], b[VE];
+      moe_widen(w0[i], a, h);
+      moe_widen(w1[i], b, h);
+#pragma unroll
+      for (int tt = 0; tt < TT; ++tt) {
+        float x[VE];
+        moe_widen(hs[tt * pieces + i], x, h);
+#pragma unroll
+        for (int j = 0; j < VE; ++j) {
+          acc[tt] = fmaf(x[j], a[j], acc[tt]);
+          acc[TT + tt] = fmaf(x[j], b[j], acc[TT + tt]);
+        }
+      }
+    }
+    int mine = 0;
+#pragma unroll
+    for (int o = 16, n = N; o > 0; o >>= 1, n >>= 1) {
+      if (n > 1) {
+        const bool up = (lane & o) != 0;
+        mine = 2 * mine + (up ? 1 : 0);
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i)
+          if (i < n / 2) {
+            const float keep_ = up ? acc[i + n / 2] : acc[i], give = up ? acc[i] : acc[i + n / 2];
+            acc[i] = keep_ + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+      } else acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+    }
+    const int e = e0 + mine / TT;
+    if (lane % (32 / N) == 0 && e < E) sc[(mine % TT) * E + e] = acc[0];
+  }
+  __syncthreads();
+  if (warp < nt) moe_choose(sc + warp * E, gs + warp * groups, lane, t0 + warp, ids, wts, E, top, renorm, sigmoid, groups, keep, group_top, wscale);
+}
+
 extern "C" int hb_moe_route(int dtype, const void* h, int ld, const void* w_router, int* ids, float* weights, int n_tokens,
                             int D, int E, int top, int renorm, int sigmoid, int groups, int keep, int group_top,
                             float wscale, void* stream) {
@@ -152,29 +236,36 @@ extern "C" int hb_moe_route(int dtype, const void* h, int ld, const void* w_rout
   const size_t smem = (size_t)(E + groups) * sizeof(float);
   HB_REQUIRE(smem <= 48 * 1024, "moe_route: %d experts exceed what a block keeps in shared memory", E);
   dim3 grid(n_tokens);
+  // Eight tokens a CTA once that gives half of the SMs one; one token a CTA of 16 warps for fewer (a decode step).
+  const int es = dtype == HB_F32 ? 4 : 2;
+  const bool rows16 = (D * es) % 16 == 0 && ((long long)ld * es) % 16 == 0 && (((uintptr_t)h | (uintptr_t)w_router) & 15) == 0;
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  auto need = [&](int tt) { return (size_t)tt * ((size_t)D * es + (size_t)(E + groups) * sizeof(float)); };
+  const int tt = n_tokens >= 4 * sms && need(8) <= 100 * 1024 ? 8 : 1;
+  if (rows16 && need(tt) <= 100 * 1024) {
+#define MR_GO(T, TT, W)                                                                                                                        \
+  do {                                                                                                                                         \
+    if (need(TT) > 48 * 1024) cudaFuncSetAttribute(moe_route_tile_kernel<T, TT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(TT)); \
+    hb_launch(moe_route_tile_kernel<T, TT, W>, dim3(ceil_div(n_tokens, TT)), dim3(W * 32), need(TT), (cudaStream_t)stream, (const T*)h, ld,      \
+              (const T*)w_router, ids, weights, n_tokens, D, E, top, renorm, sigmoid, groups, keep, group_top, wscale);                         \
+  } while (0)
+    if (dtype == HB_F32) {
+      if (tt == 8) MR_GO(float, 8, 8); else MR_GO(float, 1, 16);
+    } else {
+      if (tt == 8) MR_GO(bf16, 8, 8); else MR_GO(bf16, 1, 16);
+    }
+#undef MR_GO
+    HB_CHECK_LAUNCH("moe_route");
+    return 0;
+  }
   if (dtype == HB_F32)
     hb_launch(moe_route_kernel<float>, grid, dim3(MOE_ROUTE_WARPS * 32), smem, (cudaStream_t)stream, (const float*)h, ld, (const float*)w_router, ids, weights, n_tokens, D, E, top, renorm, sigmoid, groups, keep, group_top, wscale);
   else
     hb_launch(moe_route_kernel<bf16>, grid, dim3(MOE_ROUTE_WARPS * 32), smem, (cudaStream_t)stream, (const bf16*)h, ld, (const bf16*)w_router, ids, weights, n_tokens, D, E, top, renorm, sigmoid, groups, keep, group_top, wscale);
   HB_CHECK_LAUNCH("moe_route");
   return 0;
-}
-
-// A gated expert's hidden value from its two products.  The clamped form (HB_ACT_SWISH_CLAMP, with a limit L):
-// g' = min(g, L), v' = clamp(v, -L, L), g' sigmoid(1.702 g') (v' + 1); every other activation: act(g) v.
-__device__ __forceinline__ float moe_act(float z, int act);
-__device__ __forceinline__ float moe_glu(float g, float v, int act, float limit) {
-  if (act == HB_ACT_SWISH_CLAMP) {
-    g = fminf(g, limit);
-    v = fminf(fmaxf(v, -limit), limit);
-    return (g / (1.0f + expf(-HB_SWISH_CLAMP_SLOPE * g))) * (v + 1.0f);
-  }
-  return moe_act(g, act) * v;
-}
-__device__ __forceinline__ float moe_act(float z, int act) {
-  if (act == HB_ACT_GELU) return 0.5f * z * (1.0f + erff(z * 0.70710678118654752440f));
-  if (act == HB_ACT_GELU_TANH) return 0.5f * z * (1.0f + tanhf(0.79788456080286535588f * (z + 0.044715f * z * z * z)));
-  return z / (1.0f + expf(-z));
 }
 
 // mid[(t*top + r), f] = act(Up_e[f, :] . h[t, :]),  e = ids[t, r]; gated: act(gate row f . h) * (up row f . h) of
@@ -424,20 +515,57 @@ moe_grouped_gemm_kernel(const bf16* __restrict__ A, int lda, const bf16* __restr
     }
 }
 
-// slot: where each pair's row lies in `part` (null: at the pair's own index); wts null: weights of 1
-__global__ void moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts, float* __restrict__ y, int ldy,
-                                   int D, int top, int accumulate, const int* __restrict__ slot) {
+// slot: where each pair's row lies in `part` (null: at the pair's own index); wts null: weights of 1.  V = 4: four columns a
+// thread (D, ldy multiples of 4, rows on 16 bytes), the rows of four pairs asked for at once.
+// Bound by the pairs' rows.  Measured on a B200, 3,600 tokens of 2,048 numbers, 4 pairs each, inside a step: 65 -> 34 us.
+template <int V>
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts, float* __restrict__ y, int ldy, int D, int top,
+                   int accumulate, const int* __restrict__ slot) {
   pdl_wait();
   pdl_launch();
-  const int t = blockIdx.y, d = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.y, d = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (d >= D) return;
-  float acc = 0.0f;
-  for (int r = 0; r < top; ++r) {
-    const size_t u = (size_t)t * top + r;
-    acc = fmaf(wts ? wts[u] : 1.0f, part[(slot ? (size_t)slot[u] : u) * D + d], acc);
-  }
+  float acc[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) acc[j] = 0.0f;
   float* o = y + (size_t)t * ldy + d;
-  *o = accumulate ? *o + acc : acc;
+  float old[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) old[j] = 0.0f;
+  if (accumulate) {
+    if constexpr (V == 4) { const float4 x = *reinterpret_cast<const float4*>(o); old[0] = x.x; old[1] = x.y; old[2] = x.z; old[3] = x.w; }
+    else old[0] = *o;
+  }
+  for (int r0 = 0; r0 < top; r0 += 4) {
+    float w[4], x[4][V];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      w[r] = 0.0f;
+      if (r0 + r >= top) continue;
+      const size_t u = (size_t)t * top + r0 + r;
+      w[r] = wts ? wts[u] : 1.0f;
+      const float* p = part + (slot ? (size_t)slot[u] : u) * D + d;
+      if constexpr (V == 4) { const float4 v = *reinterpret_cast<const float4*>(p); x[r][0] = v.x; x[r][1] = v.y; x[r][2] = v.z; x[r][3] = v.w; }
+      else x[r][0] = *p;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (r0 + r < top)
+#pragma unroll
+        for (int j = 0; j < V; ++j) acc[j] = fmaf(w[r], x[r][j], acc[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < V; ++j) acc[j] = accumulate ? old[j] + acc[j] : acc[j];
+  if constexpr (V == 4) *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  else *o = acc[0];
+}
+
+static void moe_combine(const float* part, const float* wts, float* y, int ldy, int n_tokens, int D, int top, int accumulate, const int* slot, cudaStream_t s) {
+  if (D % 4 == 0 && ldy % 4 == 0 && (((uintptr_t)part | (uintptr_t)y) & 15) == 0)
+    hb_launch(moe_combine_kernel<4>, dim3(ceil_div(D, 1024), n_tokens), dim3(256), 0, s, part, wts, y, ldy, D, top, accumulate, slot);
+  else
+    hb_launch(moe_combine_kernel<1>, dim3(ceil_div(D, 256), n_tokens), dim3(256), 0, s, part, wts, y, ldy, D, top, accumulate, slot);
 }
 
 extern "C" long long hb_moe_grouped_scratch_ints(int n_tokens, int E, int top) {
@@ -469,8 +597,7 @@ extern "C" int hb_moe_experts_grouped_bf16(const void* h, int ld, const void* up
             weigh_input ? weights : (const float*)nullptr);
   hb_launch(moe_grouped_gemm_kernel<false>, dim3(max_tiles, ceil_div(D, MG_TN)), dim3(MG_THREADS), 0, s, (const bf16*)mid, F,
             (const bf16*)down, (void*)part, D, (const int*)pair_off, (const int*)tile_off, (const int*)list, E, D, F, top, act, 0, 0.0f, (const float*)nullptr);
-  hb_launch(moe_combine_kernel, dim3(ceil_div(D, 256), n_tokens), dim3(256), 0, s, (const float*)part, weigh_input ? (const float*)nullptr : weights, y, ldy, D, top, accumulate,
-            (const int*)nullptr);
+  moe_combine(part, weigh_input ? nullptr : weights, y, ldy, n_tokens, D, top, accumulate, nullptr, s);
   HB_CHECK_LAUNCH("moe_experts_grouped");
   return 0;
 }
@@ -562,8 +689,7 @@ extern "C" int hb_moe_experts_tc_bf16(const void* h, int ld, const void* up, con
   rc = hb_gemm_tcgen05_grouped_bf16(mid, F, down, F, part, D, rows, D, F, E, HB_EPI_STORE_F32, 0.0f, nullptr, rows_used, tile_expert,
                                     error_flag, stream);
   if (rc) return rc;
-  hb_launch(moe_combine_kernel, dim3(ceil_div(D, 256), n_tokens), dim3(256), 0, s, (const float*)part, row_scale ? (const float*)nullptr : weights, y, ldy,
-            D, top, accumulate, (const int*)slot);
+  moe_combine(part, row_scale ? nullptr : weights, y, ldy, n_tokens, D, top, accumulate, slot, s);
   HB_CHECK_LAUNCH("moe_experts_tc (combine)");
   return 0;
 }

@@ -104,6 +104,9 @@ _SIGS = {
                      c_int, c_int, c_float, c_void_p],
     "hb_moe_experts": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                        c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
+    "hb_moe_experts_few_ok": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int],
+    "hb_moe_experts_few_bf16": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
     "hb_group_rmsnorm": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
     "hb_group_rmsnorm_residual": [c_int, c_void_p, c_int, c_void_p, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_int, c_int, c_int, c_float, c_void_p],
@@ -171,7 +174,7 @@ def _fn(name: str):
 
 
 # kernels each launcher starts (for honest launch counts)
-_KERNELS_PER_CALL = {"hb_attention_decode_bf16": 2, "hb_argmax": 2, "hb_sample": 2, "hb_moe_experts": 2,
+_KERNELS_PER_CALL = {"hb_attention_decode_bf16": 2, "hb_argmax": 2, "hb_sample": 2, "hb_moe_experts": 2, "hb_moe_experts_few_bf16": 2,
                      "hb_moe_experts_grouped_bf16": 4, "hb_moe_experts_tc_bf16": 5, "hb_ssd_chunked_bf16": 3}
 _launches = 0
 
@@ -985,6 +988,14 @@ def moe_experts(h, up, down, ids, weights, mid, y, act, accumulate=False, gated=
     _check(h, None, "h"); _check(up, h.dtype, "up"); _check(down, h.dtype, "down"); _check(mid, h.dtype, "mid"); _check(y, torch.float32, "y")
     if not (up.is_contiguous() and down.is_contiguous() and mid.is_contiguous()):
         raise BackendError("moe_experts: up, down and mid must be contiguous")
+    # bfloat16 steps of up to 32 tokens read every chosen expert once for all its tokens; the rest a warp per output number
+    T, top, E, D, F = h.shape[0], ids.shape[1], up.shape[0], h.shape[1], down.shape[2]
+    if h.dtype == torch.bfloat16 and _fn("hb_moe_experts_few_ok")(h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), mid.data_ptr(),
+                                                                  T, top, E, D, F, int(gated)):
+        _run("hb_moe_experts_few_bf16", h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), ids.data_ptr(), weights.data_ptr(),
+             mid.data_ptr(), y.data_ptr(), y.stride(0), T, D, E, F, top, int(act), int(gated), float(act_limit), 1 if weigh_input else 0,
+             1 if accumulate else 0, _stream())
+        return
     _run("hb_moe_experts", dtype_code(h.dtype), h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), ids.data_ptr(),
          weights.data_ptr(), mid.data_ptr(), y.data_ptr(), y.stride(0), h.shape[0], h.shape[1], down.shape[2], ids.shape[1],
          int(act), int(gated), float(act_limit), 1 if weigh_input else 0, 1 if accumulate else 0, _stream())
