@@ -55,7 +55,7 @@ static inline cudaError_t hb_launch_ex(int want_pdl, void (*kernel)(KArgs...), d
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   const int mode = hb_pdl_enabled();
-  cfg.numAttrs = (mode == 1 || (mode == 2 && want_pdl)) ? 1 : 0;
+  cfg.numAttrs = want_pdl >= 0 && (mode == 1 || (mode == 2 && want_pdl)) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>
@@ -68,6 +68,12 @@ template <typename... KArgs, typename... Args>
 static inline cudaError_t hb_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                         Args&&... args) {
   return hb_launch_ex(1, kernel, grid, block, smem, stream, static_cast<KArgs>(args)...);
+}
+// For kernels whose CTAs should spread evenly over the SMs (long ones, about one CTA an SM): never before the predecessor's end.
+template <typename... KArgs, typename... Args>
+static inline cudaError_t hb_launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                          Args&&... args) {
+  return hb_launch_ex(-1, kernel, grid, block, smem, stream, static_cast<KArgs>(args)...);
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -26,6 +26,7 @@
 //   hb_general_delta_scan      the recurrence
 #include "api.h"
 #include "common.cuh"
+#include "scan_rows.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // A CTA takes one head of GP_TOK tokens, a thread one key channel of it (a head wider than the block: several): the
@@ -251,7 +252,7 @@ extern "C" int hb_operand_parts(const float* x, int ld, int fine, int coarse, vo
 }
 
 // ---------------------------------------------------------------------------------------------
-// The recurrence.  A CTA of four warps owns 128 / R value channels of one head of one sequence; a column of the
+// The recurrence for the sizes that scan_rows.cuh does not take.  A CTA of four warps owns 128 / R value channels of one head of one sequence; a column of the
 // state is held by R neighbouring lanes of one warp, RPT rows each in registers (lane g holds rows 4 (i R + g) .. + 3,
 // i = 0 .. RPT / 4 - 1, so that the R lanes read neighbouring 16-byte pieces of a vector and no two meet in a bank).
 // A token costs two sums over the key channels, the second after the first (u^T S before the update, S^T r after
@@ -397,6 +398,14 @@ extern "C" int hb_general_delta_scan(const float* prep, const float* v, int ldv,
                                      void* stream) {
   HB_REQUIRE(n_seqs > 0 && heads > 0 && dk > 0 && dv > 0, "general_delta_scan: sizes must be positive");
   HB_REQUIRE(dk <= 1024, "general_delta_scan: %d key channels per head exceed the supported maximum 1024", dk);
+  ScanRows sr{};
+  for (int j = 0; j < 5; ++j) { sr.vec[j] = prep + (size_t)j * dk; sr.ldvec[j] = (long long)heads * 5 * dk; }
+  sr.v = v; sr.ldv = ldv; sr.state = state; sr.seq_slot = seq_slot; sr.seq_start = seq_start; sr.out = out; sr.ldo = ldo;
+  sr.H = heads; sr.G = heads; sr.dv = dv;
+  if (scan_rows<SCAN_GENERAL>(sr, n_seqs, dk, (cudaStream_t)stream)) {
+    HB_CHECK_LAUNCH("general_delta_scan");
+    return 0;
+  }
   // lanes per column: about 8 rows per lane; 4 when that grid would leave more than half of the SMs without a CTA.
   // The state in memory does not depend on the choice; the order of the sums over the key channels does.
   int sms = 0, dev = 0;

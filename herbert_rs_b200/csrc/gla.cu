@@ -12,6 +12,7 @@
 // norm are float on both paths; q, k, v, g and W1 h come from the projection as floats.
 #include "api.h"
 #include "common.cuh"
+#include "scan_rows.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // a[t, c] = exp(logsigmoid(z) / tau),  z = b[c] + sum_r low[t, r] * W2[c, r].  A CTA takes GD_TOK tokens whose
@@ -65,7 +66,7 @@ extern "C" int hb_gla_decay(int dtype, const float* low, int ld, const void* w2,
 }
 
 // ---------------------------------------------------------------------------------------------
-// The recurrence.  A block owns COLS (32, 16 or 8) value channels of one head of one sequence and walks
+// The recurrence for the sizes that scan_rows.cuh does not take.  A block owns COLS (32, 16 or 8) value channels of one head of one sequence and walks
 // that sequence's tokens of the step in order; thread (x, y) keeps RPT consecutive state rows of column x
 // in registers, 128 / COLS groups of rows side by side (narrower blocks when a step has few sequences and
 // heads, so that one long prompt still spreads over the GPU).  q, k, v and the decays of `chunk` tokens at a time are copied into shared memory
@@ -198,6 +199,15 @@ extern "C" int hb_gla_scan(const float* proj, int ld, int q_off, int k_off, int 
   HB_REQUIRE(dk <= 16 * 64, "gla_scan: %d key channels per head exceed the supported maximum 1024", dk);
   HB_REQUIRE(heads <= 65535 && ceil_div(dv, 8) <= 65535, "gla_scan: too many heads or value channels");
   cudaStream_t s = (cudaStream_t)stream;
+  ScanRows sr{};
+  sr.vec[0] = proj + q_off; sr.vec[1] = proj + k_off; sr.vec[2] = decay;
+  sr.ldvec[0] = sr.ldvec[1] = ld; sr.ldvec[2] = (long long)heads * dk;
+  sr.v = proj + v_off; sr.ldv = ld; sr.state = state; sr.seq_slot = seq_slot; sr.seq_start = seq_start; sr.out = out; sr.ldo = ldo;
+  sr.H = heads; sr.G = heads; sr.dv = dv; sr.scale = qscale;
+  if (scan_rows<SCAN_GLA>(sr, n_seqs, dk, s)) {
+    HB_CHECK_LAUNCH("gla_scan");
+    return 0;
+  }
   const int wide = dk % 4 == 0 && ld % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && (((uintptr_t)proj | (uintptr_t)decay) & 15) == 0;
   // the widest blocks that still give every SM one (a long prompt alone: narrower blocks, more of them)
   int sms = 0, dev = 0;

@@ -22,6 +22,7 @@
 //                       + eps'), where o[n], the column behind the head's n, is a normaliser's read-out
 #include "api.h"
 #include "common.cuh"
+#include "scan_rows.cuh"
 
 __global__ void silu_columns_kernel(float* __restrict__ x, int ld, int col0, int cols, int rows) {
   pdl_wait();
@@ -80,7 +81,7 @@ extern "C" int hb_delta_prepare(float* qk, int ld, int q_off, int k_off, int qk_
 }
 
 // ---------------------------------------------------------------------------------------------
-// The recurrence.  A CTA of four warps owns 128 / R value channels of one head of one sequence; a column of the
+// The recurrence for the sizes that scan_rows.cuh does not take.  A CTA of four warps owns 128 / R value channels of one head of one sequence; a column of the
 // state is held by R neighbouring lanes of one warp, RPT rows each in registers (lane g holds rows 4 (i R + g) .. + 3,
 // i = 0 .. RPT / 4 - 1, so that the R lanes read neighbouring 16-byte pieces of a key and no two meet in a bank), so the two sums over
 // the key channels (S^T k and S^T q) end with shuffles inside the warp and no barrier stands between two tokens.
@@ -504,6 +505,14 @@ extern "C" int hb_linear_scan(int delta, const float* q, int ldq, const float* k
   HB_REQUIRE(heads % qk_heads == 0, "linear_scan: %d heads are not a multiple of %d query/key heads", heads, qk_heads);
   HB_REQUIRE(dk <= 2048, "linear_scan: %d key channels per head exceed the supported maximum 2048", dk);
   HB_REQUIRE(delta ? gates != nullptr : decay != nullptr, "linear_scan: the delta rule needs its gates, the decaying form its decays");
+  ScanRows sr{};
+  sr.vec[0] = q; sr.ldvec[0] = ldq; sr.vec[1] = k; sr.ldvec[1] = ldk;
+  sr.v = v; sr.ldv = ldv; sr.gates = gates; sr.decay = decay; sr.state = state; sr.seq_slot = seq_slot; sr.seq_start = seq_start;
+  sr.out = out; sr.ldo = ldo; sr.H = heads; sr.G = qk_heads; sr.dv = dv;
+  if (delta ? scan_rows<SCAN_DELTA>(sr, n_seqs, dk, (cudaStream_t)stream) : scan_rows<SCAN_DECAY>(sr, n_seqs, dk, (cudaStream_t)stream)) {
+    HB_CHECK_LAUNCH("linear_scan");
+    return 0;
+  }
   // lanes per column: about 16 rows per lane, 8 when that grid would leave more than half of the SMs without a CTA
   // (one long prompt alone).  The state in memory does not depend on the choice; the order of the sums does.
   int sms = 0, dev = 0;
