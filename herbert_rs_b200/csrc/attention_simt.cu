@@ -1,12 +1,12 @@
 // Grouped-query softmax attention over the paged cache, CUDA cores only, any head size up to
-// 512 and any number of heads and groups.  One CTA per (token, query head).
+// 512 and any number of heads and groups.  Eight or two warps of a CTA per (token, query head).
 //
 // This is the attention of the true 32-bit path (prefill and decode alike) and the any-shape
 // fallback of the bfloat16 path.  It follows the reference's online-softmax form
 // (generic_attention/prefill/kernel_f32.rs:61-111): for every key j in the query's range,
 //   s_j = (q . k_j) * scale;  m' = max(m, s_j);  l = l*exp(m-m') + exp(s_j-m');
 //   o = o*exp(m-m') + exp(s_j-m') * v_j;   result o / l,
-// here taken 32 keys at a time, the runs of 32 keys dealt to the CTA's warps, whose (m, l, o) are joined in order at the end.  Range of the query at position p: keys lo..p with
+// here taken 8 keys at a time, the runs of 8 keys dealt to the unit's warps, whose (m, l, o) are joined in order at the end.  Range of the query at position p: keys lo..p with
 // lo = max(0, p - window + 1) when window > 0, else 0 (causal; decode.rs:126-295 scans 0..=pos).
 // Query head h reads key/value head h / (nh/nkv) (loader_common.rs:1003-1005).
 // Two options for other designs: a cap on the scores, s <- cap * tanh(s / cap) after the scale
@@ -21,6 +21,7 @@
 
 #define ATT_MAX_HD 512      // heads of up to 128 and 256 channels take instances with fewer registers for a result
 #define ATT_WARPS 8
+#define ATT_RUN 8           // keys that a warp takes at a time
 
 struct AttnArgs {
   const void* q;
@@ -60,31 +61,38 @@ template <int V> __device__ __forceinline__ void att_load(float* d, const bf16* 
 }
 
 // Bound by the latency of the loads of keys and values: eight lanes share a key's row, so that a load covers whole
-// 128-byte lines, a warp has the rows of several keys under way, and a CTA's eight warps take different runs of keys.
+// 128-byte lines, all rows of a run of eight keys are asked for at once, and a CTA's eight warps take different runs.
 // (One warp per unit with a key a lane read a line per element and took 198 us for 3 sequences of about 150 keys, 16 heads of
-// 128 float channels, on a B200; this form takes 18 us.)
-template <typename T, int MAX_HD, int V>
+// 128 float channels, on a B200; runs of 32 keys, four rows at a time, 18 us; this form 9.7 us.)
+template <typename T, int MAX_HD, int V, int WPU>
 __global__ void __launch_bounds__(ATT_WARPS * 32) attention_simt_kernel(AttnArgs a) {
-  __shared__ __align__(16) float qs[MAX_HD];
+  constexpr int UNITS = ATT_WARPS / WPU;                   // (token, head) pairs of this CTA
+  __shared__ __align__(16) float qs_all[UNITS][MAX_HD];
   __shared__ float os[ATT_WARPS][MAX_HD];
   __shared__ float ms[ATT_WARPS], ls[ATT_WARPS];
   constexpr int NV = (MAX_HD + 32 * V - 1) / (32 * V);     // runs of V channels of a result per lane
+  constexpr int KV = MAX_HD / (8 * V);                     // ... and of a key
+  constexpr bool PREFETCH = MAX_HD <= 128;                 // a run's values fit the registers beside its keys
   pdl_wait();
   pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x / a.nh, h = blockIdx.x % a.nh;
+  const int mine = warp / WPU, part = warp % WPU;          // the unit of this warp, and which of its warps it is
+  const long long last = (long long)a.n_tokens * a.nh - 1, want = (long long)blockIdx.x * UNITS + mine;
+  const long long unit = want < last ? want : last;        // past the last unit: it once more, not stored
+  const int t = (int)(unit / a.nh), h = (int)(unit % a.nh);
   const int kvh = h / (a.nh / a.nkv);
   const int p = a.tok_pos[t], b = a.tok_seq[t];
   const int lo = (a.window > 0 && p - a.window + 1 > 0) ? p - a.window + 1 : 0;
   const T* qp = (const T*)a.q + (size_t)t * a.ldq + (size_t)h * a.hd;
-  for (int d = threadIdx.x; d < a.hd; d += ATT_WARPS * 32) qs[d] = to_f32(qp[d]);
+  float* qs = qs_all[mine];
+  for (int d = part * 32 + lane; d < a.hd; d += WPU * 32) qs[d] = to_f32(qp[d]);
   __syncthreads();
   const int* pages = a.seq_pages + (size_t)b * a.pages_stride;
   const T* kc = (const T*)a.kcache;
   const T* vc = (const T*)a.vcache;
 
   float m = -INFINITY, l = 0.0f;
-  if (a.sink != nullptr && warp == 0) { m = a.sink[h]; l = 1.0f; }
+  if (a.sink != nullptr && part == 0) { m = a.sink[h]; l = 1.0f; }
   const bool gated = a.gate_bias != nullptr;
   const float gb = gated ? a.gate_bias[h] : 0.0f;
   float o[NV * V];
@@ -92,60 +100,84 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_simt_kernel(AttnArgs
   for (int i = 0; i < NV * V; ++i) o[i] = 0.0f;
   const int eight = lane & 7, quarter = lane >> 3;
 
-  for (int j0 = lo + warp * 32; j0 <= p; j0 += ATT_WARPS * 32) {
-    const int j = j0 + lane, jc = j <= p ? j : p;          // lanes past the last key read its row and drop the result
-    const long long row = (((long long)pages[jc / a.page_size] * a.nkv + kvh) * a.page_size + jc % a.page_size) * a.hd;
-    float s = 0.0f;
+  for (int j0 = lo + part * ATT_RUN; j0 <= p; j0 += WPU * ATT_RUN) {
+    long long row[2];                                      // this lane's keys j0 + quarter and j0 + 4 + quarter; past the last key: its row, the result dropped
 #pragma unroll
-    for (int sub = 0; sub < 8; ++sub) {                    // four keys at a time, eight lanes each
-      const T* kr = kc + __shfl_sync(0xffffffffu, row, sub * 4 + quarter);
+    for (int u = 0; u < 2; ++u) {
+      const int j = j0 + 4 * u + quarter, jc = j <= p ? j : p;
+      row[u] = (((long long)pages[jc / a.page_size] * a.nkv + kvh) * a.page_size + jc % a.page_size) * a.hd;
+    }
+    float x[2][KV][V], y[PREFETCH ? ATT_RUN : 1][NV][V];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int i = 0; i < KV; ++i) {
+        const int d = V * (eight + 8 * i);
+        if (d < a.hd) att_load<V>(x[u][i], kc + row[u] + d);
+      }
+    if constexpr (PREFETCH) {                              // the values do not wait for the scores
+#pragma unroll
+      for (int k = 0; k < ATT_RUN; ++k) {
+        const T* vr = vc + __shfl_sync(0xffffffffu, row[k >> 2], (k & 3) * 8);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const int d = V * (lane + 32 * i);
+          if (d < a.hd) att_load<V>(y[k][i], vr + d);
+        }
+      }
+    }
+    float s[2], pj[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
       float dot = 0.0f;
 #pragma unroll
-      for (int i = 0; i < MAX_HD / (8 * V); ++i) {
+      for (int i = 0; i < KV; ++i) {
         const int d = V * (eight + 8 * i);
-        if (d < a.hd) {
-          float x[V];
-          att_load<V>(x, kr + d);
+        if (d < a.hd)
 #pragma unroll
-          for (int c = 0; c < V; ++c) dot = fmaf(qs[d + c], x[c], dot);
-        }
+          for (int c = 0; c < V; ++c) dot = fmaf(qs[d + c], x[u][i][c], dot);
       }
       dot += __shfl_xor_sync(0xffffffffu, dot, 1);
       dot += __shfl_xor_sync(0xffffffffu, dot, 2);
       dot += __shfl_xor_sync(0xffffffffu, dot, 4);
-      const float mine = __shfl_sync(0xffffffffu, dot, (lane & 3) * 8);
-      if (sub == (lane >> 2)) s = mine;
+      s[u] = dot * a.scale;
+      if (a.softcap > 0.0f) s[u] = a.softcap * tanhf(s[u] / a.softcap);
+      if (j0 + 4 * u + quarter > p) s[u] = -INFINITY;
     }
-    s *= a.scale;
-    if (a.softcap > 0.0f) s = a.softcap * tanhf(s / a.softcap);
-    if (j > p) s = -INFINITY;
-    float pj;
     if (gated) {
-      pj = (j <= p) ? 1.0f / (1.0f + expf(-(s + gb))) : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) pj[u] = j0 + 4 * u + quarter <= p ? 1.0f / (1.0f + expf(-(s[u] + gb))) : 0.0f;
     } else {
-      const float m_new = fmaxf(m, warp_max(s));
-      const float corr = expf(m - m_new);  // m = -inf on the first chunk: exp(-inf) = 0
-      pj = (j <= p) ? expf(s - m_new) : 0.0f;
-      l = l * corr + warp_sum(pj);
+      float top = fmaxf(s[0], s[1]);
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 8));
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+      const float m_new = fmaxf(m, top);
+      const float corr = expf(m - m_new);  // m = -inf on the first run: exp(-inf) = 0
+#pragma unroll
+      for (int u = 0; u < 2; ++u) pj[u] = j0 + 4 * u + quarter <= p ? expf(s[u] - m_new) : 0.0f;
+      float sum = pj[0] + pj[1];
+      sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+      l = l * corr + sum;
       m = m_new;
 #pragma unroll
       for (int i = 0; i < NV * V; ++i) o[i] *= corr;
     }
-    const int nk = p - j0 + 1 < 32 ? p - j0 + 1 : 32;
-#pragma unroll 4
-    for (int k = 0; k < nk; ++k) {
-      const float pk = __shfl_sync(0xffffffffu, pj, k);
-      const T* vr = vc + __shfl_sync(0xffffffffu, row, k);
+    const int nk = p - j0 + 1 < ATT_RUN ? p - j0 + 1 : ATT_RUN;
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int d = V * (lane + 32 * i);
-        if (d < a.hd) {
-          float x[V];
-          att_load<V>(x, vr + d);
+    for (int k = 0; k < ATT_RUN; ++k) {
+      const float pk = __shfl_sync(0xffffffffu, pj[k >> 2], (k & 3) * 8);
+      const long long vrow = PREFETCH ? 0 : __shfl_sync(0xffffffffu, row[k >> 2], (k & 3) * 8);
+      if (k < nk)
 #pragma unroll
-          for (int c = 0; c < V; ++c) o[i * V + c] = fmaf(pk, x[c], o[i * V + c]);
+        for (int i = 0; i < NV; ++i) {
+          const int d = V * (lane + 32 * i);
+          if (d < a.hd) {
+            if constexpr (!PREFETCH) att_load<V>(y[0][i], vc + vrow + d);
+#pragma unroll
+            for (int c = 0; c < V; ++c) o[i * V + c] = fmaf(pk, y[PREFETCH ? k : 0][i][c], o[i * V + c]);
+          }
         }
-      }
     }
   }
   if (lane == 0) { ms[warp] = m; ls[warp] = l; }
@@ -157,28 +189,30 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_simt_kernel(AttnArgs
       for (int c = 0; c < V; ++c) os[warp][d + c] = o[i * V + c];
   }
   __syncthreads();
-  float top = ms[0], inv = 1.0f, part[ATT_WARPS];
+  const int w0 = mine * WPU;                               // the unit's warps
+  float top = ms[w0], inv = 1.0f, f[WPU];
 #pragma unroll
-  for (int w = 1; w < ATT_WARPS; ++w) top = fmaxf(top, ms[w]);
+  for (int w = 1; w < WPU; ++w) top = fmaxf(top, ms[w0 + w]);
   if (gated) {
 #pragma unroll
-    for (int w = 0; w < ATT_WARPS; ++w) part[w] = 1.0f;
+    for (int w = 0; w < WPU; ++w) f[w] = 1.0f;
   } else {
     float sum = 0.0f;
 #pragma unroll
-    for (int w = 0; w < ATT_WARPS; ++w) {
-      part[w] = ms[w] == -INFINITY ? 0.0f : expf(ms[w] - top);      // a warp without keys: nothing
-      sum = fmaf(ls[w], part[w], sum);
+    for (int w = 0; w < WPU; ++w) {
+      f[w] = ms[w0 + w] == -INFINITY ? 0.0f : expf(ms[w0 + w] - top);      // a warp without keys: nothing
+      sum = fmaf(ls[w0 + w], f[w], sum);
     }
     inv = sum > 0.0f ? 1.0f / sum : 0.0f;
   }
+  if (want > last) return;
   if (a.out_gate != nullptr) inv *= 1.0f / (1.0f + expf(-a.out_gate[(size_t)t * a.ldg + h]));
   T* op = (T*)a.out + (size_t)t * a.ldo + (size_t)h * a.hd;
   float* of = (float*)a.out + (size_t)t * a.ldo + (size_t)h * a.hd;
-  for (int d = threadIdx.x; d < a.hd; d += ATT_WARPS * 32) {
-    float v = os[0][d] * part[0];
+  for (int d = part * 32 + lane; d < a.hd; d += WPU * 32) {
+    float v = os[w0][d] * f[0];
 #pragma unroll
-    for (int w = 1; w < ATT_WARPS; ++w) v = fmaf(os[w][d], part[w], v);
+    for (int w = 1; w < WPU; ++w) v = fmaf(os[w0 + w][d], f[w], v);
     if (a.out_f32) of[d] = v * inv;
     else op[d] = from_f32<T>(v * inv);
   }
@@ -197,12 +231,22 @@ extern "C" int hb_attention_simt(int dtype, const void* q, int ldq, void* out, i
   HB_REQUIRE(gate_bias == nullptr || sink == nullptr, "attention: sigmoid weights have no sink");
   AttnArgs a{q, ldq, out, ldo, kcache, vcache, tok_seq, tok_pos, seq_pages, pages_stride,
              n_tokens, nh, nkv, hd, page_size, scale, window, softcap, sink, gate_bias, out_gate, ldg, out_f32};
-  const long long blocks = (long long)n_tokens * nh;
-  HB_REQUIRE(blocks < 2147483647LL, "attention: too many (token, head) pairs");
+  const long long units = (long long)n_tokens * nh;
+  HB_REQUIRE(units < 2147483647LL, "attention: too many (token, head) pairs");
   // four elements a load where every head's row starts on four
   const int es = dtype == HB_F32 ? 4 : 2;
   const bool v4 = hd % 4 == 0 && (((uintptr_t)kcache | (uintptr_t)vcache) & (uintptr_t)(4 * es - 1)) == 0;
-#define AS_GO(T, MAX_HD, V) hb_launch(attention_simt_kernel<T, MAX_HD, V>, dim3((unsigned)blocks), dim3(ATT_WARPS * 32), 0, (cudaStream_t)stream, a)
+  // Eight warps share a unit's keys where units are few (a decode step); two where they fill the GPU several times over (a
+  // prompt: 4,000 units of up to 150 keys 54 -> 38 us, since a unit's start and end cost as much as its keys)
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const bool many = units >= 8LL * sms;
+#define AS_GO(T, MAX_HD, V)                                                                                                                  \
+  do {                                                                                                                                       \
+    if (many) hb_launch(attention_simt_kernel<T, MAX_HD, V, 2>, dim3((unsigned)ceil_div_ll(units, ATT_WARPS / 2)), dim3(ATT_WARPS * 32), 0, (cudaStream_t)stream, a); \
+    else hb_launch(attention_simt_kernel<T, MAX_HD, V, 8>, dim3((unsigned)units), dim3(ATT_WARPS * 32), 0, (cudaStream_t)stream, a);          \
+  } while (0)
 #define AS_SIZE(T)                                                                        \
   do {                                                                                    \
     if (!v4) AS_GO(T, 512, 1);                                                            \

@@ -30,7 +30,12 @@ def test_gemm_f32_rows_and_tiles(M, N, K):
 @pytest.mark.parametrize("nh,nkv,hd", [(2, 1, 33), (4, 2, 128), (2, 2, 132), (2, 1, 500)])
 @pytest.mark.parametrize("window", [None, 257])
 def test_attention_simt_runs_of_keys(dtype, nh, nkv, hd, window):
-    lens, qlens = [1, 32, 33, 256, 257, 600], [1, 2, 1, 1, 3, 1]
+    few = ([1, 32, 33, 256, 257, 600], [1, 2, 1, 1, 3, 1])
+    for lens, qlens in (few, ([620, 9], [600, 9])):          # eight warps a unit, and two
+        _runs(dtype, nh, nkv, hd, window, lens, [min(n, q) for n, q in zip(lens, qlens)])
+
+
+def _runs(dtype, nh, nkv, hd, window, lens, qlens):
     c = _attention_case(dtype, nh, nkv, hd, lens, qlens, window)
     out = torch.empty(c["q"].shape, device="cuda", dtype=dtype)
     ops.attention_simt(dev(c["q"]), c["q"].shape[1], out, dev(c["k"]), dev(c["v"]), dev(c["tok_seq"]), dev(c["tok_pos"]),
