@@ -17,6 +17,7 @@ extern "C" {
 #define HB_EPI_STORE_F32 1  // C (float)            = A W^T
 #define HB_EPI_RESIDUAL 2   // C (float)           += A W^T
 #define HB_EPI_SWIGLU 3     // C (activation dtype) = silu(gate) * up, W rows in groups of 8 gate, 8 up
+#define HB_EPI_ACT 5        // C (activation dtype) = act(A W^T) (4 is a product's own); the product grouped by expert only
 
 // activations of the gated and routed feed-forwards
 #define HB_ACT_SILU 0       // z / (1 + exp(-z))
@@ -112,8 +113,8 @@ int hb_gemm_tcgen05_set_workspace(float* floats, int* counters, int ctas);
 int hb_gemm_tcgen05_bf16(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N, int K, int
     epi, float glu_limit, int* error_flag, void* stream);
 int hb_gemm_tcgen05_grouped_bf16(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M_max,
-    int N, int K, int E, int epi, float glu_limit, const float* row_scale, const int* rows_used, const int*
-    tile_expert, int* error_flag, void* stream);
+    int N, int K, int E, int epi, float glu_limit, int act, const float* row_scale, const int* rows_used,
+    const int* tile_expert, int* error_flag, void* stream);
 int hb_gemm_tcgen05_qkv_ok(int M, int N);
 int hb_gemm_tcgen05_qkv_bf16(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N,
     int K, const float* in_sumsq, int in_parts, int in_stride, float in_eps, const float* qw, const float* kw,
@@ -175,7 +176,8 @@ long long hb_moe_grouped_scratch_ints(int n_tokens, int E, int top);
 int hb_moe_experts_tc_rows(int n_tokens, int E, int top);
 int hb_moe_experts_tc_bf16(const void* h, int ld, const void* up, const void* down, const int* ids, const
     float* weights, int* ints, void* sorted, void* mid, float* part, float* y, int ldy, int n_tokens, int D,
-    int E, int F, int top, float act_limit, float* row_scale, int accumulate, int* error_flag, void* stream);
+    int E, int F, int top, int act, int gated, float act_limit, float* row_scale, int accumulate, int* error_flag,
+    void* stream);
 int hb_moe_experts_grouped_bf16(const void* h, int ld, const void* up, const void* down, const int* ids, const
     float* weights, int* scratch, void* mid, float* part, float* y, int ldy, int n_tokens, int D, int E, int
     F, int top, int act, int gated, float act_limit, int weigh_input, int accumulate, void* stream);

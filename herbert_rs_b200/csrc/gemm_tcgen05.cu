@@ -793,17 +793,17 @@ extern "C" int hb_gemm_tcgen05_bf16(const void* A, int lda, const void* W, int l
 // A product grouped by expert: A [M_max, K] holds rows sorted by expert, each expert's run padded to whole tiles of
 // 128 rows; W [E * N, K] stacks the experts' matrices; tile i of A (128 rows) is multiplied by the matrix of expert
 // tile_expert[i]; only the first *rows_used rows are computed (both written on the device before this launch).
-// C [M_max, N] (EPI_STORE, EPI_STORE_F32) or [M_max, N / 2] (EPI_SWIGLU; with glu_limit > 0 the clamped form of the gated
+// C [M_max, N] (EPI_STORE, EPI_STORE_F32, EPI_ACT: with the activation `act`) or [M_max, N / 2] (EPI_SWIGLU; with glu_limit > 0 the clamped form of the gated
 // activation).  row_scale [M_max]: a factor per row on the results, before the activation; or null.  Rows of padding are
 // computed and mean nothing.
 extern "C" int hb_gemm_tcgen05_grouped_bf16(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M_max,
-                                            int N, int K, int E, int epi, float glu_limit, const float* row_scale, const int* rows_used,
+                                            int N, int K, int E, int epi, float glu_limit, int act, const float* row_scale, const int* rows_used,
                                             const int* tile_expert, int* error_flag, void* stream) {
   HB_REQUIRE(M_max > 0 && N > 0 && K > 0 && E > 0, "gemm_tcgen05_grouped: sizes must be positive");
   HB_REQUIRE(M_max % TG_BM == 0, "gemm_tcgen05_grouped: %d rows are not whole tiles of %d", M_max, TG_BM);
   HB_REQUIRE(K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0, "gemm_tcgen05_grouped: K (%d) and the leading dimensions (%d, %d) must be multiples of 8", K, lda, ldw);
   HB_REQUIRE(((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0, "gemm_tcgen05_grouped: operands must be 16-byte aligned");
-  HB_REQUIRE(epi == HB_EPI_STORE || epi == HB_EPI_STORE_F32 || (epi == HB_EPI_SWIGLU && N % 16 == 0),
+  HB_REQUIRE(epi == HB_EPI_STORE || epi == HB_EPI_STORE_F32 || epi == HB_EPI_ACT || (epi == HB_EPI_SWIGLU && N % 16 == 0),
              "gemm_tcgen05_grouped: epilogue %d with N=%d is not served", epi, N);
   HB_REQUIRE(rows_used != nullptr && tile_expert != nullptr && error_flag != nullptr, "gemm_tcgen05_grouped: needs the row count, the tiles' experts and an error flag");
   HB_REQUIRE((long long)E * N < 2147483647LL, "gemm_tcgen05_grouped: too many weight rows");
@@ -817,6 +817,7 @@ extern "C" int hb_gemm_tcgen05_grouped_bf16(const void* A, int lda, const void* 
   TgNorm none{};
   none.glu_limit = epi == HB_EPI_SWIGLU ? glu_limit : 0.0f;
   none.row_scale = row_scale;
+  none.act = act;
   HB_REQUIRE(row_scale == nullptr || epi == HB_EPI_SWIGLU, "gemm_tcgen05_grouped: a factor per row goes with the gated epilogue");
   TgGrouped grp;
   grp.rows_used = rows_used;
@@ -827,10 +828,12 @@ extern "C" int hb_gemm_tcgen05_grouped_bf16(const void* A, int lda, const void* 
                      : tg_launch<128, HB_EPI_SWIGLU, true>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
   if (BN == 256) {
     if (epi == HB_EPI_SWIGLU) return tg_launch<256, HB_EPI_SWIGLU, false>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
+    if (epi == HB_EPI_ACT) return tg_launch<256, HB_EPI_ACT, false>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
     if (epi == HB_EPI_STORE) return tg_launch<256, HB_EPI_STORE, false>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
     return tg_launch<256, HB_EPI_STORE_F32, false>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
   }
   if (epi == HB_EPI_SWIGLU) return tg_launch<128, HB_EPI_SWIGLU, false>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
+  if (epi == HB_EPI_ACT) return tg_launch<128, HB_EPI_ACT, false>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
   if (epi == HB_EPI_STORE) return tg_launch<128, HB_EPI_STORE, false>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
   return tg_launch<128, HB_EPI_STORE_F32, false>(ma, mw, C, ldc, M_max, N, K, error_flag, s, none, grp);
 }

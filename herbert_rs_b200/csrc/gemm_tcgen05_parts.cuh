@@ -4,6 +4,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "moe_act.cuh"
 #include "tcgen05_utils.cuh"
 
 #define TG_BM 128
@@ -36,6 +37,7 @@ struct TgNorm {
   float glu_limit;
   // A factor per row of A by which the results are multiplied, in place of 1 / rms (the product grouped by expert); or null
   const float* row_scale;
+  int act;                 // HB_EPI_ACT: the activation (HB_ACT_SILU, HB_ACT_GELU, HB_ACT_GELU_TANH)
 };
 
 // The q/k/v product whose epilogue also does what follows it in an attention layer with heads of
@@ -87,7 +89,11 @@ __device__ __forceinline__ void tg_epilogue32(unsigned (&r)[32], int m, int n, i
           for (int j = 0; j < 8; ++j)
             if (n + blk * 16 + 8 + j < N) out[blk * 8 + j] = __float2bfloat16_rn(y[blk * 8 + j]);
       }
-    } else if (EPI == HB_EPI_STORE) {
+    } else if (EPI == HB_EPI_STORE || EPI == HB_EPI_ACT) {
+      if (EPI == HB_EPI_ACT) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(moe_act(__uint_as_float(r[j]), nm.act));
+      }
       bf16* out = (bf16*)Cv + (size_t)m * ldc + n;
       if (n + 32 <= N && ((((size_t)m * ldc + n) & 7) == 0)) {
 #pragma unroll

@@ -603,14 +603,14 @@ extern "C" int hb_moe_experts_grouped_bf16(const void* h, int ld, const void* up
 }
 
 // ---------------------------------------------------------------------------------------------
-// Long prompts, gated experts with silu (act_limit 0) or the clamped activation (act_limit L > 0), bfloat16: the grouped
-// products on tcgen05.  The pairs are sorted by
+// Long prompts, gated experts with silu (act_limit 0) or the clamped activation (act_limit L > 0), or plain experts with
+// an activation, bfloat16: the grouped products on tcgen05.  The pairs are sorted by
 // expert into a buffer in which every expert's run is padded to whole tiles of 128 rows, so that a tile of the
 // tensor-memory product (gemm_tcgen05.cu, grouped mode) belongs to one expert:
 //   sort:     counts per expert, padded offsets, slot[pair] = its row, tile_expert[tile], rows in use (and, where the
 //             weights multiply the experts' inputs, the weight of every row, by which the product's epilogue multiplies)
 //   gather:   sorted[slot[pair]] = h[pair / top]
-//   product:  mid = silu(gate) * up of sorted x W1_e (the dense feed-forward's fused epilogue)
+//   product:  mid = silu(gate) * up of sorted x W1_e (the dense feed-forward's fused epilogue), or act(sorted x W1_e)
 //   product:  part = mid x W2_e (float)
 //   combine:  y[t] (+)= sum_r weights[t, r] * part[slot[t * top + r]]
 // Rows of padding are computed and never read.  A pair's numbers do not depend on its place.
@@ -660,16 +660,18 @@ extern "C" int hb_moe_experts_tc_rows(int n_tokens, int E, int top) {
   return tiles * 128 > 2147483647LL ? -1 : (int)(tiles * 128);
 }
 
-// up [E, 2F, D] with gate and up rows in groups of 8; row_scale: `rows` floats if the weights multiply the experts' inputs,
+// up [E, 2F, D] with gate and up rows in groups of 8 (`gated` 2), or [E, F, D] (0); row_scale: `rows` floats if the weights multiply the experts' inputs,
 // else null; ints: n_tokens * top + rows / 128 + 1; sorted [rows, D] and
 // mid [rows, F] bfloat16, part [rows, D] floats, with rows = hb_moe_experts_tc_rows(...).
 extern "C" int hb_moe_experts_tc_bf16(const void* h, int ld, const void* up, const void* down, const int* ids,
                                       const float* weights, int* ints, void* sorted, void* mid, float* part, float* y, int ldy,
-                                      int n_tokens, int D, int E, int F, int top, float act_limit, float* row_scale, int accumulate,
-                                      int* error_flag, void* stream) {
+                                      int n_tokens, int D, int E, int F, int top, int act, int gated, float act_limit, float* row_scale,
+                                      int accumulate, int* error_flag, void* stream) {
   HB_REQUIRE(n_tokens > 0 && D > 0 && E > 0 && F > 0 && top > 0, "moe_experts_tc: sizes must be positive");
   HB_REQUIRE(E <= MG_MAX_EXPERTS, "moe_experts_tc: at most %d experts", MG_MAX_EXPERTS);
   HB_REQUIRE(D % 8 == 0 && F % 8 == 0 && ld % 8 == 0 && ((uintptr_t)h & 15) == 0, "moe_experts_tc: widths must be multiples of 8, rows 16-byte aligned");
+  HB_REQUIRE(gated == 2 || (gated == 0 && row_scale == nullptr && (act == HB_ACT_SILU || act == HB_ACT_GELU || act == HB_ACT_GELU_TANH)),
+             "moe_experts_tc: gated experts in groups of 8, or plain ones with silu or a gelu whose weights multiply their outputs");
   HB_REQUIRE(n_tokens <= 65535, "moe_experts_tc: at most 65535 tokens per call");
   const int rows = hb_moe_experts_tc_rows(n_tokens, E, top);
   HB_REQUIRE(rows > 0, "moe_experts_tc: too many pairs");
@@ -683,10 +685,12 @@ extern "C" int hb_moe_experts_tc_bf16(const void* h, int ld, const void* up, con
   hb_launch(moe_gather_rows_kernel, dim3(n_pairs), dim3(D / 8 >= 128 ? 128 : 64), 0, s, (const bf16*)h, ld, (const int*)slot,
             (bf16*)sorted, D / 8, top);
   HB_CHECK_LAUNCH("moe_experts_tc (sort, gather)");
-  int rc = hb_gemm_tcgen05_grouped_bf16(sorted, D, up, D, mid, F, rows, 2 * F, D, E, HB_EPI_SWIGLU, act_limit, row_scale, rows_used,
-                                        tile_expert, error_flag, stream);
+  int rc = gated ? hb_gemm_tcgen05_grouped_bf16(sorted, D, up, D, mid, F, rows, 2 * F, D, E, HB_EPI_SWIGLU, act_limit, 0, row_scale, rows_used,
+                                                tile_expert, error_flag, stream)
+                 : hb_gemm_tcgen05_grouped_bf16(sorted, D, up, D, mid, F, rows, F, D, E, HB_EPI_ACT, 0.0f, act, nullptr, rows_used,
+                                                tile_expert, error_flag, stream);
   if (rc) return rc;
-  rc = hb_gemm_tcgen05_grouped_bf16(mid, F, down, F, part, D, rows, D, F, E, HB_EPI_STORE_F32, 0.0f, nullptr, rows_used, tile_expert,
+  rc = hb_gemm_tcgen05_grouped_bf16(mid, F, down, F, part, D, rows, D, F, E, HB_EPI_STORE_F32, 0.0f, 0, nullptr, rows_used, tile_expert,
                                     error_flag, stream);
   if (rc) return rc;
   moe_combine(part, row_scale ? nullptr : weights, y, ldy, n_tokens, D, top, accumulate, slot, s);

@@ -90,8 +90,8 @@ _SIGS = {
                                     c_void_p],
     "hb_moe_experts_tc_rows": [c_int, c_int, c_int],
     "hb_moe_experts_tc_bf16": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p,
-                               c_void_p],
+                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int,
+                               c_void_p, c_void_p],
     "hb_latent_attention_mma_ok": [c_int, c_int],
     "hb_latent_attention_mma_bf16": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
@@ -937,19 +937,23 @@ def moe_grouped_ok(h, up, gated=0) -> bool:
 
 def moe_tc_ok(h, up, top, gated, act) -> bool:
     """Whether the grouped products run on tcgen05: what `moe_grouped_ok` asks, gated experts with silu or the clamped
-    activation (the product's fused epilogue), and enough (token, expert) pairs that tiles of 128 rows per expert fill."""
-    return (options.moe_tc and moe_grouped_ok(h, up, gated) and gated == GATED_GROUPS_OF_8 and act in (ACT_SILU, ACT_SWISH_CLAMP)
+    activation, or plain ones with silu or a gelu (the product's epilogues), and enough (token, expert) pairs that tiles of
+    128 rows per expert fill (3,400 tokens, 4 of 32 plain experts of 1,408 over 2,048: the two products 185 us against 574 on mma.sync)."""
+    acts = (ACT_SILU, ACT_SWISH_CLAMP) if gated else (ACT_SILU, ACT_GELU, ACT_GELU_TANH)
+    return (options.moe_tc and moe_grouped_ok(h, up, gated) and gated in (0, GATED_GROUPS_OF_8) and act in acts
             and h.shape[0] * int(top) >= MOE_TC_MIN_PAIRS)
 
 
-def moe_experts_tc(h, up, down, ids, weights, y, accumulate, scratch, act_limit=0.0, weigh_input=False) -> None:
-    """moe_experts for long prompts, gated experts with silu (or, with act_limit > 0, the clamped activation): the pairs
+def moe_experts_tc(h, up, down, ids, weights, y, accumulate, scratch, act_limit=0.0, weigh_input=False, gated=GATED_GROUPS_OF_8,
+                   act=ACT_SILU) -> None:
+    """moe_experts for long prompts, gated experts with silu (or, with act_limit > 0, the clamped activation) or plain ones (gated 0) with `act`: the pairs
     sorted by expert into runs padded to tiles of 128 rows, both products on tcgen05 (the first with the gated
     activation in its epilogue)."""
     _check(h, torch.bfloat16, "h"); _check(up, torch.bfloat16, "up"); _check(down, torch.bfloat16, "down"); _check(y, torch.float32, "y")
     T, top = ids.shape
-    E, F2, D = up.shape
-    F = F2 // 2
+    E, F, D = up.shape
+    if gated:
+        F //= 2
     rows = int(_fn("hb_moe_experts_tc_rows")(T, E, top))
     if rows <= 0:
         raise BackendError("moe_experts_tc: too many (token, expert) pairs")
@@ -961,7 +965,7 @@ def moe_experts_tc(h, up, down, ids, weights, y, accumulate, scratch, act_limit=
     _tcgen05_workspace(y.device)
     _run("hb_moe_experts_tc_bf16", h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), ids.data_ptr(), weights.data_ptr(),
          ints.data_ptr(), srt.data_ptr(), mid.data_ptr(), part.data_ptr(), y.data_ptr(), y.stride(0), T, D, E, F, top,
-         float(act_limit), _ptr(row_scale), 1 if accumulate else 0, _error_flag(y.device).data_ptr(), _stream())
+         int(act), int(gated), float(act_limit), _ptr(row_scale), 1 if accumulate else 0, _error_flag(y.device).data_ptr(), _stream())
 
 
 def moe_experts_grouped(h, up, down, ids, weights, y, act, accumulate, scratch, gated=0, act_limit=0.0, weigh_input=False) -> None:

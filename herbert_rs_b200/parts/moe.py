@@ -99,7 +99,8 @@ class RoutedFeedForward(FeedForward):
                       s.group_top, s.weight_scale)
         if ops.moe_tc_ok(h, self.up, s.top_k, self.gated, self.act):
             ops.moe_experts_tc(h, self.up, self.down, ids, weights, residual, accumulate, ws.take,
-                               act_limit=self.act_limit if self.act == ops.ACT_SWISH_CLAMP else 0.0, weigh_input=s.weigh_input)
+                               act_limit=self.act_limit if self.act == ops.ACT_SWISH_CLAMP else 0.0, weigh_input=s.weigh_input,
+                               gated=self.gated, act=self.act)
         elif ops.moe_grouped_ok(h, self.up, self.gated):
             ops.moe_experts_grouped(h, self.up, self.down, ids, weights, residual, self.act, accumulate, ws.take, gated=self.gated,
                                     act_limit=self.act_limit, weigh_input=s.weigh_input)

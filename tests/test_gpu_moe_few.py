@@ -42,6 +42,60 @@ def test_moe_few(T, top, E, D, F, gated, weigh_input, accumulate, twice):
                 m = torch.nn.functional.gelu(z)
             ref[t] += (1.0 if weigh_input else w) * (downd[e].double() @ m)
             size[t] += (1.0 if weigh_input else w) * (downd[e].double().abs() @ m.abs())
-    # the hidden values are rounded to bfloat16 once (2^-9 each); float sums add far less
+    # the hidden values are rounded to bfloat16 once (2^-8 each); float sums add far less
     want = ref + (y0.to(DEV).double() if accumulate else 0.0)
     assert ((y.double() - want).abs() <= size * 2.0 ** -8 + 1e-5).all()
+
+
+@pytest.mark.parametrize("act", [ops.ACT_GELU, ops.ACT_SILU, ops.ACT_GELU_TANH])
+@pytest.mark.parametrize("T,top,E,D,F", [(300, 2, 5, 136, 72), (130, 4, 16, 264, 392), (700, 1, 3, 512, 128)])
+def test_moe_tc_plain_experts(act, T, top, E, D, F):
+    g = torch.Generator(device=DEV).manual_seed(T + D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    h, up, down = rnd(T, D).bfloat16(), (rnd(E, F, D) / D ** 0.5).bfloat16(), (rnd(E, D, F) / F ** 0.5).bfloat16()
+    ids = torch.stack([torch.randperm(E, generator=g, device=DEV)[:top] for _ in range(T)]).int()
+    wts = torch.rand(T, top, generator=g, device=DEV)
+    y0 = rnd(T, D)
+    assert ops.moe_tc_ok(h, up, top, 0, act) == (T * top >= ops.MOE_TC_MIN_PAIRS)
+    assert not ops.moe_tc_ok(h, up, top, 0, ops.ACT_RELU)
+    fn = {ops.ACT_GELU: torch.nn.functional.gelu, ops.ACT_SILU: torch.nn.functional.silu,
+          ops.ACT_GELU_TANH: lambda z: torch.nn.functional.gelu(z, approximate="tanh")}[act]
+    for accumulate in (True, False):
+        y = y0.clone()
+        ops.moe_experts_tc(h, up, down, ids, wts, y, accumulate, lambda s, dt: torch.empty(s, dtype=dt, device=DEV), gated=0, act=act)
+        mid = fn(torch.einsum("td,efd->tef", h.double(), up.double()))
+        chosen = torch.zeros(T, E, dtype=torch.float64, device=DEV).scatter_add_(1, ids.long(), wts.double())
+        ref = torch.einsum("te,tef,edf->td", chosen, mid, down.double())
+        size = torch.einsum("te,tef,edf->td", chosen, mid.abs(), down.double().abs())
+        # the hidden values are rounded to bfloat16 once; float sums and the fast exponential add far less
+        assert ((y.double() - ref - (y0.double() if accumulate else 0.0)).abs() <= size * 2.0 ** -8 + 1e-5).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [1, 7, 600, 1189])
+@pytest.mark.parametrize("E,top,groups,keep", [(1, 1, 1, 1), (15, 3, 3, 2), (32, 4, 8, 4), (70, 6, 1, 1)])
+@pytest.mark.parametrize("D", [8, 20, 264, 2048])
+def test_moe_route_tiles(dtype, T, E, top, groups, keep, D):
+    g = torch.Generator(device=DEV).manual_seed(T + E + D)
+    h, r = torch.randn(T, D, generator=g, device=DEV).to(dtype), (torch.randn(E, D, generator=g, device=DEV) / D ** 0.5).to(dtype)
+    ids = torch.full((T, top), -1, dtype=torch.int32, device=DEV)
+    wts = torch.zeros(T, top, device=DEV)
+    ops.moe_route(h, r, ids, wts, top, renorm=True, score=1, groups=groups, keep=keep, weight_scale=1.5)
+    s = torch.sigmoid(h.double() @ r.double().T)
+    if groups > 1:
+        best = s.view(T, groups, -1).topk(2, -1).values.sum(-1)
+        kept = torch.zeros_like(best, dtype=torch.bool).scatter_(1, best.topk(keep, -1).indices, True)
+        clear = best.sort(-1, descending=True).values
+        sure = clear[:, keep - 1] - clear[:, keep] > 1e-5 if keep < groups else torch.ones(T, dtype=torch.bool, device=DEV)
+        masked = s.masked_fill(~kept.repeat_interleave(E // groups, 1), -1.0)
+    else:
+        sure, masked = torch.ones(T, dtype=torch.bool, device=DEV), s
+    ranked = masked.sort(-1, descending=True).values
+    if top < E:
+        sure &= ranked[:, top - 1] - ranked[:, top] > 1e-5
+    assert (ids >= 0).all() and (ids < E).all()
+    # where the last choice is no tie within float rounding, the choices are the largest scores; the weights are theirs
+    want = masked.topk(top, -1)
+    assert torch.equal(ids.long().sort(-1).values[sure], want.indices.sort(-1).values[sure])
+    got = torch.gather(s, 1, ids.long())
+    assert float((wts.double() - 1.5 * got / got.sum(-1, keepdim=True)).abs().max()) < 2e-5
