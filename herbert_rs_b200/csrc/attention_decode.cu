@@ -670,20 +670,40 @@ __global__ void attention_decode_combine_kernel(const float* __restrict__ part_o
   pdl_launch();
   const int h = blockIdx.x, b = blockIdx.y;
   const size_t base = ((size_t)b * nh + h) * nsplit;
+  const float* ml = part_ml + 2 * base;
+  // Eight splits' numbers are asked for at a time and taken in order: the kernel is a chain of ways to L2 and back
+  // (16 splits, inside a step: 5.1 -> 3.5 us).
   float mm = sink ? sink[h] : -INFINITY;
-  for (int s = 0; s < nsplit; ++s) mm = fmaxf(mm, part_ml[(base + s) * 2]);
+  for (int s0 = 0; s0 < nsplit; s0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = s0 + j < nsplit ? ml[2 * (s0 + j)] : -INFINITY;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mm = fmaxf(mm, v[j]);
+  }
   float ll = sink ? __expf(sink[h] - mm) : 0.0f;
-  for (int s = 0; s < nsplit; ++s) {
-    const float ms = part_ml[(base + s) * 2];
-    if (ms != -INFINITY) ll += __expf(ms - mm) * part_ml[(base + s) * 2 + 1];
+  for (int s0 = 0; s0 < nsplit; s0 += 8) {
+    float2 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = s0 + j < nsplit ? make_float2(ml[2 * (s0 + j)], ml[2 * (s0 + j) + 1]) : make_float2(-INFINITY, 0.0f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (v[j].x != -INFINITY) ll += __expf(v[j].x - mm) * v[j].y;
   }
   float inv = gated ? 1.0f : (ll > 0.0f ? 1.0f / ll : 0.0f);    // sigmoid weights: every m is 0, the partial sums add up
   if (out_gate != nullptr) inv *= 1.0f / (1.0f + expf(-out_gate[(size_t)b * ldg + h]));      // a gate per token and head
   for (int d = threadIdx.x; d < hd; d += blockDim.x) {
     float acc = 0.0f;
-    for (int s = 0; s < nsplit; ++s) {
-      const float ms = part_ml[(base + s) * 2];
-      if (ms != -INFINITY) acc += __expf(ms - mm) * part_o[(base + s) * hd + d];
+    for (int s0 = 0; s0 < nsplit; s0 += 8) {
+      float m[8], o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        m[j] = s0 + j < nsplit ? ml[2 * (s0 + j)] : -INFINITY;
+        o[j] = s0 + j < nsplit ? part_o[(base + s0 + j) * hd + d] : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (m[j] != -INFINITY) acc += __expf(m[j] - mm) * o[j];
     }
     out[(size_t)b * ldo + (size_t)h * hd + d] = __float2bfloat16_rn(acc * inv);
   }
