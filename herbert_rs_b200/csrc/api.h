@@ -148,6 +148,10 @@ int hb_headwise_gemm(int dtype, int out_dtype, const float* in, int ld_in, int i
 int hb_latent_attention(int dtype, const float* q, int ldq, float* out, int ldo, const void* cache, const float*
     sink, const int* tok_seq, const int* tok_pos, const int* seq_pages, int pages_stride, int n_tokens, int
     heads, int rank, int rot, int page_size, int window, void* stream);
+int hb_latent_prefill_tc_ok(int rank, int rot, int page_size);
+int hb_latent_prefill_tc_bf16(const float* q, int ldq, float* out, int ldo, const void* cache, long long cache_rows,
+    const float* sink, const int* seq_start, const int* seq_pos0, const int* seq_pages, int pages_stride, int n_seqs,
+    int max_q_len, int heads, int rank, int rot, int page_size, int window, int* error_flag, void* stream);
 int hb_latent_attention_mma_ok(int rank, int rot);
 int hb_latent_attention_mma_bf16(const float* q, int ldq, float* out, int ldo, const void* cache, const float*
     sink, const int* seq_start, const int* seq_pos0, const int* seq_pages, int pages_stride, int n_seqs, int

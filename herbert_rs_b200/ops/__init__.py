@@ -95,6 +95,9 @@ _SIGS = {
     "hb_latent_attention_mma_ok": [c_int, c_int],
     "hb_latent_attention_mma_bf16": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "hb_latent_prefill_tc_ok": [c_int, c_int, c_int],
+    "hb_latent_prefill_tc_bf16": [c_void_p, c_int, c_void_p, c_int, c_void_p, ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
+                                  c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "hb_gla_decay": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
     "hb_gla_scan": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                     c_int, c_int, c_int, c_float, c_void_p],
@@ -463,6 +466,16 @@ def headwise_gemm(src, src_head_stride, w, out, out_head_stride, scale=1.0, gate
          src.shape[0], H, K, N, float(scale), _stream())
 
 
+def latent_prefill_tc_ok(q, out, cache, heads, rank, rot, page_size, batch) -> bool:
+    """Whether a step's attention over the latent runs on tcgen05: bfloat16, sizes and pages that its tiles take, and enough
+    tiles of 128 (token, head) rows that every SM has one (fewer: the kernel that cuts keys into ranges)."""
+    H, W = int(heads), int(rank) + int(rot)
+    return (cache.dtype == torch.bfloat16 and cache.is_contiguous() and (q.shape[0] * H // 128) * -(-int(rank) // 256) >= sm_count(out.device)
+            and -(-batch.max_q_len * H // 128) <= 65535 and 0 < cache.numel() // W <= 2147483647 and cache.numel() % (W * int(page_size)) == 0
+            and (q.stride(0) | out.stride(0)) % 4 == 0 and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0
+            and bool(_fn("hb_latent_prefill_tc_ok")(int(rank), int(rot), int(page_size))))
+
+
 def latent_attention(q, out, cache, sink, tok_seq, tok_pos, seq_pages, heads, rank, rot, page_size, window, batch=None,
                      scratch=None) -> None:
     """out[t, h, :rank] = sum_j p_j c_j over the cached rows [c_j | r_j] that the token may see, with
@@ -474,6 +487,12 @@ def latent_attention(q, out, cache, sink, tok_seq, tok_pos, seq_pages, heads, ra
     _check(q, torch.float32, "q"); _check(out, torch.float32, "out")
     if sink is not None:
         _check(sink, torch.float32, "sink")
+    if batch is not None and options.latent_attention == "mma" and latent_prefill_tc_ok(q, out, cache, heads, rank, rot, page_size, batch):
+        _run("hb_latent_prefill_tc_bf16", q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), cache.data_ptr(),
+             cache.numel() // (int(rank) + int(rot)), _ptr(sink), batch.seq_start.data_ptr(), batch.seq_pos0.data_ptr(), seq_pages.data_ptr(),
+             seq_pages.stride(0), batch.n_seqs, batch.max_q_len, int(heads), int(rank), int(rot), int(page_size), int(window or 0),
+             _error_flag(out.device).data_ptr(), _stream())
+        return
     if batch is not None and cache.dtype == torch.bfloat16 and options.latent_attention == "mma" \
             and _fn("hb_latent_attention_mma_ok")(int(rank), int(rot)):
         ctas = batch.n_seqs * -(-batch.max_q_len * int(heads) // 32)
@@ -938,7 +957,7 @@ def moe_grouped_ok(h, up, gated=0) -> bool:
 def moe_tc_ok(h, up, top, gated, act) -> bool:
     """Whether the grouped products run on tcgen05: what `moe_grouped_ok` asks, gated experts with silu or the clamped
     activation, or plain ones with silu or a gelu (the product's epilogues), and enough (token, expert) pairs that tiles of
-    128 rows per expert fill (3,400 tokens, 4 of 32 plain experts of 1,408 over 2,048: the two products 185 us against 574 on mma.sync)."""
+    128 rows per expert fill (2,673 tokens, 4 of 32 plain experts of 1,408 over 2,048: the two products 185 us against 574 on mma.sync)."""
     acts = (ACT_SILU, ACT_SWISH_CLAMP) if gated else (ACT_SILU, ACT_GELU, ACT_GELU_TANH)
     return (options.moe_tc and moe_grouped_ok(h, up, gated) and gated in (0, GATED_GROUPS_OF_8) and act in acts
             and h.shape[0] * int(top) >= MOE_TC_MIN_PAIRS)

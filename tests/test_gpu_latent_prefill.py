@@ -1,0 +1,73 @@
+"""Prompts' attention over a cached latent on tcgen05 against float64: both halves of the latent, blocks beyond its width, windows,
+sinks, starts behind cached keys, shuffled pages, rows that do not fill a tile."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from herbert_rs_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("H,rank,rot", [(16, 512, 64), (16, 256, 32), (5, 320, 16), (8, 64, 0), (3, 512, 0), (40, 128, 64)])
+@pytest.mark.parametrize("window,sunk,page", [(None, False, 64), (100, True, 128), (None, True, 64)])
+def test_latent_prefill(H, rank, rot, window, sunk, page):
+    need = -(-150 * 128 // (H * -(-rank // 256)))
+    qlens = [need, 1, 67, 130]
+    pos0 = [0, 200, 63, 0]
+    lens = [p + n for p, n in zip(pos0, qlens)]
+    g = torch.Generator(device=DEV).manual_seed(H + rank + rot)
+    W = rank + rot
+    total = sum(-(-n // page) for n in lens)
+    order = torch.randperm(total + 2, generator=g, device=DEV)
+    cache = torch.zeros(total + 2, 1, page, W, dtype=torch.bfloat16, device=DEV)
+    stride = max(-(-n // page) for n in lens) + 1
+    pages = torch.zeros(len(lens), stride, dtype=torch.int32, device=DEV)
+    keys, at = [], 0
+    for b, n in enumerate(lens):
+        k = torch.randn(n, W, generator=g, device=DEV).bfloat16()
+        keys.append(k)
+        for i in range(-(-n // page)):
+            pages[b, i] = order[at]
+            part = k[i * page:(i + 1) * page]
+            cache[order[at], 0, :len(part)] = part
+            at += 1
+    T = sum(qlens)
+    q = torch.randn(T, H * W, generator=g, device=DEV) * (2.0 / W ** 0.5)
+    sink = torch.randn(H, generator=g, device=DEV) if sunk else None
+    start = [sum(qlens[:i]) for i in range(len(qlens) + 1)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(n_seqs=len(lens), n_tokens=T, max_q_len=max(qlens), seq_start=i32(start), seq_pos0=i32(pos0))
+    out = torch.full((T, H * rank), 9.0, device=DEV)
+    assert ops.latent_prefill_tc_ok(q, out, cache, H, rank, rot, page, batch)
+    tok_seq = i32(sum(([b] * n for b, n in enumerate(qlens)), []))
+    tok_pos = i32(sum((list(range(p, p + n)) for p, n in zip(pos0, qlens)), []))
+    ops.latent_attention(q, out, cache, sink, tok_seq, tok_pos, pages, H, rank, rot, page, window, batch=batch)
+    ops.check_kernel_errors()
+    for b, n in enumerate(qlens):
+        k = keys[b].double()
+        qb = q[start[b]:start[b + 1]].bfloat16().double().view(n, H, W)
+        s = torch.einsum("thw,jw->thj", qb, k)
+        pos = torch.arange(pos0[b], pos0[b] + n, device=DEV)[:, None]
+        j = torch.arange(lens[b], device=DEV)[None]
+        seen = (j <= pos) & (j > pos - window if window else torch.ones_like(j, dtype=torch.bool))
+        s = s.masked_fill(~seen[:, None], float("-inf"))
+        if sunk:
+            s = torch.cat([s, sink.double()[None, :, None].expand(n, H, 1)], -1)
+        p = torch.softmax(s, -1)[..., :lens[b]]
+        ref = torch.einsum("thj,jr->thr", p, k[:, :rank])
+        got = out[start[b]:start[b + 1]].view(n, H, rank).double()
+        # weights are rounded to bfloat16 (2^-8 of each) before their product with the values, and so in their sum
+        bound = torch.einsum("thj,jr->thr", p, k[:, :rank].abs()) * 2.0 ** -7 + 1e-5
+        assert ((got - ref).abs() <= bound).all(), (b, float((got - ref).abs().max()))
+
+
+def test_small_steps_and_odd_pages_keep_their_kernels():
+    b = SimpleNamespace(n_seqs=1, max_q_len=600)
+    for page, n, want in ((64, 600, True), (64, 590, False), (48, 600, False), (32, 600, False)):
+        cache = torch.zeros(4, 1, page, 576, dtype=torch.bfloat16, device=DEV)
+        q, out = torch.zeros(n, 16 * 576, device=DEV), torch.zeros(n, 16 * 512, device=DEV)
+        assert ops.latent_prefill_tc_ok(q, out, cache, 16, 512, 64, page, b) == want
+    assert not ops.latent_prefill_tc_ok(q, out, cache.float(), 16, 512, 64, 64, b)
