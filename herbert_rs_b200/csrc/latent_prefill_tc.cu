@@ -3,7 +3,7 @@
 //
 // A CTA takes 128 consecutive rows (token, head), head fastest, of one sequence, and 256 of the latent's columns.  The
 // queries, rounded to bfloat16 once, stay in shared memory (up to 144 KB); a tile of 64 keys (up to 72 KB) is fetched by TMA
-// in blocks of 64 columns, each with a barrier of its own.  Tensor memory holds the sums over the values (256 columns)
+// in blocks of 64 columns, with a barrier for each of the two kinds below.  Tensor memory holds the sums over the values (256 columns)
 // and two buffers of scores.  The latent's 512 columns do not fit beside the scores, so two CTAs share a tile of
 // rows and both compute its scores: half as many operations again, on a unit that is twelve times as fast as the warp-level instruction.
 //   A-blocks     the columns whose values belong to the other CTA, and the rotated part: free as soon as the scores have read
@@ -13,8 +13,9 @@
 // run while the row threads take this tile's softmax.  A thread owns a row (as in attention_prefill_tc.cu): P goes back over
 // the scores, O is rescaled only when a tile's maximum exceeds the row's reference by more than 2^8.
 // Bound by the reads of the queries from shared memory (4 KB per 128 x 64 x 16 product).
-// Measured on a B200 alone, 16 heads, latent 512 + 64: four prompts of 714 to 2,000 tokens 1,057 us on mma.sync -> 558, four of 336 to
-// 1,500 467 -> 264; of that about 26 us a CTA go into its queries and results.  (32 keys a tile with two sets of blocks: 831.)
+// Measured on a B200 alone, 16 heads, latent 512 + 64: four prompts of 714 to 2,000 tokens 1,057 us on mma.sync -> 389, four of 336 to
+// 1,500 467 -> 191; of that about 26 us a CTA go into its queries and results.  (One barrier a block of columns and a loop over
+// the steps of K: 557 and 263, the MMA lane's own instructions were the limit; 32 keys a tile with two sets of blocks: 590.)
 #include "api.h"
 #include "common.cuh"
 #include "tcgen05_utils.cuh"
@@ -73,12 +74,12 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
   const int NB = (a.W + 63) >> 6;                                          // blocks of 64 columns; beyond W: zeros on both sides
   const unsigned q_s = base, k_s = q_s + NB * LP_QBLOCK, bars = k_s + NB * LP_KBLOCK;
   const int own0 = half * (LP_HALF / 64), nown = min(LP_HALF, a.rank - half * LP_HALF) >> 6, na = NB - nown;
-  auto kfull = [&](int blk) { return bars + blk * 8; };
-  const unsigned a_free = bars + LP_MAX_BLOCKS * 8, s_full = a_free + 8, p_ready = s_full + 16, o_full = p_ready + 8;
+  auto kfull = [&](int kind) { return bars + kind * 8; };                 // 0: a tile's A-blocks, 1: its own blocks
+  const unsigned a_free = bars + 16, s_full = a_free + 8, p_ready = s_full + 16, o_full = p_ready + 8;
   volatile unsigned* tmem_slot = reinterpret_cast<volatile unsigned*>(gen + (o_full + 8 - base));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < LP_MAX_BLOCKS; ++i) mbar_init(kfull(i), 1);
+    for (int i = 0; i < 2; ++i) mbar_init(kfull(i), 1);
     mbar_init(a_free, 1);
     mbar_init(s_full, 1);
     mbar_init(s_full + 8, 1);
@@ -134,14 +135,13 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
       for (int j = 0; j < n; ++j) {
         const int key0 = (tile0 + j) * LP_KEYS, lp = key0 / a.page_size;   // page_size is a multiple of 64: a tile lies in one page
         const int row = pages[lp < a.pages_stride ? lp : a.pages_stride - 1] * a.page_size + key0 % a.page_size;
-        auto fetch = [&](int blk) {
-          mbar_expect_tx(kfull(blk), LP_KBLOCK);
-          tma_load_2d(k_s + blk * LP_KBLOCK, &map_c, blk * 64, row, kfull(blk));
-        };
+        auto fetch = [&](int blk, unsigned full) { tma_load_2d(k_s + blk * LP_KBLOCK, &map_c, blk * 64, row, full); };
         if (na > 0 && j > 0 && !mbar_wait(a_free, (j - 1) & 1)) { atomicExch(a.error_flag, 41); break; }
-        for (int i = 0; i < na; ++i) fetch(a_block(i));
+        if (na > 0) mbar_expect_tx(kfull(0), na * LP_KBLOCK);
+        for (int i = 0; i < na; ++i) fetch(a_block(i), kfull(0));
         if (j > 0 && !mbar_wait(o_full, (j - 1) & 1)) { atomicExch(a.error_flag, 42); break; }
-        for (int i = 0; i < nown; ++i) fetch(own0 + i);
+        mbar_expect_tx(kfull(1), nown * LP_KBLOCK);
+        for (int i = 0; i < nown; ++i) fetch(own0 + i, kfull(1));
       }
     }
   } else if (warp == 1) {
@@ -151,22 +151,23 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
       const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(nown * 8) << 17) | ((unsigned)(LP_ROWS >> 4) << 24);
       const unsigned long long desc_q = umma_desc_sw128(q_s), desc_k = umma_desc_sw128(k_s);
       const unsigned long long desc_v = umma_desc_sw128_mn(k_s + own0 * LP_KBLOCK, LP_KBLOCK);
-      auto scores = [&](int j, int blk, bool first) -> bool {
-        if (!mbar_wait(kfull(blk), j & 1)) { atomicExch(a.error_flag, 43); return false; }
-        tc_fence_after();
-        const int ks_n = min(4, (a.W - blk * 64) >> 4);                    // W is a multiple of 16
-        for (int ks = 0; ks < ks_n; ++ks)
+      auto scores = [&](int j, int blk, bool first) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)                                     // columns past W are zeros on both sides
           tc_mma_bf16(tm_s0 + (j & 1) * LP_KEYS, desc_q + ((blk * LP_QBLOCK + ks * 32) >> 4), desc_k + ((blk * LP_KBLOCK + ks * 32) >> 4), idesc_qk,
                       first && ks == 0 ? 0u : 1u);
-        return true;
       };
       bool ok = true;
       auto a_scores = [&](int j) {
-        for (int i = 0; i < na && ok; ++i) ok = scores(j, a_block(i), i == 0);
+        if (na > 0 && !mbar_wait(kfull(0), j & 1)) { atomicExch(a.error_flag, 43); ok = false; }
+        tc_fence_after();
+        for (int i = 0; i < na && ok; ++i) scores(j, a_block(i), i == 0);
         if (na > 0 && ok) tc_commit(a_free);
       };
       auto own_scores = [&](int j) {
-        for (int i = 0; i < nown && ok; ++i) ok = scores(j, own0 + i, na == 0 && i == 0);
+        if (!mbar_wait(kfull(1), j & 1)) { atomicExch(a.error_flag, 43); ok = false; }
+        tc_fence_after();
+        for (int i = 0; i < nown && ok; ++i) scores(j, own0 + i, na == 0 && i == 0);
         if (ok) tc_commit(s_full + (j & 1) * 8);
       };
       a_scores(0);
