@@ -64,6 +64,9 @@ __device__ __forceinline__ float warp_dot(const bf16* a, const bf16* w, int n, i
 }
 
 // The choice of one token by one warp, from its experts' dot products s [E] (overwritten); gs: [groups] floats.
+// Scores that are not numbers beat nothing: once only such experts are left, the lowest index of them is taken, with a weight that
+// is not a number.  So every index lies in [0, E) and no token names an expert twice, whatever the scores; `top` is at most
+// the experts of `keep` groups, and a group whose score is not a number stays open, so there is always one left.
 __device__ __forceinline__ void moe_choose(float* s, float* gs, int lane, int t, int* __restrict__ ids, float* __restrict__ wts, int E, int top,
                                            int renorm, int sigmoid, int groups, int keep, int group_top, float wscale) {
   if (sigmoid) {
@@ -113,6 +116,15 @@ __device__ __forceinline__ void moe_choose(float* s, float* gs, int lane, int t,
       const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
     }
+    if (bi == E) {               // all lanes alike
+      bi = E - 1;
+      for (int e = lane; e < E; e += 32)
+        if (s[e] != s[e]) bi = min(bi, e);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) bi = min(bi, __shfl_xor_sync(0xffffffffu, bi, o));
+      best = s[bi];
+    }
+    __syncwarp();                // every lane has read the scores: one of them changes next
     if (lane == 0) {
       ids[(size_t)t * top + r] = bi;
       wts[(size_t)t * top + r] = best * wscale;

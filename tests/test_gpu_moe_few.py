@@ -99,3 +99,38 @@ def test_moe_route_tiles(dtype, T, E, top, groups, keep, D):
     assert torch.equal(ids.long().sort(-1).values[sure], want.indices.sort(-1).values[sure])
     got = torch.gather(s, 1, ids.long())
     assert float((wts.double() - 1.5 * got / got.sum(-1, keepdim=True)).abs().max()) < 2e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [3, 1201])
+@pytest.mark.parametrize("E,top,groups,keep,score", [(32, 4, 8, 4, 1), (32, 4, 1, 1, 0), (15, 15, 3, 3, 0), (16, 2, 4, 1, 1), (6, 2, 1, 1, 1)])
+@pytest.mark.parametrize("D", [20, 264])
+def test_moe_route_scores_that_are_not_numbers(dtype, T, E, top, groups, keep, score, D):
+    """A token whose scores are not numbers gets experts that exist, each once, and weights that are not numbers; no other token
+    notices it.  An expert whose scores are not numbers is taken when nothing else is left."""
+    g = torch.Generator(device=DEV).manual_seed(T + E + D)
+    h, r = torch.randn(T, D, generator=g, device=DEV).to(dtype), (torch.randn(E, D, generator=g, device=DEV) / D ** 0.5).to(dtype)
+
+    def route(h, r, top, keep):
+        ids = torch.full((len(h), top), -7, dtype=torch.int32, device=DEV)
+        wts = torch.zeros(len(h), top, device=DEV)
+        ops.moe_route(h, r, ids, wts, top, renorm=True, score=score, groups=groups, keep=keep)
+        return ids, wts
+    ids0, wts0 = route(h, r, top, keep)
+    bad = torch.tensor([t for t in (1, 7, 8, 600, T - 1) if t < T], device=DEV).unique()
+    good = torch.ones(T, dtype=torch.bool, device=DEV)
+    good[bad] = False
+    broken = h.clone()
+    broken[bad[0]] = float("nan")
+    broken[bad[1:], 3] = float("nan")
+    ids, wts = route(broken, r, top, keep)
+    assert torch.equal(ids[good], ids0[good]) and torch.equal(wts[good], wts0[good])
+    assert torch.equal(ids[bad], torch.arange(top, dtype=torch.int32, device=DEV).expand(len(bad), top))
+    assert wts[bad].isnan().all()
+    if score == 1:                                # a softmax over a score that is no number has none that is
+        r2 = r.clone()
+        r2[E // 2] = float("nan")
+        ids, wts = route(h, r2, E if groups == 1 else keep * (E // groups), keep)
+        assert (ids >= 0).all() and (ids < E).all() and (ids.sort(-1).values.diff(dim=-1) > 0).all()
+        assert ((ids == E // 2) == (torch.arange(ids.shape[1], device=DEV) == ids.shape[1] - 1))[(ids == E // 2).any(-1)].all()
+        assert groups > 1 or (ids[:, -1] == E // 2).all()
