@@ -169,7 +169,7 @@ int hb_layernorm_residual(int dtype, const float* y, int ldy, const float* w, co
 int hb_moe_route(int dtype, const void* h, int ld, const void* w_router, int* ids, float* weights, int n_tokens,
     int D, int E, int top, int renorm, int sigmoid, int groups, int keep, int group_top, float wscale, void* stream);
 int hb_moe_experts(int dtype, const void* h, int ld, const void* up, const void* down, const int* ids, const
-    float* weights, void* mid, float* y, int ldy, int n_tokens, int D, int F, int top, int act, int gated,
+    float* weights, void* mid, float* y, int ldy, int n_tokens, int D, int E, int F, int top, int act, int gated,
     float act_limit, int weigh_input, int accumulate, void* stream);
 int hb_moe_experts_few_ok(const void* h, int ld, const void* up, const void* down, const void* mid, int n_tokens, int top,
     int E, int D, int F, int gated);

@@ -19,6 +19,8 @@
 // product with the activation; their second product with the weighted sum.  A warp computes one
 // output number from one weight row read along its length, which is what a step of few tokens
 // wants: every weight row of a chosen expert is read once per token that chose it.
+//
+// A pair whose index lies outside the experts contributes nothing, in every kernel of the feed-forward alike (the router gives none).
 #include "api.h"
 #include "common.cuh"
 #include "moe_act.cuh"
@@ -285,13 +287,14 @@ extern "C" int hb_moe_route(int dtype, const void* h, int ld, const void* w_rout
 template <typename T>
 __global__ void __launch_bounds__(MOE_WARPS * 32)
 moe_up_kernel(const T* __restrict__ h, int ld, const T* __restrict__ up, const int* __restrict__ ids, const float* __restrict__ in_w,
-              T* __restrict__ mid, int D, int F, int top, int act, int gated, float limit) {
+              T* __restrict__ mid, int D, int E, int F, int top, int act, int gated, float limit) {
   pdl_wait();
   pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int f = blockIdx.y * MOE_WARPS + warp, u = blockIdx.x;  // u = t*top + r
   if (f >= F) return;
   const int e = ids[u];
+  if ((unsigned)e >= (unsigned)E) return;
   const T* hr = h + (size_t)(u / top) * ld;
   if (gated) {
     const int grow = gated == 2 ? (f >> 3) * 16 + (f & 7) : f, urow = gated == 2 ? grow + 8 : F + f;
@@ -310,7 +313,7 @@ moe_up_kernel(const T* __restrict__ h, int ld, const T* __restrict__ up, const i
 template <typename T>
 __global__ void __launch_bounds__(MOE_WARPS * 32)
 moe_down_kernel(const T* __restrict__ mid, const T* __restrict__ down, const int* __restrict__ ids, const float* __restrict__ wts,
-                float* __restrict__ y, int ldy, int D, int F, int top, int accumulate) {
+                float* __restrict__ y, int ldy, int D, int E, int F, int top, int accumulate) {
   pdl_wait();
   pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -319,6 +322,7 @@ moe_down_kernel(const T* __restrict__ mid, const T* __restrict__ down, const int
   float acc = 0.0f;
   for (int r = 0; r < top; ++r) {
     const int u = t * top + r;
+    if ((unsigned)ids[u] >= (unsigned)E) continue;
     const T* w = down + ((size_t)ids[u] * D + d) * F;
     const T* m = mid + (size_t)u * F;
     acc = fmaf(wts ? wts[u] : 1.0f, warp_dot(m, w, F, lane), acc);
@@ -330,9 +334,9 @@ moe_down_kernel(const T* __restrict__ mid, const T* __restrict__ down, const int
 }
 
 extern "C" int hb_moe_experts(int dtype, const void* h, int ld, const void* up, const void* down, const int* ids,
-                              const float* weights, void* mid, float* y, int ldy, int n_tokens, int D, int F, int top,
-                              int act, int gated, float act_limit, int weigh_input, int accumulate, void* stream) {
-  HB_REQUIRE(n_tokens > 0 && D > 0 && F > 0 && top > 0, "moe_experts: sizes must be positive");
+                              const float* weights, void* mid, float* y, int ldy, int n_tokens, int D, int E, int F,
+                              int top, int act, int gated, float act_limit, int weigh_input, int accumulate, void* stream) {
+  HB_REQUIRE(n_tokens > 0 && D > 0 && E > 0 && F > 0 && top > 0, "moe_experts: sizes must be positive");
   HB_REQUIRE(!weigh_input || gated, "moe_experts: the weight multiplies the input of gated experts only");
   const float* in_w = weigh_input ? weights : nullptr;
   const float* out_w = weigh_input ? nullptr : weights;
@@ -342,11 +346,11 @@ extern "C" int hb_moe_experts(int dtype, const void* h, int ld, const void* up, 
   cudaStream_t s = (cudaStream_t)stream;
   dim3 g1(n_tokens * top, ceil_div(F, MOE_WARPS)), g2(n_tokens, ceil_div(D, MOE_WARPS));
   if (dtype == HB_F32) {
-    hb_launch(moe_up_kernel<float>, g1, dim3(MOE_WARPS * 32), 0, s, (const float*)h, ld, (const float*)up, ids, in_w, (float*)mid, D, F, top, act, gated, act_limit);
-    hb_launch(moe_down_kernel<float>, g2, dim3(MOE_WARPS * 32), 0, s, (const float*)mid, (const float*)down, ids, out_w, y, ldy, D, F, top, accumulate);
+    hb_launch(moe_up_kernel<float>, g1, dim3(MOE_WARPS * 32), 0, s, (const float*)h, ld, (const float*)up, ids, in_w, (float*)mid, D, E, F, top, act, gated, act_limit);
+    hb_launch(moe_down_kernel<float>, g2, dim3(MOE_WARPS * 32), 0, s, (const float*)mid, (const float*)down, ids, out_w, y, ldy, D, E, F, top, accumulate);
   } else {
-    hb_launch(moe_up_kernel<bf16>, g1, dim3(MOE_WARPS * 32), 0, s, (const bf16*)h, ld, (const bf16*)up, ids, in_w, (bf16*)mid, D, F, top, act, gated, act_limit);
-    hb_launch(moe_down_kernel<bf16>, g2, dim3(MOE_WARPS * 32), 0, s, (const bf16*)mid, (const bf16*)down, ids, out_w, y, ldy, D, F, top, accumulate);
+    hb_launch(moe_up_kernel<bf16>, g1, dim3(MOE_WARPS * 32), 0, s, (const bf16*)h, ld, (const bf16*)up, ids, in_w, (bf16*)mid, D, E, F, top, act, gated, act_limit);
+    hb_launch(moe_down_kernel<bf16>, g2, dim3(MOE_WARPS * 32), 0, s, (const bf16*)mid, (const bf16*)down, ids, out_w, y, ldy, D, E, F, top, accumulate);
   }
   HB_CHECK_LAUNCH("moe_experts");
   return 0;
@@ -378,7 +382,8 @@ moe_group_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __restric
   pdl_launch();
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
-  for (int u = threadIdx.x; u < n_pairs; u += blockDim.x) atomicAdd(&cnt[ids[u]], 1);
+  for (int u = threadIdx.x; u < n_pairs; u += blockDim.x)
+    if ((unsigned)ids[u] < (unsigned)E) atomicAdd(&cnt[ids[u]], 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     int p = 0, tl = 0;
@@ -398,7 +403,7 @@ moe_group_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __restric
   __syncthreads();
   for (int u = threadIdx.x; u < n_pairs; u += blockDim.x) {
     const int e = ids[u];
-    list[off[e] + atomicAdd(&cnt[e], 1)] = u;
+    if ((unsigned)e < (unsigned)E) list[off[e] + atomicAdd(&cnt[e], 1)] = u;
   }
 }
 
@@ -527,13 +532,13 @@ moe_grouped_gemm_kernel(const bf16* __restrict__ A, int lda, const bf16* __restr
     }
 }
 
-// slot: where each pair's row lies in `part` (null: at the pair's own index); wts null: weights of 1.  V = 4: four columns a
+// slot: where each pair's row lies in `part` (null: at the pair's own index); wts null: weights of 1; pairs without an expert are left out.  V = 4: four columns a
 // thread (D, ldy multiples of 4, rows on 16 bytes), the rows of four pairs asked for at once.
 // Bound by the pairs' rows.  Measured on a B200, 3,600 tokens of 2,048 numbers, 4 pairs each, inside a step: 65 -> 34 us.
 template <int V>
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts, float* __restrict__ y, int ldy, int D, int top,
-                   int accumulate, const int* __restrict__ slot) {
+moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts, float* __restrict__ y, int ldy, int D, int E, int top,
+                   int accumulate, const int* __restrict__ slot, const int* __restrict__ ids) {
   pdl_wait();
   pdl_launch();
   const int t = blockIdx.y, d = (blockIdx.x * blockDim.x + threadIdx.x) * V;
@@ -554,8 +559,11 @@ moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       w[r] = 0.0f;
+#pragma unroll
+      for (int j = 0; j < V; ++j) x[r][j] = 0.0f;
       if (r0 + r >= top) continue;
       const size_t u = (size_t)t * top + r0 + r;
+      if ((unsigned)ids[u] >= (unsigned)E) continue;
       w[r] = wts ? wts[u] : 1.0f;
       const float* p = part + (slot ? (size_t)slot[u] : u) * D + d;
       if constexpr (V == 4) { const float4 v = *reinterpret_cast<const float4*>(p); x[r][0] = v.x; x[r][1] = v.y; x[r][2] = v.z; x[r][3] = v.w; }
@@ -573,11 +581,12 @@ moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts
   else *o = acc[0];
 }
 
-static void moe_combine(const float* part, const float* wts, float* y, int ldy, int n_tokens, int D, int top, int accumulate, const int* slot, cudaStream_t s) {
+static void moe_combine(const float* part, const float* wts, float* y, int ldy, int n_tokens, int D, int E, int top, int accumulate, const int* slot, const int* ids,
+                        cudaStream_t s) {
   if (D % 4 == 0 && ldy % 4 == 0 && (((uintptr_t)part | (uintptr_t)y) & 15) == 0)
-    hb_launch(moe_combine_kernel<4>, dim3(ceil_div(D, 1024), n_tokens), dim3(256), 0, s, part, wts, y, ldy, D, top, accumulate, slot);
+    hb_launch(moe_combine_kernel<4>, dim3(ceil_div(D, 1024), n_tokens), dim3(256), 0, s, part, wts, y, ldy, D, E, top, accumulate, slot, ids);
   else
-    hb_launch(moe_combine_kernel<1>, dim3(ceil_div(D, 256), n_tokens), dim3(256), 0, s, part, wts, y, ldy, D, top, accumulate, slot);
+    hb_launch(moe_combine_kernel<1>, dim3(ceil_div(D, 256), n_tokens), dim3(256), 0, s, part, wts, y, ldy, D, E, top, accumulate, slot, ids);
 }
 
 extern "C" long long hb_moe_grouped_scratch_ints(int n_tokens, int E, int top) {
@@ -609,7 +618,7 @@ extern "C" int hb_moe_experts_grouped_bf16(const void* h, int ld, const void* up
             weigh_input ? weights : (const float*)nullptr);
   hb_launch(moe_grouped_gemm_kernel<false>, dim3(max_tiles, ceil_div(D, MG_TN)), dim3(MG_THREADS), 0, s, (const bf16*)mid, F,
             (const bf16*)down, (void*)part, D, (const int*)pair_off, (const int*)tile_off, (const int*)list, E, D, F, top, act, 0, 0.0f, (const float*)nullptr);
-  moe_combine(part, weigh_input ? nullptr : weights, y, ldy, n_tokens, D, top, accumulate, nullptr, s);
+  moe_combine(part, weigh_input ? nullptr : weights, y, ldy, n_tokens, D, E, top, accumulate, nullptr, ids, s);
   HB_CHECK_LAUNCH("moe_experts_grouped");
   return 0;
 }
@@ -634,7 +643,8 @@ moe_sort_padded_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __r
   pdl_launch();
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
-  for (int u = threadIdx.x; u < n_pairs; u += blockDim.x) atomicAdd(&cnt[ids[u]], 1);
+  for (int u = threadIdx.x; u < n_pairs; u += blockDim.x)
+    if ((unsigned)ids[u] < (unsigned)E) atomicAdd(&cnt[ids[u]], 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     int tl = 0;
@@ -651,6 +661,7 @@ moe_sort_padded_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __r
   __syncthreads();
   for (int u = threadIdx.x; u < n_pairs; u += blockDim.x) {
     const int e = ids[u];
+    if ((unsigned)e >= (unsigned)E) { slot[u] = -1; continue; }
     slot[u] = off[e] + atomicAdd(&cnt[e], 1);
     if (row_scale) row_scale[slot[u]] = wts[u];
   }
@@ -661,6 +672,7 @@ __global__ void moe_gather_rows_kernel(const bf16* __restrict__ h, int ld, const
   pdl_wait();
   pdl_launch();
   const int u = blockIdx.x;
+  if (slot[u] < 0) return;
   const uint4* src = reinterpret_cast<const uint4*>(h + (size_t)(u / top) * ld);
   uint4* dst = reinterpret_cast<uint4*>(sorted + (size_t)slot[u] * D8 * 8);
   for (int i = threadIdx.x; i < D8; i += blockDim.x) dst[i] = src[i];
@@ -705,7 +717,7 @@ extern "C" int hb_moe_experts_tc_bf16(const void* h, int ld, const void* up, con
   rc = hb_gemm_tcgen05_grouped_bf16(mid, F, down, F, part, D, rows, D, F, E, HB_EPI_STORE_F32, 0.0f, 0, nullptr, rows_used, tile_expert,
                                     error_flag, stream);
   if (rc) return rc;
-  moe_combine(part, row_scale ? nullptr : weights, y, ldy, n_tokens, D, top, accumulate, slot, s);
+  moe_combine(part, row_scale ? nullptr : weights, y, ldy, n_tokens, D, E, top, accumulate, slot, ids, s);
   HB_CHECK_LAUNCH("moe_experts_tc (combine)");
   return 0;
 }

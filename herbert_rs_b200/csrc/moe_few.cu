@@ -45,7 +45,7 @@ struct FwSorted {
   int pair[FW_MAX_PAIRS];
 };
 
-// Every thread of the CTA; cnt: n_experts ints of shared memory.  An index outside the experts (scores that are not numbers) is left out.
+// Every thread of the CTA; cnt: n_experts ints of shared memory.  An index outside the experts is left out.
 __device__ __forceinline__ void fw_sort(FwSorted& o, int* cnt, const int* __restrict__ ids, int n_pairs, int E, int cap) {
   const int tid = threadIdx.x, lane = tid & 31;
   for (int e = tid; e < E; e += FW_THREADS) cnt[e] = 0;

@@ -106,7 +106,7 @@ _SIGS = {
     "hb_moe_route": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                      c_int, c_int, c_float, c_void_p],
     "hb_moe_experts": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                       c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
+                       c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
     "hb_moe_experts_few_ok": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int],
     "hb_moe_experts_few_bf16": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                 c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
@@ -1020,7 +1020,7 @@ def moe_experts(h, up, down, ids, weights, mid, y, act, accumulate=False, gated=
              1 if accumulate else 0, _stream())
         return
     _run("hb_moe_experts", dtype_code(h.dtype), h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), ids.data_ptr(),
-         weights.data_ptr(), mid.data_ptr(), y.data_ptr(), y.stride(0), h.shape[0], h.shape[1], down.shape[2], ids.shape[1],
+         weights.data_ptr(), mid.data_ptr(), y.data_ptr(), y.stride(0), T, D, E, F, top,
          int(act), int(gated), float(act_limit), 1 if weigh_input else 0, 1 if accumulate else 0, _stream())
 
 

@@ -134,3 +134,45 @@ def test_moe_route_scores_that_are_not_numbers(dtype, T, E, top, groups, keep, s
         assert (ids >= 0).all() and (ids < E).all() and (ids.sort(-1).values.diff(dim=-1) > 0).all()
         assert ((ids == E // 2) == (torch.arange(ids.shape[1], device=DEV) == ids.shape[1] - 1))[(ids == E // 2).any(-1)].all()
         assert groups > 1 or (ids[:, -1] == E // 2).all()
+
+
+@pytest.mark.parametrize("path,dtype,T", [("experts", torch.float32, 9), ("experts", torch.bfloat16, 9), ("experts", torch.bfloat16, 40),
+                                          ("grouped", torch.bfloat16, 300), ("tc", torch.bfloat16, 300)])
+@pytest.mark.parametrize("gated", [0, 2])
+def test_pairs_without_an_expert_contribute_nothing(path, dtype, T, gated):
+    """Indices outside the experts: left out by every kernel, and nothing is written beside the scratch arrays."""
+    E, top, D, F = 7, 3, 136, 72
+    g = torch.Generator(device=DEV).manual_seed(T + gated)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    h, up, down = rnd(T, D).to(dtype), (rnd(E, 2 * F if gated else F, D) / D ** 0.5).to(dtype), (rnd(E, D, F) / F ** 0.5).to(dtype)
+    ids = torch.stack([torch.randperm(E, generator=g, device=DEV)[:top] for _ in range(T)]).int()
+    wts = torch.rand(T, top, generator=g, device=DEV)
+    missing = torch.rand(T, top, generator=g, device=DEV) < 0.3
+    missing[2] = True                               # a token with no expert at all
+    broken = torch.where(missing, torch.tensor([E, -1, 2 ** 30], dtype=torch.int32, device=DEV).expand(T, top), ids)
+    torch.cuda.synchronize()
+
+    def call(ids, wts):
+        y, guards = torch.zeros(T, D, device=DEV), []
+
+        def scratch(shape, dt):
+            n = 1
+            for k in shape:
+                n *= k
+            whole = torch.full((n + 4096,), 77, dtype=dt, device=DEV)
+            whole[2048:2048 + n] = 0
+            guards.append((whole, n))
+            return whole[2048:2048 + n].view(shape)
+        if path == "experts":
+            ops.moe_experts(h, up, down, ids, wts, scratch((T * top, F), dtype), y, ops.ACT_SILU, gated=gated)
+        elif path == "grouped":
+            ops.moe_experts_grouped(h, up, down, ids, wts, y, ops.ACT_SILU, False, scratch, gated=gated)
+        else:
+            ops.moe_experts_tc(h, up, down, ids, wts, y, False, scratch, gated=gated)
+        for whole, n in guards:
+            assert (whole[:2048] == 77).all() and (whole[2048 + n:] == 77).all()
+        return y
+    got, want = call(broken, wts), call(ids, wts.masked_fill(missing, 0.0))
+    # the same products; a weight of 0 adds 0, so only the order of the kept pairs' sums may differ
+    assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+    assert (got[2] == 0).all()
