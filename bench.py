@@ -354,6 +354,11 @@ DESIGN_SIZES = {
 }
 
 
+# launchers that do the same work for different sizes of a step
+EXPERTS = ("hb_moe_experts", "hb_moe_experts_few_bf16", "hb_moe_experts_grouped_bf16", "hb_moe_experts_tc_bf16")
+LATENT_ATTENTION = ("hb_latent_attention", "hb_latent_attention_mma_bf16", "hb_latent_prefill_tc_bf16")
+
+
 def _launcher_work(name, n, ctx):
     """(FLOPs, bytes) that all `n` launches of a launcher do in one step of `ctx` (a dict of the step's
     and the model's sizes), for the launchers compared between the two models; None for the others."""
@@ -362,7 +367,7 @@ def _launcher_work(name, n, ctx):
     es = 2
     if ctx["kind"] == "kebisun":
         H, rk, dr, dn, dv, D = ctx["heads"], ctx["kv_rank"], ctx["rot"], ctx["dim"], ctx["vdim"], ctx["width"]
-        if name in ("hb_latent_attention", "hb_latent_attention_mma_bf16"):
+        if name in LATENT_ATTENTION:
             return n * 2.0 * pairs * H * (2 * rk + dr), n * (B * L * (rk + dr) * es + T * H * (2 * rk + dr) * 4)
         if name == "hb_headwise_gemm":      # two per latent layer: dn -> rk and rk -> dv
             per = n / 2.0
@@ -372,7 +377,7 @@ def _launcher_work(name, n, ctx):
         if name == "hb_gla_scan":
             gh, dk, gv = ctx["gla_heads"], ctx["gla_dk"], ctx["gla_dv"]
             return n * 4.0 * T * gh * dk * gv, n * (T * gh * (3 * dk + 2 * gv) * 4 + 2 * B * gh * dk * gv * 4)
-        if name in ("hb_moe_experts", "hb_moe_experts_grouped_bf16"):
+        if name in EXPERTS:
             E, top, F = ctx["experts"], ctx["top"], ctx["expert_ff"]
             return n * 4.0 * T * top * F * D, n * (min(E, T * top) * 2 * F * D * es + T * D * (es + 4))
     elif ctx["kind"] == "votapel":
@@ -383,7 +388,7 @@ def _launcher_work(name, n, ctx):
             return n * 6.0 * T * D, n * T * D * (4 + 4 + 4 + es)
         if name == "hb_qk_prepare_cache":
             return n * 2.0 * T * (H + KV) * hd, n * T * (H + KV) * hd * (4 + es)
-        if name in ("hb_moe_experts", "hb_moe_experts_grouped_bf16", "hb_moe_experts_tc_bf16"):
+        if name in EXPERTS:
             E, top, F = ctx["experts"], ctx["top"], ctx["expert_ff"]
             return n * 6.0 * T * top * F * D, n * (min(E, T * top) * 3 * F * D * es + T * D * (es + 4))
         if name == "hb_moe_route":
@@ -431,7 +436,7 @@ def _launcher_work(name, n, ctx):
             return n * 6.0 * T * (H + 2 * KV) * hd, n / 2.0 * T * ((2 * H + 2 * KV) * hd * (4 + es))
         if name == "hb_gated_rmsnorm":
             return n * 8.0 * T * dh * dn, n * T * dh * dn * (4 + 4 + es)
-        if name in ("hb_moe_experts", "hb_moe_experts_grouped_bf16", "hb_moe_experts_tc_bf16"):
+        if name in EXPERTS:
             E, top, F = ctx["experts"], ctx["top"], ctx["expert_ff"]
             return n * 6.0 * T * top * F * D, n * (min(E, T * top) * 3 * F * D * es + T * D * (es + 4))
         if name == "hb_moe_route":
@@ -444,7 +449,7 @@ def _launcher_work(name, n, ctx):
         if name in ("hb_attention_prefill_tc_bf16", "hb_attention_prefill_bf16", "hb_attention_decode_bf16", "hb_attention_simt"):
             # two maps per head over one value; the zero channels of a map's query are not counted
             return n * 2.0 * pairs * H * 2 * (dk + dv), n * (B * L * KV * (2 * dk + dv) * es + T * H * (2 * dk + dv) * es)
-        if name in ("hb_latent_attention", "hb_latent_attention_mma_bf16"):
+        if name in LATENT_ATTENTION:
             return n * 2.0 * pairs * lh * (2 * rk + dr), n * (B * L * (rk + dr) * es + T * lh * (2 * rk + dr) * 4)
         if name == "hb_headwise_gemm":
             per = n / 2.0
@@ -493,7 +498,7 @@ def _launcher_work(name, n, ctx):
         if name == "hb_gated_rmsnorm":
             per = n / 2.0
             return per * 8.0 * T * (mh * mv + dh * dw), per * T * (mh * mv + dh * dw) * (4 + 4 + es)
-        if name in ("hb_moe_experts", "hb_moe_experts_grouped_bf16", "hb_moe_experts_tc_bf16"):
+        if name in EXPERTS:
             E, top, F = ctx["experts"], ctx["top"], ctx["expert_ff"]
             return n * 6.0 * T * top * F * D, n * (min(E, T * top) * 3 * F * D * es + T * D * (es + 4))
         if name == "hb_moe_route":
