@@ -75,8 +75,8 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
   const unsigned q_s = base, k_s = q_s + NB * LP_QBLOCK, bars = k_s + NB * LP_KBLOCK;
   const int own0 = half * (LP_HALF / 64), nown = min(LP_HALF, a.rank - half * LP_HALF) >> 6, na = NB - nown;
   auto kfull = [&](int kind) { return bars + kind * 8; };                 // 0: a tile's A-blocks, 1: its own blocks
-  const unsigned a_free = bars + 16, s_full = a_free + 8, p_ready = s_full + 16, o_full = p_ready + 8;
-  volatile unsigned* tmem_slot = reinterpret_cast<volatile unsigned*>(gen + (o_full + 8 - base));
+  const unsigned a_free = bars + 16, s_full = a_free + 8, p_ready = s_full + 16, o_full = p_ready + 8, drained = o_full + 8;
+  volatile unsigned* tmem_slot = reinterpret_cast<volatile unsigned*>(gen + (drained + 8 - base));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) mbar_init(kfull(i), 1);
@@ -85,6 +85,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
     mbar_init(s_full + 8, 1);
     mbar_init(p_ready, 4);
     mbar_init(o_full, 1);
+    mbar_init(drained, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -132,6 +133,7 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
   if (warp == 0) {
     if (lane == 0) {
       const int* pages = a.seq_pages + (size_t)b * a.pages_stride;
+      int sent_a = 0, sent_own = 0;
       for (int j = 0; j < n; ++j) {
         const int key0 = (tile0 + j) * LP_KEYS, lp = key0 / a.page_size;   // page_size is a multiple of 64: a tile lies in one page
         const int row = pages[lp < a.pages_stride ? lp : a.pages_stride - 1] * a.page_size + key0 % a.page_size;
@@ -139,10 +141,15 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
         if (na > 0 && j > 0 && !mbar_wait(a_free, (j - 1) & 1)) { atomicExch(a.error_flag, 41); break; }
         if (na > 0) mbar_expect_tx(kfull(0), na * LP_KBLOCK);
         for (int i = 0; i < na; ++i) fetch(a_block(i), kfull(0));
+        ++sent_a;
         if (j > 0 && !mbar_wait(o_full, (j - 1) & 1)) { atomicExch(a.error_flag, 42); break; }
         mbar_expect_tx(kfull(1), nown * LP_KBLOCK);
         for (int i = 0; i < nown; ++i) fetch(own0 + i, kfull(1));
+        ++sent_own;
       }
+      // no copy is under way when the CTA ends, also after a wait that gave up (here or in another warp)
+      if (na > 0 && sent_a > 0 && !mbar_wait(kfull(0), (sent_a - 1) & 1)) atomicExch(a.error_flag, 48);
+      if (sent_own > 0 && !mbar_wait(kfull(1), (sent_own - 1) & 1)) atomicExch(a.error_flag, 48);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -184,6 +191,9 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
         tc_commit(o_full);
         if (j + 1 < n) own_scores(j + 1);
       }
+      // ... and no product either: the tensor memory is given back and its operands' shared memory ends with the CTA
+      tc_commit(drained);
+      if (!mbar_wait(drained, 0)) atomicExch(a.error_flag, 49);
     }
   } else if (warp < 6) {
     const int quad = warp & 3, r = quad * 32 + lane, row = r0 + r;         // a warp reads the tensor memory lanes of its quadrant
