@@ -266,10 +266,10 @@ headwise_mma_kernel(const float* __restrict__ in, int ld_in, int in_hs, const bf
 // a head 70 -> 41 us, 512 -> 128 with gates 107 -> 79 us.
 #define HL_T 128
 template <typename TO>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 headwise_mma_wide_kernel(const float* __restrict__ in, int ld_in, int in_hs, const bf16* __restrict__ w, TO* __restrict__ out,
                          int ld_out, int out_hs, const float* __restrict__ gate, int ld_gate, int n_tokens, int K, int N,
-                         float scale, int pairs) {
+                         float scale, int pairs, int gate_pairs) {
   __shared__ __align__(16) bf16 As[2][HL_T][HM_TK + 8];
   __shared__ __align__(16) bf16 Ws[2][HL_T][HM_TK + 8];
   pdl_wait();
@@ -351,6 +351,21 @@ headwise_mma_wide_kernel(const float* __restrict__ in, int ld_in, int in_hs, con
       if (tk >= n_tokens) continue;
       const float* gr = gate ? gate + (size_t)tk * ld_gate + (size_t)h * N : nullptr;
       TO* o = out + (size_t)tk * ld_out + (size_t)h * out_hs;
+      float gv[8][2];                                              // a row's gates, asked for together
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        const int n = n0 + wn + nt * 8 + 2 * t;
+        gv[nt][0] = gv[nt][1] = 0.0f;
+        if (gr && gate_pairs && n < N) {                           // N is even
+          const float2 x = *reinterpret_cast<const float2*>(gr + n);
+          gv[nt][0] = x.x;
+          gv[nt][1] = x.y;
+        } else if (gr) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+            if (n + c < N) gv[nt][c] = gr[n + c];
+        }
+      }
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) {
         const int n = n0 + wn + nt * 8 + 2 * t;
@@ -358,7 +373,7 @@ headwise_mma_wide_kernel(const float* __restrict__ in, int ld_in, int in_hs, con
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           v[c] = acc[m][nt][half * 2 + c] * scale;
-          if (gr && n + c < N) v[c] *= 1.0f / (1.0f + expf(-gr[n + c]));
+          if (gr) v[c] *= 1.0f / (1.0f + expf(-gv[nt][c]));
         }
         if (pairs && n + 1 < N) {
           if constexpr (sizeof(TO) == 4) *reinterpret_cast<float2*>(o + n) = make_float2(v[0], v[1]);
@@ -386,12 +401,13 @@ extern "C" int hb_headwise_gemm(int dtype, int out_dtype, const float* in, int l
     if (n_tokens >= HL_T && N >= HL_T) {
       const dim3 grid(ceil_div(n_tokens, HL_T), heads, ceil_div(N, HL_T));
       const int pairs = ld_out % 2 == 0 && out_head_stride % 2 == 0 && ((uintptr_t)out & 7) == 0;
+      const int gate_pairs = N % 2 == 0 && ld_gate % 2 == 0 && ((uintptr_t)gate & 7) == 0;
       if (out_dtype == HB_F32)
         hb_launch(headwise_mma_wide_kernel<float>, grid, dim3(256), 0, s, in, ld_in, in_head_stride, (const bf16*)w, (float*)out, ld_out,
-                  out_head_stride, gate, ld_gate, n_tokens, K, N, scale, pairs);
+                  out_head_stride, gate, ld_gate, n_tokens, K, N, scale, pairs, gate_pairs);
       else
         hb_launch(headwise_mma_wide_kernel<bf16>, grid, dim3(256), 0, s, in, ld_in, in_head_stride, (const bf16*)w, (bf16*)out, ld_out,
-                  out_head_stride, gate, ld_gate, n_tokens, K, N, scale, pairs);
+                  out_head_stride, gate, ld_gate, n_tokens, K, N, scale, pairs, gate_pairs);
       HB_CHECK_LAUNCH("headwise_gemm");
       return 0;
     }
