@@ -249,10 +249,8 @@ extern "C" int hb_attention_simt(int dtype, const void* q, int ldq, void* out, i
   } while (0)
 #define AS_SIZE(T)                                                                        \
   do {                                                                                    \
-    if (!v4) AS_GO(T, 512, 1);                                                            \
-    else if (hd <= 128) AS_GO(T, 128, 4);                                                 \
-    else if (hd <= 256) AS_GO(T, 256, 4);                                                 \
-    else AS_GO(T, 512, 4);                                                                \
+    if (v4) { if (hd <= 128) AS_GO(T, 128, 4); else if (hd <= 256) AS_GO(T, 256, 4); else AS_GO(T, 512, 4); } \
+    else { if (hd <= 128) AS_GO(T, 128, 1); else if (hd <= 256) AS_GO(T, 256, 1); else AS_GO(T, 512, 1); }    \
   } while (0)
   if (dtype == HB_F32) AS_SIZE(float); else AS_SIZE(bf16);
 #undef AS_SIZE
