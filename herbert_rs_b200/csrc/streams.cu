@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(512) streams_kernel(JoinArgs a) {
 }
 
 // The same with u in registers too: up to four copies of rows of D <= 4,096 floats, D a multiple of 128, four columns a
-// thread.  Everything is asked for before the first sum, the small weights included, and a sum costs one barrier (row_norm.cuh).
+// thread (see streams_launch for when).  Everything is asked for before the first sum, the small weights included, and a sum costs one barrier (row_norm.cuh).
 // Bound by the copies' bytes.  Measured on a B200, 4,731 rows of four copies of 2,048, inside a step: 78 -> 66 us (368 MB).
 template <typename T, int NS>
 __global__ void __launch_bounds__(1024) streams_row_kernel(JoinArgs a) {
@@ -185,7 +185,14 @@ template <typename T, int NS>
 static int streams_launch(const JoinArgs& a, int n_rows, bool vec, cudaStream_t s) {
   if constexpr (NS <= 4) {
     const uintptr_t small = (uintptr_t)(a.h ? a.w : nullptr) | (uintptr_t)(a.h ? a.bias : nullptr);
-    if (vec && a.D % 128 == 0 && a.D <= 4096 && (small & 15) == 0) {
+    // Wide rows leave one CTA of up to 1,024 threads an SM: beyond `widest` columns the kernel above is the faster one as soon as there
+    // is more than one row an SM (this one and that one, us: four copies of 4,096, 148 rows 6.0 and 6.4, 450 rows 15.7 and 12.8; 5,000
+    // rows of one copy of 3,072 52.8 and 47.6, of two of 2,560 47.0 and 61.4, of four of 2,560 103.6 and 99.5).
+    constexpr int widest = NS == 2 ? 3072 : NS == 4 ? 2048 : 2560;
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (vec && a.D % 128 == 0 && (a.D <= widest || (a.D <= 4096 && n_rows <= sms)) && (small & 15) == 0) {
       hb_launch(streams_row_kernel<T, NS>, dim3(n_rows), dim3(a.D / 4), 0, s, a);
       HB_CHECK_LAUNCH("streams_join");
       return 0;

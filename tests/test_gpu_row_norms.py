@@ -71,3 +71,22 @@ def test_row_norms(D, rows, dtype):
         i, p = int(ids[t]), int(at[t])
         ref = table[i].float() * 1.5 + (pos[p].float() if p < 4 else 0.0) if 0 <= i < 9 else torch.zeros(D, device=DEV)
         _near(out[t], ref.double().expand(2, D), torch.float32)
+
+
+@pytest.mark.parametrize("n,D", [(1, 128), (1, 2688), (2, 256), (2, 3200), (3, 384), (3, 2560), (4, 2048), (4, 2176), (4, 4096), (4, 132), (5, 256)])
+@pytest.mark.parametrize("rows", [1, 148, 149, 300])
+@pytest.mark.parametrize("rms", [False, True])
+def test_copies_of_the_stream(n, D, rows, rms):
+    """One to four copies a row in registers and beside it: the narrowest and widest rows, and the rows an SM where wide ones change."""
+    g = torch.Generator(device=DEV).manual_seed(n * D + rows)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    x0, y, mix, ow, iw, w, bias = rnd(rows, n, D), rnd(rows, D), rnd(n, n) * 0.5, rnd(n), rnd(n), rnd(D), rnd(D)
+    x, h = x0.clone(), torch.empty(rows, D, device=DEV)
+    ops.streams_join(x, y, mix, ow, iw, norm=(w, bias, 1e-5, rms), h=h)
+    ref = torch.einsum("st,rsd->rtd", mix.double(), x0.double()) + ow.double()[:, None] * y.double()[:, None]
+    _near(x, ref, torch.float32)
+    u = torch.einsum("t,rtd->rd", iw.double(), ref)
+    mean = 0.0 if rms else u.mean(-1, keepdim=True)
+    want = (u - mean) / ((u - mean).pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * w.double() + bias.double()
+    # the norm divides by the spread of u: its float error is that of u over it, a few roundings of the largest of n + 1 terms
+    assert float((h.double() - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
