@@ -23,6 +23,7 @@
 // A pair whose index lies outside the experts contributes nothing, in every kernel of the feed-forward alike (the router gives none).
 #include "api.h"
 #include "common.cuh"
+#include "mma_utils.cuh"
 #include "moe_act.cuh"
 
 #define MOE_WARPS 4
@@ -165,7 +166,8 @@ moe_route_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr, int*
 // The same where rows are 16-byte pieces: a CTA of W warps takes TT tokens, whose inputs it keeps in shared memory, a warp two
 // experts at a time, so that a weight row is read once per TT tokens and an input piece is widened once per two experts.  The
 // 2 TT sums of the 32 lanes are added with halving exchanges; then a warp per token chooses.
-// Measured on a B200, 32 experts over 2,048 numbers, inside a step: 8 tokens 13 -> 7 us, 3,600 tokens 73 -> 38 us.
+// Bound by ways to memory and back: the tokens' inputs are copied all at once and a batch of four pieces of both weight rows is asked
+// for before the first is used (a piece at a time, eight tokens a CTA took 28 us for 600 tokens and 32 experts over 2,048, now 12).
 __device__ __forceinline__ void moe_widen(const uint4& u, float* v, const float*) {
   v[0] = __uint_as_float(u.x); v[1] = __uint_as_float(u.y); v[2] = __uint_as_float(u.z); v[3] = __uint_as_float(u.w);
 }
@@ -182,7 +184,7 @@ template <typename T, int TT, int W>
 __global__ void __launch_bounds__(W * 32)
 moe_route_tile_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr, int* __restrict__ ids, float* __restrict__ wts,
                       int n_tokens, int D, int E, int top, int renorm, int sigmoid, int groups, int keep, int group_top, float wscale) {
-  constexpr int VE = 16 / (int)sizeof(T), N = 2 * TT;
+  constexpr int VE = 16 / (int)sizeof(T), N = 2 * TT, B = 4;
   static_assert(TT <= W, "a warp per token chooses");
   extern __shared__ __align__(16) unsigned char raw[];  // [TT][D] inputs, [TT][E] scores, [TT][groups] group scores
   uint4* hs = reinterpret_cast<uint4*>(raw);
@@ -193,9 +195,12 @@ moe_route_tile_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr,
   pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = blockIdx.x * TT;
   const int nt = n_tokens - t0 < TT ? n_tokens - t0 : TT;
-  for (int tt = 0; tt < TT; ++tt)
-    for (int i = threadIdx.x; i < pieces; i += W * 32)
-      hs[tt * pieces + i] = reinterpret_cast<const uint4*>(h + (size_t)(t0 + (tt < nt ? tt : nt - 1)) * ld)[i];
+  for (int i = threadIdx.x; i < TT * pieces; i += W * 32) {      // all of them on their way before the first is waited for
+    const int tt = TT == 1 ? 0 : i / pieces;
+    cp_async16(hs + i, h + (size_t)(t0 + (tt < nt ? tt : nt - 1)) * ld + (size_t)(i - tt * pieces) * VE);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
   __syncthreads();
   for (int e0 = 2 * warp; e0 < E; e0 += 2 * W) {
     const uint4* w0 = reinterpret_cast<const uint4*>(wr + (size_t)e0 * D);
@@ -203,19 +208,30 @@ moe_route_tile_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr,
     float acc[N];                                       // [expert][token]
 #pragma unroll
     for (int i = 0; i < N; ++i) acc[i] = 0.0f;
-#pragma unroll(TT == 1 ? 4 : 1)
-    for (int i = lane; i < pieces; i += 32) {
-      float a[VE], b[VE];
-      moe_widen(w0[i], a, h);
-      moe_widen(w1[i], b, h);
+    for (int i0 = lane; i0 < pieces; i0 += 32 * B) {
+      uint4 u0[B], u1[B];                               // a batch of both rows' pieces, asked for together
 #pragma unroll
-      for (int tt = 0; tt < TT; ++tt) {
-        float x[VE];
-        moe_widen(hs[tt * pieces + i], x, h);
+      for (int q = 0; q < B; ++q) {
+        const int i = i0 + 32 * q;
+        u0[q] = u1[q] = make_uint4(0, 0, 0, 0);
+        if (i < pieces) { u0[q] = w0[i]; u1[q] = w1[i]; }
+      }
 #pragma unroll
-        for (int j = 0; j < VE; ++j) {
-          acc[tt] = fmaf(x[j], a[j], acc[tt]);
-          acc[TT + tt] = fmaf(x[j], b[j], acc[TT + tt]);
+      for (int q = 0; q < B; ++q) {
+        const int i = i0 + 32 * q;
+        if (i >= pieces) break;
+        float a[VE], b[VE];
+        moe_widen(u0[q], a, h);
+        moe_widen(u1[q], b, h);
+#pragma unroll
+        for (int tt = 0; tt < TT; ++tt) {
+          float x[VE];
+          moe_widen(hs[tt * pieces + i], x, h);
+#pragma unroll
+          for (int j = 0; j < VE; ++j) {
+            acc[tt] = fmaf(x[j], a[j], acc[tt]);
+            acc[TT + tt] = fmaf(x[j], b[j], acc[TT + tt]);
+          }
         }
       }
     }
@@ -250,26 +266,38 @@ extern "C" int hb_moe_route(int dtype, const void* h, int ld, const void* w_rout
   const size_t smem = (size_t)(E + groups) * sizeof(float);
   HB_REQUIRE(smem <= 48 * 1024, "moe_route: %d experts exceed what a block keeps in shared memory", E);
   dim3 grid(n_tokens);
-  // Eight tokens a CTA once that gives half of the SMs one; one token a CTA of 16 warps for fewer (a decode step).
+  // Tokens a CTA and its warps: one token and sixteen warps while the tokens are at most one an SM, four (two, of at most 16 experts) up to
+  // four an SM, then eight.  Eight experts give every warp of the one-token kernel one: it is the faster one until its CTAs take a second
+  // round.  us of the one-token kernel and of this one, bfloat16, experts over columns: 32 over 2,048 at 16, 440, 1,200 and 3,600 tokens 9 / 6,
+  // 10 / 9, 21 / 18, 50 / 34; 128 over 2,048 24 / 13, 27 / 22, 71 / 55, 175 / 104; 16 over 1,024 4.7 / 4.2, 5.0 / 4.9, 9.2 / 7.0, 20 / 12; 8 over 1,024
+  // 3.9 / 4.1, 4.2 / 4.4, 7.1 / 5.8, 16 / 10.
   const int es = dtype == HB_F32 ? 4 : 2;
   const bool rows16 = (D * es) % 16 == 0 && ((long long)ld * es) % 16 == 0 && (((uintptr_t)h | (uintptr_t)w_router) & 15) == 0;
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   auto need = [&](int tt) { return (size_t)tt * ((size_t)D * es + (size_t)(E + groups) * sizeof(float)); };
-  const int tt = n_tokens >= 4 * sms && need(8) <= 100 * 1024 ? 8 : 1;
-  if (rows16 && need(tt) <= 100 * 1024) {
+  const size_t most = 100 * 1024;
+  int tt = 0;
+  if (E > MOE_ROUTE_WARPS || n_tokens > 5 * sms)
+    tt = n_tokens <= sms ? 1 : n_tokens < 4 * sms ? (E > 16 ? 4 : 2) : need(8) <= most ? 8 : 4;
+  if (rows16 && tt > 0 && need(tt) <= most) {
+    const bool wide = n_tokens < 4 * sms;         // four tokens: sixteen warps, else eight
 #define MR_GO(T, TT, W)                                                                                                                        \
   do {                                                                                                                                         \
     if (need(TT) > 48 * 1024) cudaFuncSetAttribute(moe_route_tile_kernel<T, TT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(TT)); \
     hb_launch(moe_route_tile_kernel<T, TT, W>, dim3(ceil_div(n_tokens, TT)), dim3(W * 32), need(TT), (cudaStream_t)stream, (const T*)h, ld,      \
               (const T*)w_router, ids, weights, n_tokens, D, E, top, renorm, sigmoid, groups, keep, group_top, wscale);                         \
   } while (0)
-    if (dtype == HB_F32) {
-      if (tt == 8) MR_GO(float, 8, 8); else MR_GO(float, 1, 16);
-    } else {
-      if (tt == 8) MR_GO(bf16, 8, 8); else MR_GO(bf16, 1, 16);
-    }
+#define MR_SIZE(T)                                                                                                  \
+  do {                                                                                                              \
+    if (tt == 8) MR_GO(T, 8, 8);                                                                                    \
+    else if (tt == 4) { if (wide) MR_GO(T, 4, 16); else MR_GO(T, 4, 8); }                                           \
+    else if (tt == 2) MR_GO(T, 2, 8);                                                                               \
+    else MR_GO(T, 1, 16);                                                                                           \
+  } while (0)
+    if (dtype == HB_F32) MR_SIZE(float); else MR_SIZE(bf16);
+#undef MR_SIZE
 #undef MR_GO
     HB_CHECK_LAUNCH("moe_route");
     return 0;
@@ -366,7 +394,6 @@ extern "C" int hb_moe_experts(int dtype, const void* h, int ld, const void* up, 
 //   combine:        y[t] (+)= sum_r weights[t, r] * part[t * top + r]
 // Which place a pair gets inside its expert's list depends on the order in which threads arrive; a
 // pair's own numbers do not depend on its place, so the result is the same bits every time.
-#include "mma_utils.cuh"
 
 #define MG_TM 128
 #define MG_TN 128

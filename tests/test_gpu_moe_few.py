@@ -101,6 +101,14 @@ def test_moe_route_tiles(dtype, T, E, top, groups, keep, D):
     assert float((wts.double() - 1.5 * got / got.sum(-1, keepdim=True)).abs().max()) < 2e-5
 
 
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 20), (torch.bfloat16, 264), (torch.float32, 4096), (torch.bfloat16, 8192)])
+@pytest.mark.parametrize("T", [148, 149, 591, 592, 741])
+@pytest.mark.parametrize("E,top,groups,keep", [(8, 2, 1, 1), (9, 3, 3, 2), (16, 4, 4, 2), (17, 2, 1, 1)])
+def test_moe_route_tokens_a_block(dtype, D, T, E, top, groups, keep):
+    """One, two, four and eight tokens a block, at the token and expert counts where they change."""
+    test_moe_route_tiles(dtype, T, E, top, groups, keep, D)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T", [3, 1201])
 @pytest.mark.parametrize("E,top,groups,keep,score", [(32, 4, 8, 4, 1), (32, 4, 1, 1, 0), (15, 15, 3, 3, 0), (16, 2, 4, 1, 1), (6, 2, 1, 1, 1)])
