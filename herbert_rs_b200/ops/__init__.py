@@ -963,6 +963,19 @@ def moe_tc_ok(h, up, top, gated, act) -> bool:
             and h.shape[0] * int(top) >= MOE_TC_MIN_PAIRS)
 
 
+def moe_few_pays(tokens, top, experts, D, F, gated) -> bool:
+    """Whether a step of few tokens gains by reading every chosen expert once for all its tokens.  The kernels that do so sort the
+    step's pairs first, about 5 us; what they save are the matrices that several tokens choose, less where the choices spread (the
+    sum below takes them as drawn evenly).  Measured with matrices that come from memory, us a call with a warp per output number
+    and with them: 4 of 32 plain experts of 1,408 over 2,048 at 1, 2, 4, 8, 16 tokens 18 / 19, 24 / 26, 41 / 37, 61 / 52, 105 / 69; 2 of 16
+    of 768 over 1,024 at 4, 8, 12, 31 tokens 12 / 16, 18 / 18, 22 / 21, 41 / 25; 6 of 64 of 1,024 over 4,096 at 2, 8, 16 tokens 41 / 45,
+    109 / 109, 198 / 156; one of 4 of 128 over 256 at 1 and 31 tokens 4 / 9, 6 / 16."""
+    pairs = tokens * top
+    saved = pairs - experts * (1.0 - (1.0 - min(top, experts) / experts) ** tokens)
+    matrices = (3 if gated else 2) * D * F * 2
+    return saved >= 1.0 and (saved + pairs / 8) * matrices >= 32e6
+
+
 def moe_experts_tc(h, up, down, ids, weights, y, accumulate, scratch, act_limit=0.0, weigh_input=False, gated=GATED_GROUPS_OF_8,
                    act=ACT_SILU) -> None:
     """moe_experts for long prompts, gated experts with silu (or, with act_limit > 0, the clamped activation) or plain ones (gated 0) with `act`: the pairs
@@ -1011,9 +1024,10 @@ def moe_experts(h, up, down, ids, weights, mid, y, act, accumulate=False, gated=
     _check(h, None, "h"); _check(up, h.dtype, "up"); _check(down, h.dtype, "down"); _check(mid, h.dtype, "mid"); _check(y, torch.float32, "y")
     if not (up.is_contiguous() and down.is_contiguous() and mid.is_contiguous()):
         raise BackendError("moe_experts: up, down and mid must be contiguous")
-    # bfloat16 steps of up to 32 tokens read every chosen expert once for all its tokens; the rest a warp per output number
+    # bfloat16 steps of up to 32 tokens that share experts read every chosen expert once for all its tokens; the rest a warp per output number
     T, top, E, D, F = h.shape[0], ids.shape[1], up.shape[0], h.shape[1], down.shape[2]
-    if h.dtype == torch.bfloat16 and _fn("hb_moe_experts_few_ok")(h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), mid.data_ptr(),
+    few = options.moe_few == "always" or (options.moe_few == "auto" and moe_few_pays(T, top, E, D, F, gated))
+    if few and h.dtype == torch.bfloat16 and _fn("hb_moe_experts_few_ok")(h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), mid.data_ptr(),
                                                                   T, top, E, D, F, int(gated)):
         _run("hb_moe_experts_few_bf16", h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), ids.data_ptr(), weights.data_ptr(),
              mid.data_ptr(), y.data_ptr(), y.stride(0), T, D, E, F, top, int(act), int(gated), float(act_limit), 1 if weigh_input else 0,

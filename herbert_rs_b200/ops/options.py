@@ -39,6 +39,9 @@ class KernelOptions:
     latent_attention: str = "mma"
     # ... whose rows' keys are cut into at most this many ranges when a step has too few rows to fill the GPU.
     latent_max_splits: int = 16
+    # Routed feed-forward, bfloat16, steps of up to 32 tokens: every chosen expert read once for all its tokens where that pays ("auto"; see
+    # ops.moe_few_pays), "always" or "never" (a warp per output number).
+    moe_few: str = "auto"
     # Routed feed-forward, bfloat16, steps of 32 tokens and more: pairs grouped by expert, tiles on the tensor cores.
     moe_grouped: bool = True
     # ... and, for gated experts with silu and 512 (token, expert) pairs or more, those tiles on tcgen05.

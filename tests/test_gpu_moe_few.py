@@ -47,6 +47,19 @@ def test_moe_few(T, top, E, D, F, gated, weigh_input, accumulate, twice):
     assert ((y.double() - want).abs() <= size * 2.0 ** -8 + 1e-5).all()
 
 
+@pytest.mark.parametrize("T,top,E", [(1, 1, 1), (1, 4, 32), (2, 3, 40), (8, 4, 32), (9, 2, 5), (16, 4, 33), (31, 2, 2), (32, 4, 100)])
+@pytest.mark.parametrize("D,F", [(8, 8), (72, 40), (2048, 1408), (520, 264)])
+@pytest.mark.parametrize("gated,weigh_input,accumulate,twice", [(0, False, True, False), (2, False, False, True), (2, True, True, False)])
+@pytest.mark.parametrize("few", ["always", "never"])
+def test_moe_few_by_choice(T, top, E, D, F, gated, weigh_input, accumulate, twice, few):
+    """The same at every size with the experts read once for all tokens, and with a warp per output number."""
+    saved, ops.options.moe_few = ops.options.moe_few, few
+    try:
+        test_moe_few(T, top, E, D, F, gated, weigh_input, accumulate, twice)
+    finally:
+        ops.options.moe_few = saved
+
+
 @pytest.mark.parametrize("act", [ops.ACT_GELU, ops.ACT_SILU, ops.ACT_GELU_TANH])
 @pytest.mark.parametrize("T,top,E,D,F", [(300, 2, 5, 136, 72), (130, 4, 16, 264, 392), (700, 1, 3, 512, 128)])
 def test_moe_tc_plain_experts(act, T, top, E, D, F):
