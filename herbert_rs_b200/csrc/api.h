@@ -130,8 +130,8 @@ int hb_gemm_tcgen05_norm_bf16(const void* A, int lda, const void* W, int ldw, vo
 int hb_gla_decay(int dtype, const float* low, int ld, const void* w2, const float* bias, float inv_tau, float* a,
     int n_tokens, int channels, int low_rank, void* stream);
 int hb_gla_scan(const float* proj, int ld, int q_off, int k_off, int v_off, const float* decay, float* state,
-    const int* seq_slot, const int* seq_start, float* out, int ldo, int n_seqs, int heads, int dk, int dv, float
-    qscale, void* stream);
+    const int* seq_slot, const int* seq_start, float* out, int ldo, int n_seqs, int n_tokens, int heads, int dk,
+    int dv, float qscale, void* stream);
 int hb_gla_output(int dtype, const float* o, int ldo, const float* w, float eps, const float* gate, int ldg,
     void* y, int ldy, int n_tokens, int heads, int dv, void* stream);
 

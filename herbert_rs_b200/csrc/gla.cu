@@ -66,7 +66,7 @@ extern "C" int hb_gla_decay(int dtype, const float* low, int ld, const void* w2,
 }
 
 // ---------------------------------------------------------------------------------------------
-// The recurrence for the sizes that scan_rows.cuh does not take.  A block owns COLS (32, 16 or 8) value channels of one head of one sequence and walks
+// The recurrence for short steps, and for the sizes that scan_rows.cuh does not take.  A block owns COLS (32, 16 or 8) value channels of one head of one sequence and walks
 // that sequence's tokens of the step in order; thread (x, y) keeps RPT consecutive state rows of column x
 // in registers, 128 / COLS groups of rows side by side (narrower blocks when a step has few sequences and
 // heads, so that one long prompt still spreads over the GPU).  q, k, v and the decays of `chunk` tokens at a time are copied into shared memory
@@ -192,10 +192,11 @@ gla_scan_kernel(const float* __restrict__ proj, int ld, int q_off, int k_off, in
   }
 }
 
+// n_tokens: the tokens of all sequences of the step (it chooses the kernel, nothing else).
 extern "C" int hb_gla_scan(const float* proj, int ld, int q_off, int k_off, int v_off, const float* decay, float* state,
-                           const int* seq_slot, const int* seq_start, float* out, int ldo, int n_seqs, int heads, int dk,
-                           int dv, float qscale, void* stream) {
-  HB_REQUIRE(n_seqs > 0 && heads > 0 && dk > 0 && dv > 0, "gla_scan: sizes must be positive");
+                           const int* seq_slot, const int* seq_start, float* out, int ldo, int n_seqs, int n_tokens, int heads,
+                           int dk, int dv, float qscale, void* stream) {
+  HB_REQUIRE(n_seqs > 0 && n_tokens >= 0 && heads > 0 && dk > 0 && dv > 0, "gla_scan: sizes must be positive");
   HB_REQUIRE(dk <= 16 * 64, "gla_scan: %d key channels per head exceed the supported maximum 1024", dk);
   HB_REQUIRE(heads <= 65535 && ceil_div(dv, 8) <= 65535, "gla_scan: too many heads or value channels");
   cudaStream_t s = (cudaStream_t)stream;
@@ -204,15 +205,22 @@ extern "C" int hb_gla_scan(const float* proj, int ld, int q_off, int k_off, int 
   sr.ldvec[0] = sr.ldvec[1] = ld; sr.ldvec[2] = (long long)heads * dk;
   sr.v = proj + v_off; sr.ldv = ld; sr.state = state; sr.seq_slot = seq_slot; sr.seq_start = seq_start; sr.out = out; sr.ldo = ldo;
   sr.H = heads; sr.G = heads; sr.dv = dv; sr.scale = qscale;
-  if (scan_rows<SCAN_GLA>(sr, n_seqs, dk, s)) {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // scan_rows.cuh walks tokens faster but reads and writes a state row in pieces of 8 or 16 bytes, and its CTAs own 2,048 / dk columns or
+  // more: for sequences of dk / 4 tokens on average (the state's way then counts little) and about a CTA an SM.  us of the kernel above
+  // and of that one: 4 heads of 256 x 512, 4 and 16 sequences of one token 6 / 9 and 19 / 28, of 64 tokens 41 / 44 and 158 / 147, 1,500, 800, 300
+  // and 73 tokens 857 / 430; 4 heads of 128 x 256, 8 sequences of one token 4.3 / 4.6, of 32 15 / 12, one of 600 (64 CTAs) 78 / 92;
+  // 16 heads of 64 x 64, two sequences of 600 (64 CTAs) 64 / 77, four 87 / 77.
+  const bool long_enough = 4LL * n_tokens >= (long long)dk * n_seqs;
+  const bool enough_ctas = 6LL * n_seqs * heads * ceil_div_ll((long long)dv * dk, 2048) >= 5LL * sms;
+  if (long_enough && enough_ctas && scan_rows<SCAN_GLA>(sr, n_seqs, dk, s)) {
     HB_CHECK_LAUNCH("gla_scan");
     return 0;
   }
   const int wide = dk % 4 == 0 && ld % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && (((uintptr_t)proj | (uintptr_t)decay) & 15) == 0;
   // the widest blocks that still give every SM one (a long prompt alone: narrower blocks, more of them)
-  int sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int cols = dk > 512 ? 8 : dk > 256 ? 16 : 32;                    // at most 64 state rows per thread
   while (cols > 8 && (long long)n_seqs * heads * ceil_div(dv, cols) < sms) cols >>= 1;
   const int groups = GLA_THREADS / cols;

@@ -100,7 +100,7 @@ _SIGS = {
                                   c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "hb_gla_decay": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
     "hb_gla_scan": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                    c_int, c_int, c_int, c_float, c_void_p],
+                    c_int, c_int, c_int, c_int, c_float, c_void_p],
     "hb_gla_output": [c_int, c_void_p, c_int, c_void_p, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                       c_void_p],
     "hb_moe_route": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -529,7 +529,7 @@ def gla_scan(proj, q_off, k_off, v_off, decay, state, seq_slot, seq_start, out, 
     if not (state.is_contiguous() and decay.is_contiguous()):
         raise BackendError("gla_scan: state and decay must be contiguous")
     _run("hb_gla_scan", proj.data_ptr(), proj.stride(0), int(q_off), int(k_off), int(v_off), decay.data_ptr(), state.data_ptr(),
-         seq_slot.data_ptr(), seq_start.data_ptr(), out.data_ptr(), out.stride(0), int(n_seqs), int(heads), int(dk), int(dv),
+         seq_slot.data_ptr(), seq_start.data_ptr(), out.data_ptr(), out.stride(0), int(n_seqs), out.shape[0], int(heads), int(dk), int(dv),
          float(qscale), _stream())
 
 

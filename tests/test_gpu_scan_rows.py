@@ -78,3 +78,22 @@ def _check(kind, lens, H, G, dk, dv):
 @pytest.mark.parametrize("lens,H,G,dv", [([1, 1], 2, 1, 36), ([7, 8, 9, 1], 3, 3, 4), ([17], 16, 8, 128), ([33, 1, 16], 8, 4, 260), ([5] * 40, 4, 4, 132), ([3], 2, 2, 33)])
 def test_scan_rows(kind, dk, lens, H, G, dv):
     _check(kind, lens, H, H if kind in ("gla", "general") else G, dk, dv)
+
+
+@pytest.mark.parametrize("kind", ["gla", "decay", "delta", "general"])
+@pytest.mark.parametrize("dk", [64, 128, 256])
+@pytest.mark.parametrize("shape", ["many", "few"])
+def test_scan_rows_over_several_chunks(kind, dk, shape):
+    """Sequences of several chunks and a rest, four columns a thread (many CTAs) and two (about one an SM)."""
+    if shape == "many":
+        _check(kind, [33, 80, 97, 64, 65] * 5, 4, 4, dk, 260)
+    else:
+        _check(kind, [70, 65, 64], 16, 16 if kind in ("gla", "general") else 8, dk, (8448 // dk + 3) // 4 * 4)
+
+
+@pytest.mark.parametrize("dk", [64, 128, 256])
+@pytest.mark.parametrize("less", [0, 1])
+def test_gla_scan_around_the_length_where_its_kernel_changes(dk, less):
+    """dk / 4 tokens a sequence on average, and one token less."""
+    n = dk // 4
+    _check("gla", [n + 3, n - 3, n, n - less, 2 * n - 1, 1] * 2, 8, 8, dk, 132)
