@@ -705,9 +705,9 @@ __global__ void moe_gather_rows_kernel(const bf16* __restrict__ h, int ld, const
   for (int i = threadIdx.x; i < D8; i += blockDim.x) dst[i] = src[i];
 }
 
-// Rows of the sorted, padded buffers for n_tokens * top pairs of E experts.
+// Rows of the sorted, padded buffers for n_tokens * top pairs of E experts: m experts with a pair have at most (pairs + 127 m) / 128 tiles.
 extern "C" int hb_moe_experts_tc_rows(int n_tokens, int E, int top) {
-  const long long tiles = ((long long)n_tokens * top + 127) / 128 + E;
+  const long long pairs = (long long)n_tokens * top, tiles = (pairs + 127LL * (pairs < E ? pairs : E)) / 128;
   return tiles * 128 > 2147483647LL ? -1 : (int)(tiles * 128);
 }
 

@@ -957,10 +957,20 @@ def moe_grouped_ok(h, up, gated=0) -> bool:
 def moe_tc_ok(h, up, top, gated, act) -> bool:
     """Whether the grouped products run on tcgen05: what `moe_grouped_ok` asks, gated experts with silu or the clamped
     activation, or plain ones with silu or a gelu (the product's epilogues), and enough (token, expert) pairs that tiles of
-    128 rows per expert fill (2,673 tokens, 4 of 32 plain experts of 1,408 over 2,048: the two products 185 us against 574 on mma.sync)."""
+    128 rows per expert fill (plain experts, us on mma.sync and on tcgen05 with sort and sum: 4 of 32 of 1,408 over 2,048 at 512, 2,048
+    and 16,384 pairs 208 / 118, 242 / 120, 865 / 322; 8 of 512 of 512 over 1,024 at 512 and 8,192 502 / 282, 784 / 425; one of 3 of 128
+    over 512 at 512 and 16,384 35 / 24, 86 / 81).  Padding takes up to 127 rows an expert of the workspace, which the list of pairs on
+    mma.sync does without: plain experts keep that one where the padded arrays would be both more than eight times the pairs and
+    more than half of the experts' matrices."""
     acts = (ACT_SILU, ACT_SWISH_CLAMP) if gated else (ACT_SILU, ACT_GELU, ACT_GELU_TANH)
-    return (options.moe_tc and moe_grouped_ok(h, up, gated) and gated in (0, GATED_GROUPS_OF_8) and act in acts
-            and h.shape[0] * int(top) >= MOE_TC_MIN_PAIRS)
+    pairs = h.shape[0] * int(top)
+    if not (options.moe_tc and moe_grouped_ok(h, up, gated) and gated in (0, GATED_GROUPS_OF_8) and act in acts and pairs >= MOE_TC_MIN_PAIRS):
+        return False
+    if gated:
+        return True
+    E, F, D = up.shape
+    rows = int(_fn("hb_moe_experts_tc_rows")(h.shape[0], E, int(top)))
+    return 0 < rows and (rows <= 8 * pairs or rows * (6 * D + 2 * F) * 2 <= 4 * E * D * F)
 
 
 def moe_few_pays(tokens, top, experts, D, F, gated) -> bool:
