@@ -468,8 +468,13 @@ def headwise_gemm(src, src_head_stride, w, out, out_head_stride, scale=1.0, gate
 
 def latent_prefill_tc_ok(q, out, cache, heads, rank, rot, page_size, batch) -> bool:
     """Whether a step's attention over the latent runs on tcgen05: bfloat16, sizes and pages that its tiles take, and enough
-    tiles of 128 (token, head) rows that every SM has one (fewer: the kernel that cuts keys into ranges)."""
+    tiles of 128 (token, head) rows that every SM has one (fewer: the kernel that cuts keys into ranges).  A tile belongs to one
+    sequence, and beyond 256 columns two CTAs compute its scores: there, sequences of up to 32 rows stay on the kernel whose
+    tiles have 32 (512 + 64 columns, 16 heads, contexts of 300, us there and here: 1,200 sequences of one token 267 / 371, 600 of
+    two 165 / 206, 300 of four 163 / 128; of 256 + 32 columns 1,200 of one 194 / 172)."""
     H, W = int(heads), int(rank) + int(rot)
+    if rank > 256 and q.shape[0] * H <= 32 * batch.n_seqs:
+        return False
     return (cache.dtype == torch.bfloat16 and cache.is_contiguous() and (q.shape[0] * H // 128) * -(-int(rank) // 256) >= sm_count(out.device)
             and -(-batch.max_q_len * H // 128) <= 65535 and 0 < cache.numel() // W <= 2147483647 and cache.numel() % (W * int(page_size)) == 0
             and (q.stride(0) | out.stride(0)) % 4 == 0 and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0

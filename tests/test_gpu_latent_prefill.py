@@ -71,3 +71,36 @@ def test_small_steps_and_odd_pages_keep_their_kernels():
         q, out = torch.zeros(n, 16 * 576, device=DEV), torch.zeros(n, 16 * 512, device=DEV)
         assert ops.latent_prefill_tc_ok(q, out, cache, 16, 512, 64, page, b) == want
     assert not ops.latent_prefill_tc_ok(q, out, cache.float(), 16, 512, 64, 64, b)
+
+
+def test_many_short_sequences_keep_the_kernel_of_short_tiles():
+    for H, rank, n, per, want in ((16, 512, 1200, 1, False), (16, 512, 600, 2, False), (16, 512, 400, 3, True), (16, 256, 1200, 1, True),
+                                  (40, 320, 300, 1, True)):
+        cache = torch.zeros(4, 1, 64, rank + 64, dtype=torch.bfloat16, device=DEV)
+        q, out = torch.empty(n * per, H * (rank + 64), device=DEV), torch.empty(n * per, H * rank, device=DEV)
+        b = SimpleNamespace(n_seqs=n, max_q_len=per)
+        assert ops.latent_prefill_tc_ok(q, out, cache, H, rank, 64, 64, b) == want
+
+
+@pytest.mark.parametrize("H,rank,rot", [(16, 512, 64), (16, 256, 32)])
+def test_pages_that_held_something_before(H, rank, rot):
+    """Rows of a sequence's last page behind its last key hold another sequence's numbers: they do not count, whatever they are."""
+    page, W, n = 64, rank + rot, 1300
+    g = torch.Generator(device=DEV).manual_seed(H + rank)
+    cache = torch.randn(24, 1, page, W, generator=g, device=DEV).bfloat16()
+    q = torch.randn(n, H * W, generator=g, device=DEV) * (2.0 / W ** 0.5)
+    pages = torch.randperm(24, generator=g, device=DEV)[:21].int().view(1, 21).contiguous()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(n_seqs=1, n_tokens=n, max_q_len=n, seq_start=i32([0, n]), seq_pos0=i32([0]))
+    tok_seq, tok_pos = torch.zeros(n, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV)
+    outs = []
+    for behind in (None, 0.0, 3.0e38, -3.0e38):
+        c = cache.clone()
+        if behind is not None:
+            c[pages[0, 20].long(), 0, n - 20 * page:] = behind
+        out = torch.full((n, H * rank), 9.0, device=DEV)
+        assert ops.latent_prefill_tc_ok(q, out, c, H, rank, rot, page, batch)
+        ops.latent_attention(q, out, c, None, tok_seq, tok_pos, pages, H, rank, rot, page, None, batch=batch)
+        outs.append(out)
+    ops.check_kernel_errors()
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
