@@ -232,7 +232,6 @@ extern "C" int hb_attention_simt(int dtype, const void* q, int ldq, void* out, i
   AttnArgs a{q, ldq, out, ldo, kcache, vcache, tok_seq, tok_pos, seq_pages, pages_stride,
              n_tokens, nh, nkv, hd, page_size, scale, window, softcap, sink, gate_bias, out_gate, ldg, out_f32};
   const long long units = (long long)n_tokens * nh;
-  HB_REQUIRE(units < 2147483647LL, "attention: too many (token, head) pairs");
   // four elements a load where every head's row starts on four
   const int es = dtype == HB_F32 ? 4 : 2;
   const bool v4 = hd % 4 == 0 && (((uintptr_t)kcache | (uintptr_t)vcache) & (uintptr_t)(4 * es - 1)) == 0;
@@ -242,6 +241,7 @@ extern "C" int hb_attention_simt(int dtype, const void* q, int ldq, void* out, i
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const bool many = units >= 8LL * sms;
+  HB_REQUIRE(ceil_div_ll(units, ATT_WARPS / 2) < 2147483647LL, "attention: too many (token, head) pairs");
 #define AS_GO(T, MAX_HD, V)                                                                                                                  \
   do {                                                                                                                                       \
     if (many) hb_launch(attention_simt_kernel<T, MAX_HD, V, 2>, dim3((unsigned)ceil_div_ll(units, ATT_WARPS / 2)), dim3(ATT_WARPS * 32), 0, (cudaStream_t)stream, a); \
