@@ -281,7 +281,7 @@ template <bool V> struct ls_const { static constexpr bool value = V; };
 #define LS_KPAD 4      // a token's row of keys in shared memory is this much longer: rows of neighbouring tokens in other banks
 static_assert(LS_CHUNK == 16 && LS_THREADS == 128, "the chunked scan maps one entry of a 16 x 16 triangle to each of 128 threads");
 
-template <int RPT, bool DELTA>
+template <int RPT>
 __global__ void __launch_bounds__(LS_THREADS) linear_scan_chunked_kernel(ScanArgs a) {
   extern __shared__ __align__(16) float sh[];
   constexpr int C = LS_CHUNK;
@@ -310,7 +310,6 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_chunked_kernel(ScanArg
   for (int i = tid; i < 2 * stage_floats + 2 * C * C + 2 * C; i += LS_THREADS) sh[i] = 0.0f;
   __syncthreads();
   const bool wide = a.dk % 4 == 0 && a.ldq % 4 == 0 && a.ldk % 4 == 0 && (((uintptr_t)a.q | (uintptr_t)a.k) & 15) == 0;
-  const float d = DELTA ? 0.0f : a.decay[h];
   int st_lanes = 1;                                               // threads that copy one token's row of q and k
   while (st_lanes < LS_THREADS && st_lanes * 4 < a.dk) st_lanes <<= 1;
   const int st_row = tid / st_lanes, st_r = (tid % st_lanes) * 4;
@@ -339,11 +338,10 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_chunked_kernel(ScanArg
       const int tt = i >> cshift, c = blockIdx.z * cols + (i & (cols - 1));
       if (c < a.dv) ls_copy4(vs + i, a.v + (size_t)(c0 + tt) * a.ldv + h * a.dv + c);
     }
-    if (DELTA)
-      for (int i = tid; i < 2 * n; i += LS_THREADS) {
-        const int tt = i >> 1, which = i & 1;
-        ls_copy4(gs + i, a.gates + (size_t)(c0 + tt) * 2 * a.H + which * a.H + h);
-      }
+    for (int i = tid; i < 2 * n; i += LS_THREADS) {
+      const int tt = i >> 1, which = i & 1;
+      ls_copy4(gs + i, a.gates + (size_t)(c0 + tt) * 2 * a.H + which * a.H + h);
+    }
     asm volatile("cp.async.commit_group;");
   };
 
@@ -373,7 +371,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_chunked_kernel(ScanArg
         const float4* kt = reinterpret_cast<const float4*>(ks + t * KS);
         const float4* qt = reinterpret_cast<const float4*>(qs + t * KS);
         const float4* kk = reinterpret_cast<const float4*>(ks + sx * KS);
-        const bool below = DELTA && sx < t;
+        const bool below = sx < t;
         float m0 = 0.0f, m1 = 0.0f, n0 = 0.0f, n1 = 0.0f;
 #pragma unroll 4
         for (int i = 0; i < DKP / 4; ++i) {
@@ -385,10 +383,10 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_chunked_kernel(ScanArg
           }
         }
         float w = 1.0f;                                                 // g_(s+1) ... g_t
-        for (int r = sx + 1; r <= t; ++r) w *= DELTA ? gs[2 * r] : d;
+        for (int r = sx + 1; r <= t; ++r) w *= gs[2 * r];
         Nn[t * C + sx] = w * (n0 + n1);
         if (below) Mm[t * C + sx] = w * (m0 + m1);
-        if (sx == 0) Gt[t] = w * (DELTA ? gs[0] : d);
+        if (sx == 0) Gt[t] = w * gs[0];
         if (t == n - 1) Et[sx] = w;
       };
       {
@@ -412,11 +410,9 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_chunked_kernel(ScanArg
             const float4 q = q4[i * R];
             o0 = fmaf(s[4 * i], q.x, o0); o1 = fmaf(s[4 * i + 1], q.y, o1);
             o0 = fmaf(s[4 * i + 2], q.z, o0); o1 = fmaf(s[4 * i + 3], q.w, o1);
-            if (DELTA) {
-              const float4 k = k4[i * R];
-              p0 = fmaf(s[4 * i], k.x, p0); p1 = fmaf(s[4 * i + 1], k.y, p1);
-              p0 = fmaf(s[4 * i + 2], k.z, p0); p1 = fmaf(s[4 * i + 3], k.w, p1);
-            }
+            const float4 k = k4[i * R];
+            p0 = fmaf(s[4 * i], k.x, p0); p1 = fmaf(s[4 * i + 1], k.y, p1);
+            p0 = fmaf(s[4 * i + 2], k.z, p0); p1 = fmaf(s[4 * i + 3], k.w, p1);
           }
           pk[t] = p0 + p1; pq[t] = o0 + o1;
         }
@@ -425,7 +421,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_chunked_kernel(ScanArg
 #pragma unroll
         for (int t = 0; t < C; ++t) {
           pq[t] += __shfl_xor_sync(0xffffffffu, pq[t], w);
-          if (DELTA) pk[t] += __shfl_xor_sync(0xffffffffu, pk[t], w);
+          pk[t] += __shfl_xor_sync(0xffffffffu, pk[t], w);
         }
       }
       __syncthreads();                      // the triangles are complete
@@ -439,19 +435,15 @@ __global__ void __launch_bounds__(LS_THREADS) linear_scan_chunked_kernel(ScanArg
           const float v = vs[t * cols + cl];
           const float G = Gt[t];
           float row[C];                                  // a row of a triangle, four entries a load
-          if (DELTA) {
 #pragma unroll
-            for (int j = 0; 4 * j < t; ++j) {
-              const float4 x = reinterpret_cast<const float4*>(Mm + t * C)[j];
-              row[4 * j] = x.x; row[4 * j + 1] = x.y; row[4 * j + 2] = x.z; row[4 * j + 3] = x.w;
-            }
-            float acc = fmaf(-G, pk[t], v);
-#pragma unroll
-            for (int sx = 0; sx < t; ++sx) acc = fmaf(-row[sx], u[sx], acc);
-            u[t] = gs[2 * t + 1] * acc;
-          } else {
-            u[t] = v;
+          for (int j = 0; 4 * j < t; ++j) {
+            const float4 x = reinterpret_cast<const float4*>(Mm + t * C)[j];
+            row[4 * j] = x.x; row[4 * j + 1] = x.y; row[4 * j + 2] = x.z; row[4 * j + 3] = x.w;
           }
+          float now = fmaf(-G, pk[t], v);
+#pragma unroll
+          for (int sx = 0; sx < t; ++sx) now = fmaf(-row[sx], u[sx], now);
+          u[t] = gs[2 * t + 1] * now;
 #pragma unroll
           for (int j = 0; 4 * j <= t; ++j) {
             const float4 x = reinterpret_cast<const float4*>(Nn + t * C)[j];
@@ -530,6 +522,8 @@ extern "C" int hb_linear_scan(int delta, const float* q, int ldq, const float* k
   // The delta rule takes the chunked kernel when the step's longest sequence brings LS_CHUNKED_FROM tokens or more and
   // the grid leaves SMs with one CTA or none: there a CTA's time is the length of its chain of dependent operations,
   // which the chunked form shortens.  With several CTAs on every SM the token-by-token form issues fewer instructions.
+  // (us token by token and in chunks, one prompt of 2,048: 16 heads of 32 x 64 605 / 406, of 96 x 128 808 / 661, of 128 x 130 804 / 657; of 192 x
+  // 128, where a lane holds 12 rows and more, 1,061 / 1,288.)
   const bool chunked = delta && max_q_len >= LS_CHUNKED_FROM && (long long)grid.x * grid.y * grid.z < 2LL * sms;
   const size_t smem = chunked ? (size_t)(2 * LS_CHUNK * (2 * (R * rpt + LS_KPAD) + cols + 2) + 2 * LS_CHUNK * LS_CHUNK + 2 * LS_CHUNK) * sizeof(float)
                               : (size_t)(2 * LS_CHUNK * (2 * R * rpt + cols + 2) + LS_CHUNK * (LS_THREADS + LS_RED_PAD)) * sizeof(float);
@@ -540,17 +534,11 @@ extern "C" int hb_linear_scan(int delta, const float* q, int ldq, const float* k
     if (smem > 48 * 1024) cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 \
     hb_launch(KERNEL, grid, dim3(LS_THREADS), smem, s, a);                                                                      \
   } while (0)
-#define LS_GO(RPT)                                                                                                              \
-  do {                                                                                                                          \
-    if (chunked) {                                                                                                              \
-      if (delta) LS_GO_ONE((linear_scan_chunked_kernel<RPT, true>)); else LS_GO_ONE((linear_scan_chunked_kernel<RPT, false>));  \
-    } else if (delta) {                                                                                                                \
-      if (smem > 48 * 1024) cudaFuncSetAttribute(linear_scan_kernel<RPT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      hb_launch(linear_scan_kernel<RPT, true>, grid, dim3(LS_THREADS), smem, s, a);                                             \
-    } else {                                                                                                                    \
-      if (smem > 48 * 1024) cudaFuncSetAttribute(linear_scan_kernel<RPT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      hb_launch(linear_scan_kernel<RPT, false>, grid, dim3(LS_THREADS), smem, s, a);                                            \
-    }                                                                                                                           \
+#define LS_GO(RPT)                                                    \
+  do {                                                                \
+    if (chunked) LS_GO_ONE(linear_scan_chunked_kernel<RPT>);          \
+    else if (delta) LS_GO_ONE((linear_scan_kernel<RPT, true>));       \
+    else LS_GO_ONE((linear_scan_kernel<RPT, false>));                 \
   } while (0)
   if (rpt == 4) LS_GO(4); else if (rpt == 8) LS_GO(8); else if (rpt == 16) LS_GO(16); else if (rpt == 32) LS_GO(32); else LS_GO(64);
 #undef LS_GO

@@ -321,8 +321,7 @@ moe_up_kernel(const T* __restrict__ h, int ld, const T* __restrict__ up, const i
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int f = blockIdx.y * MOE_WARPS + warp, u = blockIdx.x;  // u = t*top + r
   if (f >= F) return;
-  const int e = ids[u];
-  if ((unsigned)e >= (unsigned)E) return;
+  const int e = (unsigned)ids[u] < (unsigned)E ? ids[u] : 0;      // no expert: any, its result is left out below
   const T* hr = h + (size_t)(u / top) * ld;
   if (gated) {
     const int grow = gated == 2 ? (f >> 3) * 16 + (f & 7) : f, urow = gated == 2 ? grow + 8 : F + f;
@@ -350,10 +349,11 @@ moe_down_kernel(const T* __restrict__ mid, const T* __restrict__ down, const int
   float acc = 0.0f;
   for (int r = 0; r < top; ++r) {
     const int u = t * top + r;
-    if ((unsigned)ids[u] >= (unsigned)E) continue;
-    const T* w = down + ((size_t)ids[u] * D + d) * F;
+    const bool there = (unsigned)ids[u] < (unsigned)E;           // a choice of numbers and no branch: the pairs' loads go ahead together
+    const T* w = down + ((size_t)(there ? ids[u] : 0) * D + d) * F;
     const T* m = mid + (size_t)u * F;
-    acc = fmaf(wts ? wts[u] : 1.0f, warp_dot(m, w, F, lane), acc);
+    const float more = fmaf(wts ? wts[u] : 1.0f, warp_dot(m, w, F, lane), acc);
+    acc = there ? more : acc;
   }
   if (lane == 0) {
     float* o = y + (size_t)t * ldy + d;
@@ -583,22 +583,23 @@ moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts
   }
   for (int r0 = 0; r0 < top; r0 += 4) {
     float w[4], x[4][V];
+    bool there[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       w[r] = 0.0f;
-#pragma unroll
-      for (int j = 0; j < V; ++j) x[r][j] = 0.0f;
+      there[r] = false;
       if (r0 + r >= top) continue;
       const size_t u = (size_t)t * top + r0 + r;
-      if ((unsigned)ids[u] >= (unsigned)E) continue;
+      there[r] = (unsigned)ids[u] < (unsigned)E;
       w[r] = wts ? wts[u] : 1.0f;
-      const float* p = part + (slot ? (size_t)slot[u] : u) * D + d;
+      const size_t row = slot ? (size_t)max(slot[u], 0) : u;
+      const float* p = part + row * D + d;
       if constexpr (V == 4) { const float4 v = *reinterpret_cast<const float4*>(p); x[r][0] = v.x; x[r][1] = v.y; x[r][2] = v.z; x[r][3] = v.w; }
       else x[r][0] = *p;
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
-      if (r0 + r < top)
+      if (there[r])
 #pragma unroll
         for (int j = 0; j < V; ++j) acc[j] = fmaf(w[r], x[r][j], acc[j]);
   }
