@@ -984,11 +984,12 @@ def moe_few_pays(tokens, top, experts, D, F, gated) -> bool:
     sum below takes them as drawn evenly).  Measured with matrices that come from memory, us a call with a warp per output number
     and with them: 4 of 32 plain experts of 1,408 over 2,048 at 1, 2, 4, 8, 16 tokens 18 / 19, 24 / 26, 41 / 37, 61 / 52, 105 / 69; 2 of 16
     of 768 over 1,024 at 4, 8, 12, 31 tokens 12 / 16, 18 / 18, 22 / 21, 41 / 25; 6 of 64 of 1,024 over 4,096 at 2, 8, 16 tokens 41 / 45,
-    109 / 109, 198 / 156; one of 4 of 128 over 256 at 1 and 31 tokens 4 / 9, 6 / 16."""
+    109 / 109, 198 / 156; 2 of 8 of 14,336 over 4,096 at 1 and 2 tokens 83 / 91, 145 / 139; one of 4 of 128 over 256 at 1 and 31 tokens
+    4 / 9, 6 / 16."""
     pairs = tokens * top
     saved = pairs - experts * (1.0 - (1.0 - min(top, experts) / experts) ** tokens)
     matrices = (3 if gated else 2) * D * F * 2
-    return saved >= 1.0 and (saved + pairs / 8) * matrices >= 32e6
+    return saved * matrices >= 10e6 and (saved + pairs / 8) * matrices >= 32e6
 
 
 def moe_experts_tc(h, up, down, ids, weights, y, accumulate, scratch, act_limit=0.0, weigh_input=False, gated=GATED_GROUPS_OF_8,
