@@ -58,7 +58,6 @@ __device__ __forceinline__ void lp_st32(unsigned taddr, const unsigned* r) {
         "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
         "r"(r[30]), "r"(r[31])
       : "memory");
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 __global__ void __launch_bounds__(LP_THREADS, 1)
@@ -187,7 +186,9 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
         if (!mbar_wait(p_ready, j & 1)) { atomicExch(a.error_flag, 44); break; }
         tc_fence_after();
         for (int ks = 0; ks < LP_KEYS / 16; ++ks)                          // 16 keys of P = 8 columns of tensor memory
-          lp_mma_ta(tm_o, tm_s0 + (j & 1) * LP_KEYS + ks * 8, desc_v + ((ks * 2048) >> 4), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
+          for (int part = 0; part < 2; ++part)
+            lp_mma_ta(tm_o, tm_s0 + (j & 1) * LP_KEYS + part * (LP_KEYS / 2) + ks * 8, desc_v + ((ks * 2048) >> 4), idesc_pv,
+                      (j > 0 || ks > 0 || part > 0) ? 1u : 0u);
         tc_commit(o_full);
         if (j + 1 < n) own_scores(j + 1);
       }
@@ -241,17 +242,22 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_c, LatentTcArgs
         m = mx;
       }
       const float m_use = m == -INFINITY ? 0.0f : m;
-      unsigned pk[LP_KEYS / 2];
+      unsigned pk[LP_KEYS / 2], pl[LP_KEYS / 2];                           // P as two bfloat16 parts
       float sum0 = 0.0f, sum1 = 0.0f;
 #pragma unroll
       for (int i = 0; i < LP_KEYS; i += 2) {
-        const __nv_bfloat162 v = __floats2bfloat162_rn(fast_exp2(fmaf(s[i], log2e, -m_use)), fast_exp2(fmaf(s[i + 1], log2e, -m_use)));
-        sum0 += __low2float(v);                                            // the sums take the rounded weights, the ones the product uses
-        sum1 += __high2float(v);
-        pk[i >> 1] = *reinterpret_cast<const unsigned*>(&v);
+        const float e0 = fast_exp2(fmaf(s[i], log2e, -m_use)), e1 = fast_exp2(fmaf(s[i + 1], log2e, -m_use));
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(e0, e1);
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(e0 - __low2float(hi), e1 - __high2float(hi));
+        sum0 += e0;
+        sum1 += e1;
+        pk[i >> 1] = *reinterpret_cast<const unsigned*>(&hi);
+        pl[i >> 1] = *reinterpret_cast<const unsigned*>(&lo);
       }
       l += sum0 + sum1;
-      lp_st32(tm_s, pk);                                                   // P where the row's scores were
+      lp_st32(tm_s, pk);                                                   // P where the row's scores were, its second part behind the first
+      lp_st32(tm_s + LP_KEYS / 2, pl);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cta(p_ready);
