@@ -166,14 +166,16 @@ __global__ void __launch_bounds__(SR_THREADS) scan_rows_kernel(ScanRows a) {
       const int tt = i / (COLS / VW), c = (i % (COLS / VW)) * VW, cc = blockIdx.x * COLS + c;
       if (cc >= a.dv) continue;
       const float* p = parts + ((buf * CH + tt) * NG + c / CPT) * PART + c % CPT;
-      float sum[VW], y[VW];
-      sr_get<VW>(sum, p);
+      float y[4][VW], sum[VW];                                    // four sums side by side, added in pairs
 #pragma unroll
-      for (int r = 1; r < R; ++r) {
-        sr_get<VW>(y, p + r * CPT);
+      for (int r = 0; r < R; ++r) {
+        float x[VW];
+        sr_get<VW>(x, p + r * CPT);
 #pragma unroll
-        for (int e = 0; e < VW; ++e) sum[e] += y[e];
+        for (int e = 0; e < VW; ++e) y[r & 3][e] = r < 4 ? x[e] : y[r & 3][e] + x[e];
       }
+#pragma unroll
+      for (int e = 0; e < VW; ++e) sum[e] = (y[0][e] + y[1][e]) + (y[2][e] + y[3][e]);
       if (KIND == SCAN_GLA)
 #pragma unroll
         for (int e = 0; e < VW; ++e) sum[e] *= a.scale;
