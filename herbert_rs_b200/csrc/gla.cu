@@ -209,11 +209,11 @@ extern "C" int hb_gla_scan(const float* proj, int ld, int q_off, int k_off, int 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // scan_rows.cuh walks tokens faster but reads and writes a state row in pieces of 8 or 16 bytes, and its CTAs own 2,048 / dk columns or
-  // more: for sequences of dk / 4 tokens on average (the state's way then counts little) and about a CTA an SM.  us of the kernel above
-  // and of that one: 4 heads of 256 x 512, 4 and 16 sequences of one token 6 / 9 and 19 / 28, of 64 tokens 41 / 44 and 158 / 147, 1,500, 800, 300
-  // and 73 tokens 857 / 430; 4 heads of 128 x 256, 8 sequences of one token 4.3 / 4.6, of 32 15 / 12, one of 600 (64 CTAs) 78 / 92;
-  // 16 heads of 64 x 64, two sequences of 600 (64 CTAs) 64 / 77, four 87 / 77.
-  const bool long_enough = 4LL * n_tokens >= (long long)dk * n_seqs;
+  // more: for sequences of 16 tokens on average (64 of 256 key channels, whose pieces lie further apart) and about a CTA an SM.  us of the
+  // kernel above and of that one: 4 heads of 256 x 512, 4 and 16 sequences of one token 6 / 9 and 19 / 28, 8 of 16 27 / 30, 8 of 64 80 / 78,
+  // 1,500, 800, 300 and 73 tokens 857 / 430; 4 heads of 128 x 256, 16 sequences of one token 7 / 8, of 16 17 / 15, one of 600 (64 CTAs)
+  // 78 / 92; 16 heads of 64 x 64, two sequences of 600 (64 CTAs) 64 / 77, four 87 / 77.
+  const bool long_enough = n_tokens >= (dk > 128 ? 64LL : 16LL) * n_seqs;
   const bool enough_ctas = 6LL * n_seqs * heads * ceil_div_ll((long long)dv * dk, 2048) >= 5LL * sms;
   if (long_enough && enough_ctas && scan_rows<SCAN_GLA>(sr, n_seqs, dk, s)) {
     HB_CHECK_LAUNCH("gla_scan");

@@ -94,6 +94,6 @@ def test_scan_rows_over_several_chunks(kind, dk, shape):
 @pytest.mark.parametrize("dk", [64, 128, 256])
 @pytest.mark.parametrize("less", [0, 1])
 def test_gla_scan_around_the_length_where_its_kernel_changes(dk, less):
-    """dk / 4 tokens a sequence on average, and one token less."""
-    n = dk // 4
+    """As many tokens a sequence on average as the rule asks for, and one token less."""
+    n = 64 if dk > 128 else 16
     _check("gla", [n + 3, n - 3, n, n - less, 2 * n - 1, 1] * 2, 8, 8, dk, 132)
