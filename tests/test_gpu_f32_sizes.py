@@ -41,3 +41,10 @@ def _runs(dtype, nh, nkv, hd, window, lens, qlens):
     ops.attention_simt(dev(c["q"]), c["q"].shape[1], out, dev(c["k"]), dev(c["v"]), dev(c["tok_seq"]), dev(c["tok_pos"]),
                        dev(c["table"]), nh, nkv, hd, 16, c["scale"], window)
     close(out, c["ref"], dtype, rowwise=True)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd", [1, 126, 127, 130, 254, 257, 511])
+def test_attention_simt_heads_of_no_multiple_of_four(dtype, hd):
+    """The instances for up to 128, 256 and 512 channels, a channel at a time."""
+    test_attention_simt_runs_of_keys(dtype, 2, 1, hd, None)

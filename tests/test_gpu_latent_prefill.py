@@ -104,3 +104,31 @@ def test_pages_that_held_something_before(H, rank, rot):
         outs.append(out)
     ops.check_kernel_errors()
     assert all(torch.equal(outs[0], o) for o in outs[1:])
+
+
+@pytest.mark.parametrize("H,rank,rot,below,above", [(16, 512, 64, 591, 592), (16, 256, 32, 1183, 1184)])
+def test_a_prompt_on_both_sides_of_the_rule(H, rank, rot, below, above):
+    """One token less than gives every SM a tile, and that many: the other kernel, the same numbers up to rounding."""
+    page, W = 64, rank + rot
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the token counts are those of 148 SMs")
+    g = torch.Generator(device=DEV).manual_seed(H + rank)
+    per = -(-above // page)
+    cache = torch.randn(per, 1, page, W, generator=g, device=DEV).bfloat16()
+    pages = torch.arange(per, dtype=torch.int32, device=DEV).view(1, per)
+    q = torch.randn(above, H * W, generator=g, device=DEV) * (2.0 / W ** 0.5)
+    outs = []
+    for n in (below, above):
+        batch = SimpleNamespace(n_seqs=1, n_tokens=n, max_q_len=n, seq_start=torch.tensor([0, n], dtype=torch.int32, device=DEV),
+                                seq_pos0=torch.zeros(1, dtype=torch.int32, device=DEV))
+        out = torch.full((n, H * rank), 9.0, device=DEV)
+        assert ops.latent_prefill_tc_ok(q[:n], out, cache, H, rank, rot, page, batch) == (n == above)
+        ops.latent_attention(q[:n], out, cache, None, torch.zeros(n, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV),
+                             pages, H, rank, rot, page, None, batch=batch, scratch=lambda s, dt: torch.empty(s, dtype=dt, device=DEV))
+        outs.append(out[:below].view(below, H, rank).double())
+    ops.check_kernel_errors()
+    p = torch.softmax(torch.einsum("thw,jw->thj", q[:below].bfloat16().double().view(below, H, W), cache.view(-1, W)[:below].double())
+                      .masked_fill(torch.ones(below, below, dtype=torch.bool, device=DEV).triu(1)[:, None], float("-inf")), -1)
+    # both round the softmax weights to bfloat16 (2^-8 of each), each at its own scale
+    bound = torch.einsum("thj,jr->thr", p, cache.view(-1, W)[:below, :rank].double().abs()) * 2.0 ** -7 + 1e-5
+    assert ((outs[0] - outs[1]).abs() <= bound).all()
