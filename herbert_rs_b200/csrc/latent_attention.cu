@@ -262,8 +262,10 @@ headwise_mma_kernel(const float* __restrict__ in, int ld_in, int in_hs, const bf
 
 // The same for prompts, 128 tokens x 128 outputs a CTA, a warp 32 x 64: an input row is read N / 128 times, and the next
 // slab's inputs are on their way in registers while this one is multiplied.
-// Bound by the instruction's rate and the float outputs.  Measured on a B200, 2,673 tokens, 16 heads, inside a step: 128 -> 512 numbers
-// a head 70 -> 41 us, 512 -> 128 with gates 107 -> 79 us.
+// Bound by the instruction's rate and the float outputs.  Measured on a B200, 2,673 tokens, 16 heads, inside a step, tiles of 64 x 64 ->
+// these: 128 -> 512 numbers a head 70 -> 41 us, 512 -> 128 with gates 107 -> 63 us.  At 128 to 2,673 tokens and 4 to 32 heads
+// none of 128 -> 512, 512 -> 128, 64 -> 256 and 128 -> 128 numbers takes more than 1.08 times what the small tiles take (512 -> 128, 4
+// heads, 128 tokens: 28 -> 20), so the rule needs no look at the number of CTAs.
 #define HL_T 128
 template <typename TO>
 __global__ void __launch_bounds__(256, 2)

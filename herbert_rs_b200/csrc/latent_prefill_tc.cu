@@ -13,9 +13,10 @@
 // run while the row threads take this tile's softmax.  A thread owns a row (as in attention_prefill_tc.cu): P goes back over
 // the scores, O is rescaled only when a tile's maximum exceeds the row's reference by more than 2^8.
 // Bound by the reads of the queries from shared memory (4 KB per 128 x 64 x 16 product).
-// Measured on a B200 alone, 16 heads, latent 512 + 64: four prompts of 714 to 2,000 tokens 1,057 us on mma.sync -> 389, four of 336 to
-// 1,500 467 -> 191; of that about 26 us a CTA go into its queries and results.  (One barrier a block of columns and a loop over
-// the steps of K: 557 and 263, the MMA lane's own instructions were the limit; 32 keys a tile with two sets of blocks: 590.)
+// Measured on a B200 inside a step, 16 heads, latent 512 + 64: four prompts of 714 to 2,000 tokens 1,057 us on mma.sync -> 421, four of 336
+// to 1,500 477 -> 208; of that about 26 us a CTA go into its queries and results.  (With the weights in one part 391 and 194; so, and
+// with one barrier a block of columns and a loop over the steps of K, 557 and 263: the MMA lane's own instructions were the limit;
+// with 32 keys a tile and two sets of blocks 590.)
 #include "api.h"
 #include "common.cuh"
 #include "tcgen05_utils.cuh"

@@ -14,11 +14,13 @@
 // expert's input instead of its output: then both its products are multiplied before the activation, in float, and the
 // experts' results are added as they are.
 //
-// Three launches, all reading the choice from device memory (nothing of it is known to the host, so
-// a recorded step can be replayed): the router with softmax and choice; the chosen experts' first
-// product with the activation; their second product with the weighted sum.  A warp computes one
-// output number from one weight row read along its length, which is what a step of few tokens
-// wants: every weight row of a chosen expert is read once per token that chose it.
+// All launches read the choice from device memory (nothing of it is known to the host, so a recorded step can be replayed): the
+// router with softmax and choice, then the chosen experts' products by the size of the step.
+//   bfloat16, up to 32 tokens that share experts: moe_few.cu reads every chosen expert once (ops.moe_few_pays)
+//   bfloat16, 32 tokens and more: pairs grouped by expert, tiles on the tensor cores (below; long prompts on tcgen05)
+//   the rest (float32, few tokens that share little, `gated` 1, widths that are no multiple of 8): first product with the
+//   activation, second product with the weighted sum, a warp per output number from one weight row read along its length, so
+//   every weight row of a chosen expert is read once per token that chose it.
 //
 // A pair whose index lies outside the experts contributes nothing, in every kernel of the feed-forward alike (the router gives none).
 #include "api.h"
@@ -561,7 +563,7 @@ moe_grouped_gemm_kernel(const bf16* __restrict__ A, int lda, const bf16* __restr
 
 // slot: where each pair's row lies in `part` (null: at the pair's own index); wts null: weights of 1; pairs without an expert are left out.  V = 4: four columns a
 // thread (D, ldy multiples of 4, rows on 16 bytes), the rows of four pairs asked for at once.
-// Bound by the pairs' rows.  Measured on a B200, 3,600 tokens of 2,048 numbers, 4 pairs each, inside a step: 65 -> 34 us.
+// Bound by the pairs' rows.  Measured on a B200, 3,600 tokens of 2,048 numbers, 4 pairs each, inside a step: 65 -> 36 us.
 template <int V>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts, float* __restrict__ y, int ldy, int D, int E, int top,

@@ -17,9 +17,11 @@
 // comes from another sequence; the kernel starts after the one before it has ended, since CTAs that come in beside its last
 // ones crowd on the SMs that are free first (2.5 times the time where there is one CTA an SM).
 // Bound by the token's chain (sum, exchange, update) where sequences and heads are few, else by multiply-adds and
-// shared memory alike.  Measured on a B200 alone, heads of 128 x 128 (GLA: 4 heads of 256 x 512), before -> after: inside a prompt's step
-// 16 heads x 2,048 tokens of the delta rule 1,009 -> 360 us, with constant decays 353 -> 250; two sequences of 1,301 and 700 tokens
-// of the generalised rule 1,316 -> 395; GLA over four of up to 1,500 855 -> 440.
+// shared memory alike.  Measured on a B200 inside a prompt's step, heads of 128 x 128 (GLA: 4 heads of 256 x 512), the other kernels of these
+// files -> this one: 16 heads x 2,048 tokens of the delta rule 1,014 -> 351 us, with constant decays 353 -> 245; two sequences of 1,301
+// and 700 tokens of the generalised rule 1,315 -> 425; GLA over four of up to 1,500 855 -> 407.  One token a sequence, 16 heads of
+// 128 x 128, 1, 8 and 64 sequences: the delta rule 4.5 / 10.7 / 63 -> 4.1 / 8.6 / 51, the generalised rule 5.3 / 26 / 194 -> 4.3 / 8.7 / 53
+// (GLA keeps the other kernel there: gla.cu).
 #pragma once
 #include "common.cuh"
 

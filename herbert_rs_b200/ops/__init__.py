@@ -1017,7 +1017,7 @@ def moe_experts_tc(h, up, down, ids, weights, y, accumulate, scratch, act_limit=
 
 
 def moe_experts_grouped(h, up, down, ids, weights, y, act, accumulate, scratch, gated=0, act_limit=0.0, weigh_input=False) -> None:
-    """moe_experts for many tokens: pairs grouped by expert on the device, tiles of 64 pairs on the tensor cores."""
+    """moe_experts for many tokens: pairs grouped by expert on the device, tiles of 128 pairs on the tensor cores."""
     _check(h, torch.bfloat16, "h"); _check(up, torch.bfloat16, "up"); _check(down, torch.bfloat16, "down"); _check(y, torch.float32, "y")
     T, top = ids.shape
     E, F, D = up.shape

@@ -35,7 +35,8 @@ class KernelOptions:
     pdl_eager: bool = True
     # The same inside recorded decode steps: 0 off, 1 every kernel, 2 only the products that load weights before they wait.
     pdl_graph: int = 0
-    # Attention over a cached latent, bfloat16: "mma" (tensor cores where the sizes allow), or "simt" (the any-shape kernel).
+    # Attention over a cached latent, bfloat16: "mma" (tensor cores where the sizes allow: tcgen05 for prompts that give every SM a
+    # tile, else mma.sync), or "simt" (the any-shape kernel).
     latent_attention: str = "mma"
     # ... whose rows' keys are cut into at most this many ranges when a step has too few rows to fill the GPU.
     latent_max_splits: int = 16
@@ -44,7 +45,8 @@ class KernelOptions:
     moe_few: str = "auto"
     # Routed feed-forward, bfloat16, steps of 32 tokens and more: pairs grouped by expert, tiles on the tensor cores.
     moe_grouped: bool = True
-    # ... and, for gated experts with silu and 512 (token, expert) pairs or more, those tiles on tcgen05.
+    # ... and, from 512 (token, expert) pairs on, those tiles on tcgen05: gated experts with silu or the clamped activation, plain ones
+    # with silu or a gelu (see ops.moe_tc_ok).
     moe_tc: bool = True
     # State-space recurrence, bfloat16, steps that bring many tokens: 64 tokens at a time on the tensor cores.
     ssd_chunked: bool = True
