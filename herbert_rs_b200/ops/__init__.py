@@ -980,16 +980,12 @@ def moe_tc_ok(h, up, top, gated, act) -> bool:
 
 def moe_few_pays(tokens, top, experts, D, F, gated) -> bool:
     """Whether a step of few tokens gains by reading every chosen expert once for all its tokens.  The kernels that do so sort the
-    step's pairs first, about 5 us; what they save are the matrices that several tokens choose, less where the choices spread (the
-    sum below takes them as drawn evenly).  Measured with matrices that come from memory, us a call with a warp per output number
-    and with them: 4 of 32 plain experts of 1,408 over 2,048 at 1, 2, 4, 8, 16 tokens 18 / 19, 24 / 26, 41 / 37, 61 / 52, 105 / 69; 2 of 16
-    of 768 over 1,024 at 4, 8, 12, 31 tokens 12 / 16, 18 / 18, 22 / 21, 41 / 25; 6 of 64 of 1,024 over 4,096 at 2, 8, 16 tokens 41 / 45,
-    109 / 109, 198 / 156; 2 of 8 of 14,336 over 4,096 at 1 and 2 tokens 83 / 91, 145 / 139; one of 4 of 128 over 256 at 1 and 31 tokens
-    4 / 9, 6 / 16."""
-    pairs = tokens * top
-    saved = pairs - experts * (1.0 - (1.0 - min(top, experts) / experts) ** tokens)
-    matrices = (3 if gated else 2) * D * F * 2
-    return saved * matrices >= 10e6 and (saved + pairs / 8) * matrices >= 32e6
+    step's pairs first, about 5 us, and then stream at the better rate, more so the more tokens share an expert: they pay from
+    about 36 MB of matrices on, counted once per pair.  Measured inside recorded decode steps, us a layer that they take less
+    than a warp per output number (4 of 32 experts of 1,408 over 2,048, then 2 of 16 of 768 over 1,024): plain experts at 1, 2, 4, 8 tokens
+    +11, +8, +13, +18 and -2, -4, -2, +3 (6 tokens: -0.3), gated ones +4, +5, +10, +16 and -1, -1, +1, +5; one of 4 of 128 over 256, alone, at
+    1 and 31 tokens -5, -10."""
+    return tokens * top * (3 if gated else 2) * D * F * 2 >= 36e6
 
 
 def moe_experts_tc(h, up, down, ids, weights, y, accumulate, scratch, act_limit=0.0, weigh_input=False, gated=GATED_GROUPS_OF_8,
@@ -1040,7 +1036,7 @@ def moe_experts(h, up, down, ids, weights, mid, y, act, accumulate=False, gated=
     _check(h, None, "h"); _check(up, h.dtype, "up"); _check(down, h.dtype, "down"); _check(mid, h.dtype, "mid"); _check(y, torch.float32, "y")
     if not (up.is_contiguous() and down.is_contiguous() and mid.is_contiguous()):
         raise BackendError("moe_experts: up, down and mid must be contiguous")
-    # bfloat16 steps of up to 32 tokens that share experts read every chosen expert once for all its tokens; the rest a warp per output number
+    # bfloat16 steps of up to 32 tokens read every chosen expert once for all its tokens where that pays; the rest a warp per output number
     T, top, E, D, F = h.shape[0], ids.shape[1], up.shape[0], h.shape[1], down.shape[2]
     few = options.moe_few == "always" or (options.moe_few == "auto" and moe_few_pays(T, top, E, D, F, gated))
     if few and h.dtype == torch.bfloat16 and _fn("hb_moe_experts_few_ok")(h.data_ptr(), h.stride(0), up.data_ptr(), down.data_ptr(), mid.data_ptr(),

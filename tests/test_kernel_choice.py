@@ -6,8 +6,8 @@ from herbert_rs_b200 import ops
 
 
 @pytest.mark.parametrize("top,E,D,F,gated,loses,pays", [
-    (4, 32, 2048, 1408, 0, 2, 3), (4, 32, 2048, 1408, 2, 1, 4), (2, 16, 1024, 768, 0, 8, 12), (2, 16, 1024, 768, 2, 4, 8),
-    (2, 8, 1024, 512, 0, 8, 12), (8, 128, 2048, 768, 0, 2, 4), (2, 8, 4096, 14336, 0, 1, 2), (6, 64, 4096, 1024, 0, 2, 8)])
+    (4, 32, 2048, 1408, 0, 0, 1), (4, 32, 2048, 1408, 2, 0, 1), (2, 16, 1024, 768, 0, 4, 8), (2, 16, 1024, 768, 2, 2, 4),
+    (2, 8, 1024, 512, 0, 8, 12), (8, 128, 2048, 768, 0, 0, 1)])
 def test_experts_are_read_once_where_a_step_shares_them(top, E, D, F, gated, loses, pays):
     """`loses`, `pays`: tokens at which a warp per output number and experts read once for all tokens were measured to be faster."""
     assert not any(ops.moe_few_pays(t, top, E, D, F, gated) for t in range(1, loses + 1))
