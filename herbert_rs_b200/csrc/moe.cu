@@ -16,9 +16,9 @@
 //
 // All launches read the choice from device memory (nothing of it is known to the host, so a recorded step can be replayed): the
 // router with softmax and choice, then the chosen experts' products by the size of the step.
-//   bfloat16, up to 32 tokens that share experts: moe_few.cu reads every chosen expert once (ops.moe_few_pays)
+//   bfloat16, up to 32 tokens, matrices large enough: moe_few.cu reads every chosen expert once (ops.moe_few_pays)
 //   bfloat16, 32 tokens and more: pairs grouped by expert, tiles on the tensor cores (below; long prompts on tcgen05)
-//   the rest (float32, few tokens that share little, `gated` 1, widths that are no multiple of 8): first product with the
+//   the rest (float32, few tokens of small experts, `gated` 1, widths that are no multiple of 8): first product with the
 //   activation, second product with the weighted sum, a warp per output number from one weight row read along its length, so
 //   every weight row of a chosen expert is read once per token that chose it.
 //
