@@ -26,7 +26,7 @@ template <int BN>
 struct TgSmem {
   static constexpr int kStageBytes = (TG_BM + BN) * TG_BK * 2;
   static constexpr int kStages = BN == 256 ? 4 : 6;
-  static constexpr int kBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
+  static constexpr int kBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/ + TG_EPI_WARPS * TG_TURN_BYTES;
 };
 
 #define HB_EPI_QKV 4
@@ -224,6 +224,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // tile's columns, warps 6-9 the second
     const int quad = warp & 3;
     const int c_lo = ((warp - 2) >> 2) * (BN / 64), c_hi = c_lo + BN / 64;
+    const unsigned turn = base + STAGES * STAGE_BYTES + 256 + (warp - 2) * TG_TURN_BYTES;
+    const bool turned = tg_rows_aligned<EPI, NORM>(Cv, ldc, nm);
     int local = 0;
     bool ok = true;
     TgSegments segs(sc, num_tiles, num_kb);
@@ -232,7 +234,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int buf = local & 1;
       const int m0 = (tile % tiles_m) * TG_BM, n0 = (tile / tiles_m) * BN;
       const int m = m0 + quad * 32 + lane;
-      float inv_rms = 1.0f, sq = 0.0f;
+      float inv_rms = 1.0f, sq = 0.0f, sq8[8] = {};
       if (NORM && nm.in_sumsq != nullptr && m < M) {         // while the tensor cores still work on this tile
         float sum = 0.0f;
         for (int i = 0; i < nm.in_parts; ++i) sum += nm.in_sumsq[(size_t)i * nm.in_stride + m];
@@ -321,10 +323,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(acc[j]);
         }
-        tg_epilogue32<EPI, NORM>(r, m, n0 + c * 32, M, N, Cv, ldc, nm, inv_rms, sq);
+        if (turned && n0 + c * 32 + 32 <= N) tg_epilogue32_turned<EPI, NORM>(r, turn, m - lane, n0 + c * 32, M, Cv, ldc, nm, inv_rms, sq8);
+        else tg_epilogue32<EPI, NORM>(r, m, n0 + c * 32, M, N, Cv, ldc, nm, inv_rms, sq);
       }
-      if (NORM && EPI == HB_EPI_RESIDUAL && nm.out_w != nullptr && m < M)
-        nm.out_sumsq[(size_t)(2 * (tile / tiles_m) + (c_lo > 0)) * nm.out_stride + m] = sq;
+      if (NORM && EPI == HB_EPI_RESIDUAL && nm.out_w != nullptr) {
+        sq += tg_row_sums(sq8);
+        if (m < M) nm.out_sumsq[(size_t)(2 * (tile / tiles_m) + (c_lo > 0)) * nm.out_stride + m] = sq;
+      }
     }
   }
   tc_fence_before();
@@ -350,12 +355,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 //             commit, which carries no data);
 //   acc_empty[b]  in the first CTA: the sixteen epilogue warps of the pair arrive there.
 // Whole tiles only (no tiles shared between pairs); pairs walk the tiles m fastest.
-// One head (128 columns starting at tensor-memory address taddr) of row m.  Every lane of the warp
-// runs the tensor-memory loads; rows beyond M store nothing.
+// One head (128 columns starting at tensor-memory address taddr) of the warp's 32 rows, this lane's being m.  Every lane
+// runs the tensor-memory loads and the turns; rows beyond M store nothing.  The sums of squares are a row's own lane's; values, rotation
+// tables and outputs are then taken with eight lanes a row (see tg_turn_in; a row a lane was 12,000 line accesses a tile, twice the
+// tensor work of a product with K = 1,024: 5,083 x 4,096 x 1,024 inside a step 61.6 -> 48.0 us).
 __device__ __forceinline__ void tg_epilogue_qkv(unsigned taddr, int m, int head, int M, void* Cv, int ldc, float inv_rms,
-                                                const TgQkv& q) {
+                                                const TgQkv& q, unsigned st) {
   const int heads_total = q.nh + 2 * q.nkv;
   if (head >= heads_total) return;                                  // uniform over the warp
+  const int lane = threadIdx.x & 31;
   const bool is_q = head < q.nh, is_k = !is_q && head < q.nh + q.nkv;
   const bool live = m < M;
   int pos = 0, seq = 0;
@@ -372,15 +380,7 @@ __device__ __forceinline__ void tg_epilogue_qkv(unsigned taddr, int m, int head,
       dst = (is_k ? q.kcache : q.vcache) + (((size_t)page * q.nkv + kvh) * q.page_size + (pos % q.page_size)) * 128;
     }
   }
-  auto store32 = [&](bf16* out, const float* v) {
-#pragma unroll
-    for (int j = 0; j < 32; j += 8) {
-      uint4 u;
-      u.x = pack2(v[j], v[j + 1]); u.y = pack2(v[j + 2], v[j + 3]);
-      u.z = pack2(v[j + 4], v[j + 5]); u.w = pack2(v[j + 6], v[j + 7]);
-      *reinterpret_cast<uint4*>(out + j) = u;
-    }
-  };
+  auto row_dst = [&](int row) { return reinterpret_cast<bf16*>(__shfl_sync(0xffffffffu, (unsigned long long)dst, row)); };
   if (!is_q && !is_k) {                                             // v: as projected
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
@@ -388,7 +388,16 @@ __device__ __forceinline__ void tg_epilogue_qkv(unsigned taddr, int m, int head,
       tc_ld32f(taddr + c * 32, t);
 #pragma unroll
       for (int j = 0; j < 32; ++j) t[j] *= inv_rms;
-      if (dst != nullptr) store32(dst + c * 32, t);
+      __syncwarp();
+      tg_turn_in(st, t);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = 8 * i + (lane >> 2), col = lane & 3;
+        const float4 a = tg_turn_out(st, row, 2 * col), b = tg_turn_out(st, row, 2 * col + 1);
+        bf16* out = row_dst(row);
+        if (out != nullptr) *reinterpret_cast<uint4*>(out + c * 32 + 8 * col) = make_uint4(pack2(a.x, a.y), pack2(a.z, a.w), pack2(b.x, b.y), pack2(b.z, b.w));
+      }
     }
     return;
   }
@@ -409,34 +418,50 @@ __device__ __forceinline__ void tg_epilogue_qkv(unsigned taddr, int m, int head,
     inv = 1.0f / sqrtf(ss / 128.0f + q.eps);
   }
   const int trow = pos < q.table_rows ? pos : q.table_rows - 1;
-  const float* cos_row = q.cos_tab + (size_t)trow * 64;
-  const float* sin_row = q.sin_tab + (size_t)trow * 64;
+  const float4 ones = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
 #pragma unroll 1
   for (int c = 0; c < 2; ++c) {                                     // columns 32c.. pair with columns 64 + 32c..
-    float lo[32], hi[32];
-    tc_ld32f(taddr + c * 32, lo);
-    tc_ld32f(taddr + 64 + c * 32, hi);
-    if (live) {
+    const int col = c * 32 + 4 * (lane & 7);
+    const float4 wl = w != nullptr ? *reinterpret_cast<const float4*>(w + col) : ones;
+    const float4 wh = w != nullptr ? *reinterpret_cast<const float4*>(w + 64 + col) : ones;
+    float4 lo[8], hi[8];
+    float t[32];
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        const float4 c4 = *reinterpret_cast<const float4*>(cos_row + c * 32 + j), s4 = *reinterpret_cast<const float4*>(sin_row + c * 32 + j);
-        const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
-        float wl[4] = {1.f, 1.f, 1.f, 1.f}, wh[4] = {1.f, 1.f, 1.f, 1.f};
-        if (w != nullptr) {
-          const float4 a4 = *reinterpret_cast<const float4*>(w + c * 32 + j), b4 = *reinterpret_cast<const float4*>(w + 64 + c * 32 + j);
-          wl[0] = a4.x; wl[1] = a4.y; wl[2] = a4.z; wl[3] = a4.w;
-          wh[0] = b4.x; wh[1] = b4.y; wh[2] = b4.z; wh[3] = b4.w;
-        }
+    for (int half = 0; half < 2; ++half) {
+      tc_ld32f(taddr + half * 64 + c * 32, t);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float x0 = ((lo[j + i] * inv_rms) * inv) * wl[i], x1 = ((hi[j + i] * inv_rms) * inv) * wh[i];
-          lo[j + i] = x0 * cs[i] - x1 * sn[i];
-          hi[j + i] = x0 * sn[i] + x1 * cs[i];
-        }
+      for (int j = 0; j < 32; ++j) t[j] = (t[j] * inv_rms) * inv;
+      __syncwarp();
+      tg_turn_in(st, t);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) (half ? hi : lo)[i] = tg_turn_out(st, 4 * i + (lane >> 3), lane & 7);
+    }
+#pragma unroll
+    for (int i0 = 0; i0 < 8; i0 += 4) {
+      float4 cs[4], sn[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const size_t at = (size_t)__shfl_sync(0xffffffffu, trow, 4 * (i0 + i) + (lane >> 3)) * 64 + col;
+        cs[i] = *reinterpret_cast<const float4*>(q.cos_tab + at);
+        sn[i] = *reinterpret_cast<const float4*>(q.sin_tab + at);
       }
-      if (dst != nullptr) {
-        store32(dst + c * 32, lo);
-        store32(dst + 64 + c * 32, hi);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        bf16* out = row_dst(4 * (i0 + i) + (lane >> 3));
+        const float4 a = lo[i0 + i], b = hi[i0 + i];
+        const float x0[4] = {a.x * wl.x, a.y * wl.y, a.z * wl.z, a.w * wl.w}, x1[4] = {b.x * wh.x, b.y * wh.y, b.z * wh.z, b.w * wh.w};
+        const float ct[4] = {cs[i].x, cs[i].y, cs[i].z, cs[i].w}, si[4] = {sn[i].x, sn[i].y, sn[i].z, sn[i].w};
+        float y0[4], y1[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          y0[k] = x0[k] * ct[k] - x1[k] * si[k];
+          y1[k] = x0[k] * si[k] + x1[k] * ct[k];
+        }
+        if (out != nullptr) {
+          *reinterpret_cast<uint2*>(out + col) = make_uint2(pack2(y0[0], y0[1]), pack2(y0[2], y0[3]));
+          *reinterpret_cast<uint2*>(out + 64 + col) = make_uint2(pack2(y1[0], y1[1]), pack2(y1[2], y1[3]));
+        }
       }
     }
   }
@@ -444,7 +469,7 @@ __device__ __forceinline__ void tg_epilogue_qkv(unsigned taddr, int m, int head,
 
 #define TGP_STAGES 6
 #define TGP_STAGE_BYTES ((TG_BM + 128) * TG_BK * 2)      // 128 rows of A and 128 rows of W, 64 columns each
-#define TGP_SMEM_BYTES (TGP_STAGES * TGP_STAGE_BYTES + 1024 + 256)
+#define TGP_SMEM_BYTES (TGP_STAGES * TGP_STAGE_BYTES + 1024 + 256 + TG_EPI_WARPS * TG_TURN_BYTES)
 
 template <int EPI, bool NORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TG_THREADS, 1)
@@ -554,13 +579,15 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   } else {
     const int quad = warp & 3;
     const int c_lo = ((warp - 2) >> 2) * (BN / 64), c_hi = c_lo + BN / 64;
+    const unsigned turn = base + TGP_STAGES * TGP_STAGE_BYTES + 256 + (warp - 2) * TG_TURN_BYTES;
+    const bool turned = EPI != HB_EPI_QKV && tg_rows_aligned<EPI, NORM>(Cv, ldc, nm);
     int local = 0;
     bool ok = true;
     for (int tile = pair; ok && tile < num_tiles; tile += n_pairs, ++local) {
       const int buf = local & 1;
       const int m0 = (tile % tiles_m) * 2 * TG_BM + (int)rank * TG_BM, n0 = (tile / tiles_m) * BN;
       const int m = m0 + quad * 32 + lane;
-      float inv_rms = 1.0f, sq = 0.0f;
+      float inv_rms = 1.0f, sq = 0.0f, sq8[8] = {};
       if (NORM && nm.in_sumsq != nullptr && m < M) {
         float sum = 0.0f;
         for (int i = 0; i < nm.in_parts; ++i) sum += nm.in_sumsq[(size_t)i * nm.in_stride + m];
@@ -575,7 +602,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const unsigned tmem_acc = tmem_base + (unsigned)(buf * BN);
       const unsigned acc_empty0 = mapa_shared(acc_empty(buf), 0);
       if constexpr (EPI == HB_EPI_QKV) {
-        tg_epilogue_qkv(tmem_acc + ((unsigned)(quad * 32) << 16) + (unsigned)(c_lo * 32), m, (n0 + c_lo * 32) / 128, M, Cv, ldc, inv_rms, qk);
+        tg_epilogue_qkv(tmem_acc + ((unsigned)(quad * 32) << 16) + (unsigned)(c_lo * 32), m, (n0 + c_lo * 32) / 128, M, Cv, ldc, inv_rms, qk, turn);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(acc_empty0);
@@ -589,11 +616,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(acc_empty0);
           }
-          tg_epilogue32<EPI, NORM>(r, m, n0 + c * 32, M, N, Cv, ldc, nm, inv_rms, sq);
+          if (turned && n0 + c * 32 + 32 <= N) tg_epilogue32_turned<EPI, NORM>(r, turn, m - lane, n0 + c * 32, M, Cv, ldc, nm, inv_rms, sq8);
+          else tg_epilogue32<EPI, NORM>(r, m, n0 + c * 32, M, N, Cv, ldc, nm, inv_rms, sq);
         }
       }
-      if (NORM && EPI == HB_EPI_RESIDUAL && nm.out_w != nullptr && m < M)
-        nm.out_sumsq[(size_t)(2 * (tile / tiles_m) + (c_lo > 0)) * nm.out_stride + m] = sq;
+      if (NORM && EPI == HB_EPI_RESIDUAL && nm.out_w != nullptr) {
+        sq += tg_row_sums(sq8);
+        if (m < M) nm.out_sumsq[(size_t)(2 * (tile / tiles_m) + (c_lo > 0)) * nm.out_stride + m] = sq;
+      }
     }
   }
   tc_fence_before();
