@@ -27,6 +27,7 @@ from typing import Dict, List, Optional, Sequence
 import numpy as np
 import torch
 
+from .. import ops
 from ..errors import CacheError
 from .allocator import IdPool
 
@@ -157,6 +158,8 @@ class SequenceCache:
             for g, need in enumerate(self.state_needs):
                 self.state.append(torch.zeros((len(self._state_entries[g]), num_slots, *need.shape),
                                               dtype=need.dtype, device=device))
+        # on the GPU one launch zeroes a slot's rows of every state group
+        self._clearer = ops.RowClearer(self.state) if self.state and self.state[0].is_cuda else None
 
     def _state_entry(self, need: StateNeed, step: int) -> tuple:
         """(group, entry) of one more state of this shape and dtype, owned by schedule step `step`."""
@@ -182,8 +185,11 @@ class SequenceCache:
         self.lengths[s] = 0
         self._pages[s] = [[] for _ in self.kv_needs]
         self._released[s] = [0] * len(self.kv_needs)
-        for st in self.state:
-            st[:, s].zero_()
+        if self._clearer is not None:
+            self._clearer.clear(s)
+        else:
+            for st in self.state:
+                st[:, s].zero_()
         return s
 
     def free_slot(self, slot: int) -> None:

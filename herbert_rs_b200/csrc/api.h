@@ -84,6 +84,7 @@ int hb_get_pdl(void);
 int hb_rng_normal(int dtype, void* out, long long n, unsigned long long key, float mean, float stdev, void*
     stream);
 int hb_fill(int dtype, void* out, long long n, float value, void* stream);
+int hb_clear_rows(int planes, void* const* first, const long long* entry_bytes, const long long* row_bytes, const int* entries, void* stream);
 int hb_cast(int src, const void* in, int dst, void* out, long long n, int round_bf16, void* stream);
 
 // gemm_simt.cu: matrix product of any shape on the CUDA cores (the 32-bit path)

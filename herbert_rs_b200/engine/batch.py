@@ -67,7 +67,8 @@ class StepBatch:
 
     def __init__(self, slots: Sequence[int], tokens: Sequence[Sequence[int]], pos0: Sequence[int],
                  want: Sequence[Sequence[int]], num_kv_groups: int, pages_width: Optional[int] = None,
-                 page_size: int = 64, position_components: int = 1, positions: Optional[Sequence] = None):
+                 page_size: int = 64, position_components: int = 1, positions: Optional[Sequence] = None,
+                 ids: Optional[Sequence[np.ndarray]] = None):
         self.slots = list(slots)
         self.q_lens = [len(t) for t in tokens]
         self.pos0 = list(pos0)
@@ -92,6 +93,7 @@ class StepBatch:
         self.layout = StepLayout.make(self.n_tokens, self.n_seqs, self.n_want, num_kv_groups, self.pages_width,
                                       self.n_components)
         self._tokens = tokens
+        self._ids = ids                  # per sequence the same tokens as an integer array, or None
         self._positions = positions      # per sequence: [len, C] (or [len] when C == 1), or None
         self.host: Optional[np.ndarray] = None
         self.dev: Optional[torch.Tensor] = None
@@ -102,8 +104,10 @@ class StepBatch:
         """Write every array into `buf` (int32, at least layout.total long)."""
         lay, o = self.layout, self.layout.offsets
         T, B = self.n_tokens, self.n_seqs
-        flat = np.fromiter((t for seq in self._tokens for t in seq), dtype=np.int64, count=T)
-        buf[o["token_ids"]:o["token_ids"] + T] = flat
+        if self._ids is not None:
+            np.concatenate(self._ids, out=buf[o["token_ids"]:o["token_ids"] + T], casting="unsafe")
+        else:
+            buf[o["token_ids"]:o["token_ids"] + T] = np.fromiter((t for seq in self._tokens for t in seq), dtype=np.int64, count=T)
         reps = np.asarray(self.q_lens, dtype=np.int64)
         seq_idx = np.repeat(np.arange(B, dtype=np.int32), reps)
         buf[o["tok_seq"]:o["tok_seq"] + T] = seq_idx

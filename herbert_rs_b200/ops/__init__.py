@@ -74,6 +74,7 @@ _SIGS = {
     "hb_sample": [c_void_p, c_int, c_int, c_int, c_float, c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p],
     "hb_rng_normal": [c_int, c_void_p, ctypes.c_longlong, ctypes.c_ulonglong, c_float, c_float, c_void_p],
     "hb_fill": [c_int, c_void_p, ctypes.c_longlong, c_float, c_void_p],
+    "hb_clear_rows": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "hb_cast": [c_int, c_void_p, c_int, c_void_p, ctypes.c_longlong, c_int, c_void_p],
     "hb_layernorm": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
     "hb_layernorm_residual": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
@@ -335,6 +336,31 @@ def fill(out: torch.Tensor, value: float) -> None:
         raise BackendError("fill: out must be contiguous")
     code = 2 if out.dtype == torch.int32 else dtype_code(out.dtype)
     _run("hb_fill", code, out.data_ptr(), out.numel(), float(value), _stream())
+
+
+class RowClearer:
+    """Zeroes one slot's rows of state planes [entries, slots, ...] (contiguous CUDA tensors), all planes in one launch
+    (sixteen at a time).  The planes' facts are laid out once; `clear(slot)` fills in the addresses."""
+
+    AT_ONCE = 16
+
+    def __init__(self, planes):
+        self._groups = []
+        for i in range(0, len(planes), self.AT_ONCE):
+            part = planes[i:i + self.AT_ONCE]
+            for p in part:
+                _check(p, None, "state plane")
+                if not p.is_contiguous():
+                    raise BackendError("RowClearer: state planes must be contiguous")
+            n = len(part)
+            row = [p.stride(1) * p.element_size() for p in part]
+            self._groups.append((n, part, row, (ctypes.c_longlong * n)(*[p.stride(0) * p.element_size() for p in part]),
+                                 (ctypes.c_longlong * n)(*row), (c_int * n)(*[p.shape[0] for p in part])))
+
+    def clear(self, slot: int) -> None:
+        for n, part, row, entry_bytes, row_bytes, entries in self._groups:
+            first = (c_void_p * n)(*[p.data_ptr() + slot * r for p, r in zip(part, row)])
+            _run("hb_clear_rows", n, first, entry_bytes, row_bytes, entries, _stream())
 
 
 _CAST_SRC = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
