@@ -336,6 +336,26 @@ __device__ __forceinline__ void st_bf2(bf16* p, float x, float y) {
   *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y);
 }
 
+// Which sequence a CTA of row z of the grid takes.  With a key range per sequence a full server has more CTAs than the GPU holds, and
+// CTAs start in the order of their index: the longest sequences first, so that none of them is what the last wave waits for.
+// Every CTA ranks the lengths for itself (equal ones by index).  64 sequences of 210 to 2,000 tokens, 8 kv heads, inside steps: two steps of
+// eight layers 3,010 -> 2,866 us.  Up to 16 sequences their keys are cut into ranges, or the CTAs all stand on the GPU at once.
+__device__ __forceinline__ int longest_first(const int* __restrict__ seq_len, int n, int z) {      // n <= AD_THREADS
+  __shared__ int lens[AD_THREADS], chosen;
+  const int mine = threadIdx.x < n ? seq_len[threadIdx.x] : -1;
+  lens[threadIdx.x] = mine;
+  __syncthreads();
+  int rank = 0;
+#pragma unroll 8
+  for (int j = 0; j < n; ++j) {
+    const int o = lens[j];
+    rank += o > mine || (o == mine && j < threadIdx.x);
+  }
+  if (threadIdx.x < n && rank == z) chosen = threadIdx.x;
+  __syncthreads();
+  return chosen;
+}
+
 template <int NH, bool FUSED>
 __global__ void __launch_bounds__(AD_THREADS) attention_decode_km_kernel(DecodeArgs a, DecodeFuse f) {
   constexpr int HD = 128;
@@ -344,7 +364,9 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_km_kernel(DecodeA
   __shared__ int s_last;
   // Before the wait on the kernel before: only what the host wrote ahead of the step (lengths, page
   // tables) and what earlier steps left in the cache.
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int split = blockIdx.x, kvh = blockIdx.y;
+  const bool ranked = a.nsplit == 1 && gridDim.z > 16 && gridDim.z <= AD_THREADS;
+  const int b = ranked ? longest_first(a.seq_len, gridDim.z, blockIdx.z) : blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int G = a.nh / a.nkv;
   constexpr int row_bytes = HD * 2 + 16;
