@@ -38,9 +38,11 @@ void hb_set_error(const char* fmt, ...);
 // still draining; it must then call pdl_wait() before it reads anything the predecessor wrote or
 // writes anything the predecessor may still read.  pdl_launch() tells the hardware that the next
 // kernel may start its own prologue.  It is called after pdl_wait(), so that at most one kernel
-// ahead of the running one sits on the SMs, and in the long decode kernels only when the CTA's own
-// loads are done: CTAs that wait beside working ones cost those issue slots (measured: the step
-// twice as long with the trigger at the start).  Both are no-ops for a kernel launched without the attribute.
+// ahead of the running one sits on the SMs, and in decode attention only when the CTA's own loads are done.  What makes
+// an early start pay or not is where the early CTAs come to stand: those of a kernel that leaves room for several on an SM
+// crowd on the SMs that are free first and keep crowded for their whole length.  The products of few rows (gemm_skinny.cu)
+// fill an SM's shared memory and trigger as soon as their own first loads are out; row kernels that trigger ahead of their wait
+// gained the recurrent designs 1 % and cost those with experts 5 to 20 %.  Both are no-ops for a kernel launched without the attribute.
 int hb_pdl_enabled(void);   // 0 off, 1 every kernel, 2 only the launches that ask for it (hb_launch_pdl)
 template <typename... KArgs, typename... Args>
 static inline cudaError_t hb_launch_ex(int want_pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

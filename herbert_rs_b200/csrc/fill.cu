@@ -70,6 +70,7 @@ __device__ __forceinline__ float rng_normal_from_bits(unsigned long long z) {
 
 template <typename T>
 __global__ void rng_normal_kernel(T* __restrict__ out, long long n, unsigned long long key, float mean, float stdev) {
+  pdl_wait();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const float zn = rng_normal_from_bits(rng_mix(key, (unsigned long long)i));
@@ -98,12 +99,14 @@ extern "C" int hb_rng_normal(int dtype, void* out, long long n, unsigned long lo
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void fill_kernel(T* __restrict__ out, long long n, float value) {
+  pdl_wait();
   const long long stride = (long long)gridDim.x * blockDim.x;
   const T v = from_f32<T>(value);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = v;
 }
 
 __global__ void fill_i32_kernel(int* __restrict__ out, long long n, int value) {
+  pdl_wait();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = value;
 }

@@ -296,8 +296,8 @@ _pdl_mode = None
 def set_pdl(mode: int) -> None:
     """Programmatic dependent launch: 0 off, 1 every kernel, 2 only the launches that ask for it.
     The engine switches it on for eager steps (prompts: the next kernel's CTAs start while the last
-    ones of the kernel before drain, 1-3 % of a prefill) and off for steps it records as CUDA graphs
-    (inside a replayed graph it measured slower); see `options.pdl_eager`."""
+    ones of the kernel before drain, 1-3 % of a prefill) and for steps it records as CUDA graphs (the next product's
+    first weights are under way while its predecessor ends, 3-17 % of a decode step); see `options.pdl_eager`, `options.pdl_graph`."""
     global _pdl_mode
     if _pdl_mode != int(mode):
         _libmod.load().hb_set_pdl(int(mode))

@@ -31,10 +31,10 @@ class KernelOptions:
     decode_ctas_per_sm: int = 2
     # ... and into at most this many key ranges per (sequence, kv head).
     decode_max_splits: int = 16
-    # Programmatic dependent launch for eager steps (prompts); steps recorded as CUDA graphs never use it.
+    # Programmatic dependent launch for eager steps (prompts).
     pdl_eager: bool = True
     # The same inside recorded decode steps: 0 off, 1 every kernel, 2 only the products that load weights before they wait.
-    pdl_graph: int = 0
+    pdl_graph: int = 1
     # Attention over a cached latent, bfloat16: "mma" (tensor cores where the sizes allow: tcgen05 for prompts that give every SM a
     # tile, else mma.sync), or "simt" (the any-shape kernel).
     latent_attention: str = "mma"
