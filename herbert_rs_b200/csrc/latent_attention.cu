@@ -28,23 +28,29 @@ __global__ void latent_kv_store_kernel(const float* __restrict__ kv, int ld, con
                                        const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                                        const int* __restrict__ seq_pages, int pages_stride, T* __restrict__ cache,
                                        int n_tokens, int page_size) {
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int half = rot >> 1;
+  // place and angles hang on what the host wrote: worked out while the kernel before ends
+  const int tok = t < n_tokens ? t : 0;
+  const int p = tok_pos[tok], b = tok_seq[tok];
+  const int page = seq_pages[(size_t)b * pages_stride + p / page_size];
+  float s0 = 0.0f, c0 = 1.0f;
+  if (lane < half) sincosf((float)p * freq[lane], &s0, &c0);
   pdl_wait();
   pdl_launch();
-  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= n_tokens) return;
   const float* row = kv + (size_t)t * ld;
   float ss = 0.0f;
+#pragma unroll 8
   for (int i = lane; i < rank; i += 32) ss += row[i] * row[i];
   ss = warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss / (float)rank + eps);
-  const int p = tok_pos[t], b = tok_seq[t];
-  const int page = seq_pages[(size_t)b * pages_stride + p / page_size];
   T* dst = cache + ((size_t)page * page_size + (p % page_size)) * (size_t)(rank + rot);
+#pragma unroll 8
   for (int i = lane; i < rank; i += 32) dst[i] = from_f32<T>((row[i] * inv) * nw[i]);
-  const int half = rot >> 1;
   for (int i = lane; i < half; i += 32) {
-    float s, c;
-    sincosf((float)p * freq[i], &s, &c);
+    float s = s0, c = c0;
+    if (i >= 32) sincosf((float)p * freq[i], &s, &c);
     s *= mscale;
     c *= mscale;
     const int j0 = rank + (halves ? i : 2 * i), j1 = halves ? j0 + half : j0 + 1;

@@ -117,14 +117,14 @@ __device__ __forceinline__ float head_inv_rms(const float* head, const float* bi
   return 1.0f / sqrtf(warp_sum(s) / (float)n + eps);
 }
 
-// V4: four channels a lane (see turn_channels4).
+// V4: four channels a lane (see turn_channels4).  Positions and pages are the host's and the angles hang on them alone: they are
+// worked out while the kernel before ends.
 template <typename T, bool V4>
-__global__ void __launch_bounds__(256) qkv_rotary_cache_kernel(RotPrepArgs a) {
+__global__ void __launch_bounds__(512) qkv_rotary_cache_kernel(RotPrepArgs a) {
   extern __shared__ __align__(16) float tab[];          // cos and sin of the token's angles: [rot] for q and k, [dv] for values
   __shared__ float red[32];
-  pdl_wait();
-  pdl_launch();
   const int t = blockIdx.x, p = a.tok_pos[t];
+  const int page = a.write_cache ? a.seq_pages[(size_t)a.tok_seq[t] * a.pages_stride + p / a.page_size] : 0;
   const float pos = (float)p;
   float* tab_v = tab + a.rot;
   for (int m = threadIdx.x; m < a.rot / 2; m += blockDim.x) {
@@ -140,6 +140,8 @@ __global__ void __launch_bounds__(256) qkv_rotary_cache_kernel(RotPrepArgs a) {
       tab_v[m] = c;
       tab_v[a.dv / 2 + m] = s;
     }
+  pdl_wait();
+  pdl_launch();
   __syncthreads();
   const int qn = a.nh * a.maps * a.dk, kn = a.nkv * a.maps * a.dk;
   const float* q = a.rows + (size_t)t * a.ld;
@@ -191,7 +193,6 @@ __global__ void __launch_bounds__(256) qkv_rotary_cache_kernel(RotPrepArgs a) {
     }
   }
   if (!a.write_cache) return;
-  const int page = a.seq_pages[(size_t)a.tok_seq[t] * a.pages_stride + p / a.page_size];
   const size_t in_page = (size_t)(p % a.page_size);
   for (int u = warp; u < 2 * a.nkv; u += nwarp) {          // key heads and value heads
     const int g = u >> 1;
@@ -277,35 +278,47 @@ extern "C" int hb_qkv_rotary_cache(int dtype, const float* rows, int ld, const f
   const bool v4 = ((dk | dv | hd | ld | ldq) & 3) == 0 && (in_ptrs & 15) == 0 && (out_ptrs & 15) == 0 && rot % (halves ? 8 : 4) == 0 &&
                   (fv == nullptr || dv % (halves ? 8 : 4) == 0);
   cudaStream_t s = (cudaStream_t)stream;
+  // a decode step's few CTAs take sixteen warps each, so that a warp's heads do not follow one another
+  const int threads = n_tokens <= 128 ? 512 : 256;
   if (dtype == HB_F32) {
-    if (v4) hb_launch(qkv_rotary_cache_kernel<float, true>, dim3(n_tokens), dim3(256), smem, s, a);
-    else hb_launch(qkv_rotary_cache_kernel<float, false>, dim3(n_tokens), dim3(256), smem, s, a);
+    if (v4) hb_launch(qkv_rotary_cache_kernel<float, true>, dim3(n_tokens), dim3(threads), smem, s, a);
+    else hb_launch(qkv_rotary_cache_kernel<float, false>, dim3(n_tokens), dim3(threads), smem, s, a);
   } else {
-    if (v4) hb_launch(qkv_rotary_cache_kernel<bf16, true>, dim3(n_tokens), dim3(256), smem, s, a);
-    else hb_launch(qkv_rotary_cache_kernel<bf16, false>, dim3(n_tokens), dim3(256), smem, s, a);
+    if (v4) hb_launch(qkv_rotary_cache_kernel<bf16, true>, dim3(n_tokens), dim3(threads), smem, s, a);
+    else hb_launch(qkv_rotary_cache_kernel<bf16, false>, dim3(n_tokens), dim3(threads), smem, s, a);
   }
   HB_CHECK_LAUNCH("qkv_rotary_cache");
   return 0;
 }
 
 // ---------------------------------------------------------------------------------------------
+// The angles are worked out once a token, while the kernel before ends; all heads share them.
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(512)
 rotate_heads_back_kernel(const T* __restrict__ att, int ld, int hd, const float* __restrict__ fv, int halves,
-                         const int* __restrict__ tok_pos, T* __restrict__ y, int ldy, int nh, int dv) {
-  pdl_wait();
-  pdl_launch();
+                         const int* __restrict__ tok_pos, T* __restrict__ y, int ldy, int nh, int dv, int tabled) {
+  extern __shared__ float turns[];                       // [half] sines, [half] cosines
   const int t = blockIdx.x;
   const float pos = (float)tok_pos[t];
   const T* ar = att + (size_t)t * ld;
   T* yr = y + (size_t)t * ldy;
   const int half = dv >> 1;
+  for (int m = threadIdx.x; tabled && m < half; m += blockDim.x) {
+    float s = 0.0f, c = 1.0f;
+    if (fv) sincosf(pos * fv[m], &s, &c);
+    turns[m] = s;
+    turns[half + m] = c;
+  }
+  pdl_wait();
+  pdl_launch();
+  __syncthreads();
   for (int i = threadIdx.x; i < nh * half; i += blockDim.x) {
     const int h = i / half, m = i - h * half;
     const int j0 = halves ? m : 2 * m, j1 = halves ? m + half : 2 * m + 1;
     const float u = to_f32(ar[(size_t)h * hd + j0]), w = to_f32(ar[(size_t)h * hd + j1]);
     float s = 0.0f, c = 1.0f;
-    if (fv) sincosf(pos * fv[m], &s, &c);
+    if (tabled) { s = turns[m]; c = turns[half + m]; }
+    else if (fv) sincosf(pos * fv[m], &s, &c);
     // the turn by -a
     yr[(size_t)h * dv + j0] = from_f32<T>(u * c + w * s);
     yr[(size_t)h * dv + j1] = from_f32<T>(w * c - u * s);
@@ -316,12 +329,15 @@ extern "C" int hb_rotate_heads_back(int dtype, const void* att, int ld, int hd, 
                                     void* y, int ldy, int n_tokens, int nh, int dv, void* stream) {
   HB_REQUIRE(n_tokens > 0 && nh > 0 && dv > 0 && hd >= dv, "rotate_heads_back: sizes must be positive and heads wide enough");
   HB_REQUIRE(dv % 2 == 0, "rotate_heads_back: values of %d channels have no pairs", dv);
+  const int threads = n_tokens <= 128 ? 512 : 128;
+  const int tabled = (size_t)dv * sizeof(float) <= 48 * 1024;
+  const size_t smem = tabled ? (size_t)dv * sizeof(float) : 0;
   if (dtype == HB_F32)
-    hb_launch(rotate_heads_back_kernel<float>, dim3(n_tokens), dim3(128), 0, (cudaStream_t)stream, (const float*)att, ld, hd, fv,
-              halves, tok_pos, (float*)y, ldy, nh, dv);
+    hb_launch(rotate_heads_back_kernel<float>, dim3(n_tokens), dim3(threads), smem, (cudaStream_t)stream, (const float*)att, ld, hd, fv,
+              halves, tok_pos, (float*)y, ldy, nh, dv, tabled);
   else
-    hb_launch(rotate_heads_back_kernel<bf16>, dim3(n_tokens), dim3(128), 0, (cudaStream_t)stream, (const bf16*)att, ld, hd, fv,
-              halves, tok_pos, (bf16*)y, ldy, nh, dv);
+    hb_launch(rotate_heads_back_kernel<bf16>, dim3(n_tokens), dim3(threads), smem, (cudaStream_t)stream, (const bf16*)att, ld, hd, fv,
+              halves, tok_pos, (bf16*)y, ldy, nh, dv, tabled);
   HB_CHECK_LAUNCH("rotate_heads_back");
   return 0;
 }
