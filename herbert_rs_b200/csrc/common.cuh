@@ -80,6 +80,11 @@ static inline cudaError_t hb_launch_after(void (*kernel)(KArgs...), dim3 grid, d
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Asks for `bytes` bytes from p into L2, a line a lane (a whole warp calls it): weights that a kernel reads after its wait.
+__device__ __forceinline__ void warp_prefetch_l2(const void* p, size_t bytes) {
+  for (size_t b = (threadIdx.x & 31) * 128; b < bytes; b += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)p + b));
+}
+
 // ---- conversions ---------------------------------------------------------------------------
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(bf16 v) { return __bfloat162float(v); }

@@ -50,9 +50,13 @@ __global__ void __launch_bounds__(GP_MAX_THREADS) general_delta_prepare_kernel(G
   extern __shared__ float lows[];   // [GP_TOK][rank]
   __shared__ float red[GP_TOK][GP_MAX_THREADS / 32];
   __shared__ float inv[GP_TOK];
+  const int t0 = blockIdx.x * GP_TOK, h = blockIdx.y;
+  if (a.n_tokens <= 64) {      // a decode step: the head's rows of w2, one piece of memory, come while the kernel before ends
+    const size_t bytes = (size_t)a.dk * a.rank * sizeof(T), part = (bytes / (blockDim.x >> 5) + 127) & ~(size_t)127, from = (threadIdx.x >> 5) * part;
+    if (from < bytes) warp_prefetch_l2((const char*)a.w2 + (size_t)h * bytes + from, bytes - from < part ? bytes - from : part);
+  }
   pdl_wait();
   pdl_launch();
-  const int t0 = blockIdx.x * GP_TOK, h = blockIdx.y;
   const int nt = a.n_tokens - t0 < GP_TOK ? a.n_tokens - t0 : GP_TOK;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
   for (int i = threadIdx.x; i < nt * a.rank; i += blockDim.x) {
@@ -91,7 +95,24 @@ __global__ void __launch_bounds__(GP_MAX_THREADS) general_delta_prepare_kernel(G
     const float z0 = a.w0[c], a0 = a.a0[c];
 #pragma unroll
     for (int tt = 0; tt < GP_TOK; ++tt) z[tt] = z0;
-    for (int j = 0; j < a.rank; ++j) {
+    // sixteen weights at a time where rows are whole pieces of 16 bytes: a weight at a time is a way to L1 each
+    constexpr int VE = 16 / (int)sizeof(T);
+    int j = 0;
+    if (a.rank % VE == 0 && ((uintptr_t)w2 & 15) == 0)
+      for (; j + 16 <= a.rank; j += 16) {
+        uint4 v[16 / VE];
+#pragma unroll
+        for (int q = 0; q < 16 / VE; ++q) v[q] = *reinterpret_cast<const uint4*>(wr + j + q * VE);
+        const T* e = reinterpret_cast<const T*>(v);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const float w = to_f32(e[q]);
+#pragma unroll
+          for (int tt = 0; tt < GP_TOK; ++tt)
+            if (tt < nt) z[tt] = fmaf(lows[tt * a.rank + j + q], w, z[tt]);
+        }
+      }
+    for (; j < a.rank; ++j) {
       const float w = to_f32(wr[j]);
 #pragma unroll
       for (int tt = 0; tt < GP_TOK; ++tt)

@@ -19,14 +19,17 @@
 // low-rank rows it keeps in shared memory, and a thread one channel: it reads its row of W2 once for all of them.
 #define GD_TOK 8
 #define GD_THREADS 128
+#define GD_PREFETCH_TOKENS 64      // decode steps: a prompt's CTAs share the rows anyway
 template <typename T>
 __global__ void __launch_bounds__(GD_THREADS)
 gla_decay_kernel(const float* __restrict__ low, int ld, const T* __restrict__ w2, const float* __restrict__ bias,
                  float inv_tau, float* __restrict__ a, int n_tokens, int C, int R) {
   extern __shared__ float lows[];  // [GD_TOK][R]
+  const int t0 = blockIdx.y * GD_TOK, c = blockIdx.x * GD_THREADS + threadIdx.x;
+  if (n_tokens <= GD_PREFETCH_TOKENS && (c & ~31) < C)      // this warp's rows of W2 come while the kernel before ends
+    warp_prefetch_l2(w2 + (size_t)(c & ~31) * R, (size_t)(C - (c & ~31) < 32 ? C - (c & ~31) : 32) * R * sizeof(T));
   pdl_wait();
   pdl_launch();
-  const int t0 = blockIdx.y * GD_TOK, c = blockIdx.x * GD_THREADS + threadIdx.x;
   const int nt = n_tokens - t0 < GD_TOK ? n_tokens - t0 : GD_TOK;
   for (int i = threadIdx.x; i < nt * R; i += GD_THREADS) lows[i] = low[(size_t)(t0 + i / R) * ld + i % R];
   __syncthreads();
@@ -36,7 +39,24 @@ gla_decay_kernel(const float* __restrict__ low, int ld, const T* __restrict__ w2
   const float b = bias ? bias[c] : 0.0f;
 #pragma unroll
   for (int i = 0; i < GD_TOK; ++i) z[i] = b;
-  for (int r = 0; r < R; ++r) {
+  // sixteen weights at a time where rows are whole pieces of 16 bytes: a weight at a time is a way to L1 each
+  constexpr int VE = 16 / (int)sizeof(T);
+  int r = 0;
+  if (R % VE == 0 && ((uintptr_t)w2 & 15) == 0)
+    for (; r + 16 <= R; r += 16) {
+      uint4 v[16 / VE];
+#pragma unroll
+      for (int q = 0; q < 16 / VE; ++q) v[q] = *reinterpret_cast<const uint4*>(wr + r + q * VE);
+      const T* e = reinterpret_cast<const T*>(v);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        const float w = to_f32(e[q]);
+#pragma unroll
+        for (int i = 0; i < GD_TOK; ++i)
+          if (i < nt) z[i] = fmaf(lows[i * R + r + q], w, z[i]);
+      }
+    }
+  for (; r < R; ++r) {
     const float w = to_f32(wr[r]);
 #pragma unroll
     for (int i = 0; i < GD_TOK; ++i)

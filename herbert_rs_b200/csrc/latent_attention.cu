@@ -144,11 +144,12 @@ __global__ void __launch_bounds__(HW_WARPS * 32)
 headwise_dot_kernel(const float* __restrict__ in, int ld_in, int in_hs, const TW* __restrict__ w, TO* __restrict__ out,
                     int ld_out, int out_hs, const float* __restrict__ gate, int ld_gate, int n_tokens, int K, int N,
                     float scale, int vec) {
+  const int lane = threadIdx.x & 31, n = blockIdx.x * HW_WARPS + (threadIdx.x >> 5), h = blockIdx.y, t0 = blockIdx.z * HW_TT;
+  const TW* wr = w + ((size_t)h * N + n) * K;
+  if (n < N) warp_prefetch_l2(wr, (size_t)K * sizeof(TW));      // while the kernel before ends
   pdl_wait();
   pdl_launch();
-  const int lane = threadIdx.x & 31, n = blockIdx.x * HW_WARPS + (threadIdx.x >> 5), h = blockIdx.y, t0 = blockIdx.z * HW_TT;
   if (n >= N) return;
-  const TW* wr = w + ((size_t)h * N + n) * K;
   const float* a0 = in + (size_t)t0 * ld_in + (size_t)h * in_hs;
   const int nt = n_tokens - t0 < HW_TT ? n_tokens - t0 : HW_TT;
   float acc[HW_TT];

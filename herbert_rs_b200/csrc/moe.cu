@@ -193,9 +193,11 @@ moe_route_tile_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr,
   const int pieces = D / VE;
   float* sc = reinterpret_cast<float*>(hs + (size_t)TT * pieces);
   float* gs = sc + TT * E;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = blockIdx.x * TT;
+  if (TT == 1 && 2 * warp < E)                          // a decode step: this warp's first weight rows come while the kernel before ends
+    warp_prefetch_l2(wr + (size_t)(2 * warp) * D, (size_t)(2 * warp + 1 < E ? 2 : 1) * D * sizeof(T));
   pdl_wait();
   pdl_launch();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = blockIdx.x * TT;
   const int nt = n_tokens - t0 < TT ? n_tokens - t0 : TT;
   for (int i = threadIdx.x; i < TT * pieces; i += W * 32) {      // all of them on their way before the first is waited for
     const int tt = TT == 1 ? 0 : i / pieces;
