@@ -234,7 +234,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int buf = local & 1;
       const int m0 = (tile % tiles_m) * TG_BM, n0 = (tile / tiles_m) * BN;
       const int m = m0 + quad * 32 + lane;
-      float inv_rms = 1.0f, sq = 0.0f, sq8[8] = {};
+      float inv_rms = 1.0f, sq = 0.0f;
       if (NORM && nm.in_sumsq != nullptr && m < M) {         // while the tensor cores still work on this tile
         float sum = 0.0f;
         for (int i = 0; i < nm.in_parts; ++i) sum += nm.in_sumsq[(size_t)i * nm.in_stride + m];
@@ -323,13 +323,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(acc[j]);
         }
-        if (turned && n0 + c * 32 + 32 <= N) tg_epilogue32_turned<EPI, NORM>(r, turn, m - lane, n0 + c * 32, M, Cv, ldc, nm, inv_rms, sq8);
+        if (turned && n0 + c * 32 + 32 <= N) tg_epilogue32_turned<EPI, NORM>(r, turn, m - lane, n0 + c * 32, M, Cv, ldc, nm, inv_rms, sq);
         else tg_epilogue32<EPI, NORM>(r, m, n0 + c * 32, M, N, Cv, ldc, nm, inv_rms, sq);
       }
-      if (NORM && EPI == HB_EPI_RESIDUAL && nm.out_w != nullptr) {
-        sq += tg_row_sums(sq8);
-        if (m < M) nm.out_sumsq[(size_t)(2 * (tile / tiles_m) + (c_lo > 0)) * nm.out_stride + m] = sq;
-      }
+      if (NORM && EPI == HB_EPI_RESIDUAL && nm.out_w != nullptr && m < M)
+        nm.out_sumsq[(size_t)(2 * (tile / tiles_m) + (c_lo > 0)) * nm.out_stride + m] = sq;
     }
   }
   tc_fence_before();
@@ -587,7 +585,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int buf = local & 1;
       const int m0 = (tile % tiles_m) * 2 * TG_BM + (int)rank * TG_BM, n0 = (tile / tiles_m) * BN;
       const int m = m0 + quad * 32 + lane;
-      float inv_rms = 1.0f, sq = 0.0f, sq8[8] = {};
+      float inv_rms = 1.0f, sq = 0.0f;
       if (NORM && nm.in_sumsq != nullptr && m < M) {
         float sum = 0.0f;
         for (int i = 0; i < nm.in_parts; ++i) sum += nm.in_sumsq[(size_t)i * nm.in_stride + m];
@@ -616,14 +614,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(acc_empty0);
           }
-          if (turned && n0 + c * 32 + 32 <= N) tg_epilogue32_turned<EPI, NORM>(r, turn, m - lane, n0 + c * 32, M, Cv, ldc, nm, inv_rms, sq8);
+          if (turned && n0 + c * 32 + 32 <= N) tg_epilogue32_turned<EPI, NORM>(r, turn, m - lane, n0 + c * 32, M, Cv, ldc, nm, inv_rms, sq);
           else tg_epilogue32<EPI, NORM>(r, m, n0 + c * 32, M, N, Cv, ldc, nm, inv_rms, sq);
         }
       }
-      if (NORM && EPI == HB_EPI_RESIDUAL && nm.out_w != nullptr) {
-        sq += tg_row_sums(sq8);
-        if (m < M) nm.out_sumsq[(size_t)(2 * (tile / tiles_m) + (c_lo > 0)) * nm.out_stride + m] = sq;
-      }
+      if (NORM && EPI == HB_EPI_RESIDUAL && nm.out_w != nullptr && m < M)
+        nm.out_sumsq[(size_t)(2 * (tile / tiles_m) + (c_lo > 0)) * nm.out_stride + m] = sq;
     }
   }
   tc_fence_before();

@@ -190,6 +190,9 @@ __device__ __forceinline__ float4 tg_turn_out(unsigned st, int row, int q) {    
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(st + row * 128 + ((q ^ (row & 7)) << 4)) : "memory");
   return v;
 }
+__device__ __forceinline__ void tg_turn_back(unsigned st, int row, int q, float4 v) {  // ... put back into their place
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(st + row * 128 + ((q ^ (row & 7)) << 4)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
 
 // Whether the outputs' rows can be reached 16 bytes (float) or 8 columns (bfloat16) at a time.
 template <int EPI, bool NORM>
@@ -201,10 +204,11 @@ __device__ __forceinline__ bool tg_rows_aligned(const void* Cv, int ldc, const T
          (!begin_norm || (nm.out_ld % 4 == 0 && ((uintptr_t)nm.out_xw & 7) == 0 && ((uintptr_t)nm.out_w & 15) == 0));
 }
 
-// 32 whole columns (n ..) of rows m0 .. m0 + 31, this lane's row in r; sq8[i]: this lane's share of row 4 i + lane / 8's sum of squares.
+// 32 whole columns (n ..) of rows m0 .. m0 + 31, this lane's row in r and that row's sum of squares in sq.  The sums are added column by column,
+// as above, so that a row's norm has the same bits whichever way its columns went: the updated rows go round a second time.
 template <int EPI, bool NORM>
 __device__ __forceinline__ void tg_epilogue32_turned(const unsigned (&r)[32], unsigned st, int m0, int n, int M, void* Cv, int ldc,
-                                                     const TgNorm& nm, float inv_rms, float (&sq8)[8]) {
+                                                     const TgNorm& nm, float inv_rms, float& sq) {
   const int lane = threadIdx.x & 31;
   float v[32];
 #pragma unroll
@@ -242,28 +246,23 @@ __device__ __forceinline__ void tg_epilogue32_turned(const unsigned (&r)[32], un
         }
         *reinterpret_cast<float4*>(out + (size_t)(4 * i) * ldc) = x;
         if (begin_norm) {
-          sq8[i] += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+          tg_turn_back(st, 4 * i + row0, q, x);
           *reinterpret_cast<uint2*>(nm.out_xw + (size_t)(m0 + 4 * i + row0) * nm.out_ld + n + 4 * q) = make_uint2(pack2(x.x * w4.x, x.y * w4.y), pack2(x.z * w4.z, x.w * w4.w));
         }
       }
     }
-  }
-}
-
-// The eight lanes' shares of each row's sum of squares, added and brought to the lane that owns the row.
-__device__ __forceinline__ float tg_row_sums(float (&sq8)[8]) {
-  const int lane = threadIdx.x & 31;
-  float mine = 0.0f;
+    if (begin_norm) {
+      __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float t = sq8[i];
-    t += __shfl_xor_sync(0xffffffffu, t, 1);
-    t += __shfl_xor_sync(0xffffffffu, t, 2);
-    t += __shfl_xor_sync(0xffffffffu, t, 4);
-    t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);
-    if ((lane >> 2) == i) mine = t;
+      for (int i = 0; i < 8; ++i) {
+        const float4 x = tg_turn_out(st, lane, i);
+        sq = fmaf(x.x, x.x, sq);
+        sq = fmaf(x.y, x.y, sq);
+        sq = fmaf(x.z, x.z, sq);
+        sq = fmaf(x.w, x.w, sq);
+      }
+    }
   }
-  return mine;
 }
 
 // The same for 8 consecutive output columns whose float results are in v (store, store as float, add
