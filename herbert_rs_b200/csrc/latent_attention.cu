@@ -55,8 +55,9 @@ __global__ void latent_kv_store_kernel(const float* __restrict__ kv, int ld, con
     c *= mscale;
     const int j0 = rank + (halves ? i : 2 * i), j1 = halves ? j0 + half : j0 + 1;
     const float u = row[j0], v = row[j1];
-    dst[j0] = from_f32<T>(u * c - v * s);
-    dst[j1] = from_f32<T>(v * c + u * s);
+    // spelt out: which product is rounded first must not hang on how the compiler reads the lines around
+    dst[j0] = from_f32<T>(fmaf(u, c, -(v * s)));
+    dst[j1] = from_f32<T>(fmaf(v, c, u * s));
   }
 }
 

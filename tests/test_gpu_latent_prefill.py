@@ -132,3 +132,28 @@ def test_a_prompt_on_both_sides_of_the_rule(H, rank, rot, below, above):
     # both round the softmax weights to bfloat16 (2^-8 of each), each at its own scale
     bound = torch.einsum("thj,jr->thr", p, cache.view(-1, W)[:below, :rank].double().abs()) * 2.0 ** -7 + 1e-5
     assert ((outs[0] - outs[1]).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("halves", [True, False])
+@pytest.mark.parametrize("rank,rot", [(512, 64), (40, 6), (64, 80)])
+def test_the_rotated_key_rounds_its_second_product_first(rank, rot, halves):
+    """u c - v s and v c + u s with the product of s rounded and the other one taken exactly (a multiply-add): the same bits however the
+    kernel around is written.  float64 holds the exact product and the sum closely enough to be rounded once to float, but for ties
+    at its 53rd bit: none in these numbers."""
+    T, page, P = 500, 64, 8
+    g = torch.Generator(DEV).manual_seed(rot)
+    kv = torch.randn(T, rank + rot, device=DEV, generator=g)
+    freq = (10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) * 2 / rot)).float().to(DEV)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    cache = torch.zeros(P, 1, page, rank + rot, device=DEV)
+    mscale = 1.25
+    ops.latent_kv_store(kv, torch.ones(rank, device=DEV), 1e-6, freq, mscale, rank, rot, torch.zeros_like(pos), pos,
+                        torch.arange(P, dtype=torch.int32, device=DEV).view(1, P), cache, page, halves=halves)
+    ang = pos.float()[:, None] * freq
+    s, c = torch.sin(ang) * mscale, torch.cos(ang) * mscale
+    r = kv[:, rank:]
+    u, v = (r[:, :rot // 2], r[:, rot // 2:]) if halves else (r[:, 0::2], r[:, 1::2])
+    got = cache.view(-1, rank + rot)[:T, rank:]
+    a, b = (got[:, :rot // 2], got[:, rot // 2:]) if halves else (got[:, 0::2], got[:, 1::2])
+    assert torch.equal(a, (u.double() * c.double() - (v * s).double()).float())
+    assert torch.equal(b, (v.double() * c.double() + (u * s).double()).float())
