@@ -122,7 +122,7 @@ __device__ __forceinline__ float head_inv_rms(const float* head, const float* bi
 template <typename T, bool V4>
 __global__ void __launch_bounds__(512) qkv_rotary_cache_kernel(RotPrepArgs a) {
   extern __shared__ __align__(16) float tab[];          // cos and sin of the token's angles: [rot] for q and k, [dv] for values
-  __shared__ float red[32];
+  __shared__ float red[16];
   const int t = blockIdx.x, p = a.tok_pos[t];
   const int page = a.write_cache ? a.seq_pages[(size_t)a.tok_seq[t] * a.pages_stride + p / a.page_size] : 0;
   const float pos = (float)p;
@@ -151,18 +151,27 @@ __global__ void __launch_bounds__(512) qkv_rotary_cache_kernel(RotPrepArgs a) {
   const float* bk = a.bias ? a.bias + qn : nullptr;
   const float* bv = a.bias ? a.bias + qn + kn : nullptr;
   float inv_q = 1.0f, inv_k = 1.0f;
-  if (a.norm == 1) {
+  if (a.norm == 1) {      // each sum by 256 threads, whatever the step's size: a token's bits do not hang on how many tokens come with it
     float sq = 0.0f, sk = 0.0f;
-    for (int i = threadIdx.x; i < qn; i += blockDim.x) {
-      const float x = q[i] + (bq ? bq[i] : 0.0f);
-      sq = fmaf(x, x, sq);
-    }
-    for (int i = threadIdx.x; i < kn; i += blockDim.x) {
-      const float x = k[i] + (bk ? bk[i] : 0.0f);
-      sk = fmaf(x, x, sk);
-    }
-    sq = block_sum(sq, red);
-    sk = block_sum(sk, red);
+    const bool for_q = threadIdx.x < 256, for_k = threadIdx.x + 256 >= blockDim.x;
+    if (for_q)
+      for (int i = threadIdx.x; i < qn; i += 256) {
+        const float x = q[i] + (bq ? bq[i] : 0.0f);
+        sq = fmaf(x, x, sq);
+      }
+    if (for_k)
+      for (int i = threadIdx.x & 255; i < kn; i += 256) {
+        const float x = k[i] + (bk ? bk[i] : 0.0f);
+        sk = fmaf(x, x, sk);
+      }
+    sq = warp_sum(sq);
+    sk = warp_sum(sk);
+    const int w8 = (threadIdx.x >> 5) & 7, l = threadIdx.x & 31;
+    if (l == 0 && for_q) red[w8] = sq;
+    if (l == 0 && for_k) red[8 + w8] = sk;
+    __syncthreads();
+    sq = warp_sum(l < 8 ? red[l] : 0.0f);
+    sk = warp_sum(l < 8 ? red[8 + l] : 0.0f);
     inv_q = 1.0f / sqrtf(sq / (float)qn + a.eps);
     inv_k = 1.0f / sqrtf(sk / (float)kn + a.eps);
   }

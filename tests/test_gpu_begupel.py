@@ -680,3 +680,24 @@ def test_command_line_trace_replay_and_prompts_in_pieces(mixed, tmp_path, capsys
                           hb.SamplingParams(temperature=0.8, top_k=20, top_p=0.95, seed=5))
         outs.append(res.tokens)
     assert outs[0] == outs[1]
+
+
+def test_a_token_is_normed_to_the_same_bits_in_small_and_large_steps():
+    """Steps of few tokens take more threads a token: the sums behind the norm of the whole projection must be the same ones."""
+    g = torch.Generator().manual_seed(8)
+    H, G, dk, T, page = 16, 8, 128, 150, 64
+    rows = torch.randn(T, (H + 2 * G) * dk, generator=g).to(DEV)
+    wq, wk = (1 + 0.2 * torch.randn(H * dk, generator=g)).to(DEV), (1 + 0.2 * torch.randn(G * dk, generator=g)).to(DEV)
+    fqk = P.pair_frequencies(10000.0, 64, torch.float64).float().to(DEV)
+    pages = torch.arange(3, dtype=torch.int32, device=DEV).view(1, 3)
+
+    def run(cuts):
+        cache = torch.zeros(2, 3, G, page, dk, device=DEV)
+        q = torch.zeros(T, H * dk, device=DEV)
+        for a, b in zip(cuts, cuts[1:]):
+            batch = SimpleNamespace(tok_seq=i32([0] * (b - a)), tok_pos=i32(list(range(a, b))))
+            ops.qkv_rotary_cache(rows[a:b], wq, wk, 1e-5, fqk, 64, True, None, batch, pages, q[a:b], cache[0], cache[1], H, G, dk, dk, dk, page)
+        return q, cache
+
+    whole, parts = run([0, T]), run([0, 1, 30, T])
+    assert torch.equal(whole[0], parts[0]) and torch.equal(whole[1], parts[1])
