@@ -684,9 +684,9 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_km_kernel(DecodeA
 
 // out[b][h][:] = sum_s e^{m_s - m} O_s / sum_s e^{m_s - m} l_s.  A sink (a number per head) joins the
 // denominator here, once, whatever the number of splits: m covers it and e^{sink - m} is added.
-__global__ void attention_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void attention_decode_combine_kernel(const float* part_o, const float* part_ml,
                                                 bf16* __restrict__ out, int ldo, int nh, int hd, int nsplit,
-                                                const float* __restrict__ sink, int gated, const float* __restrict__ out_gate,
+                                                const float* __restrict__ sink, int gated, const float* out_gate,
                                                 int ldg) {
   pdl_wait();
   pdl_launch();
@@ -737,7 +737,7 @@ struct DecodeDifference {
   float lambda, factor, eps;
   int dv;                    // 0: every query head on its own
 };
-__global__ void attention_decode_difference_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void attention_decode_difference_kernel(const float* part_o, const float* part_ml,
                                                    bf16* __restrict__ out, int ldo, int nh, int hd, int nsplit,
                                                    DecodeDifference df) {
   extern __shared__ float sh[];          // [2][nsplit] factors of the key ranges, then [dv]

@@ -26,7 +26,7 @@ template <typename T> __device__ __forceinline__ float tanh_of(float z) {
 // V: channels per thread (4: every pointer on 16 bytes and every row length a multiple of 4).
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-residual_tanh_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ yb, float mult, float* x, const int* __restrict__ rows,
+residual_tanh_kernel(const float* y, int ldy, const float* __restrict__ yb, float mult, float* x, const int* __restrict__ rows,
                      TanhNorm n1, TanhNorm n2, int dim, long long total) {
   pdl_wait();
   pdl_launch();

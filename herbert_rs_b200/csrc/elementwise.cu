@@ -14,7 +14,7 @@
 
 // ---------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void embed_kernel(const T* __restrict__ table, const int* __restrict__ ids,
+__global__ void embed_kernel(const T* __restrict__ table, const int* ids,
                              float* __restrict__ out, int copies, int hidden, int vocab, float scale,
                              const T* __restrict__ pos_table, const int* __restrict__ positions, int n_positions) {
   pdl_wait();
@@ -44,7 +44,7 @@ __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict_
 // The same, 16 bytes of the table a thread: where hidden allows it and all rows start on 16 bytes.
 template <typename T>
 __global__ void __launch_bounds__(1024)
-embed_row_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ out, int copies, int hidden, int vocab, float scale,
+embed_row_kernel(const T* __restrict__ table, const int* ids, float* __restrict__ out, int copies, int hidden, int vocab, float scale,
                  const T* __restrict__ pos_table, const int* __restrict__ positions, int n_positions) {
   constexpr int E = 16 / (int)sizeof(T);
   pdl_wait();
@@ -102,7 +102,7 @@ extern "C" int hb_embed(int dtype, const void* table, const int* ids, float* out
 // ---------------------------------------------------------------------------------------------
 // One block per output row.  rows == nullptr: row r of x; else row rows[r] of x (gather).
 template <typename T>
-__global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void rmsnorm_kernel(const float* x, const float* __restrict__ w,
                                T* __restrict__ out, const int* __restrict__ rows, int dim, float eps) {
   __shared__ float red[32];
   pdl_wait();
@@ -132,7 +132,7 @@ __device__ __forceinline__ void store4(bf16* o, float4 v) {
   *reinterpret_cast<uint2*>(o) = u;
 }
 template <typename T>
-__global__ void rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void rmsnorm_vec_kernel(const float* x, const float* __restrict__ w,
                                    T* __restrict__ out, const int* __restrict__ rows, int dim, float eps) {
   __shared__ float red[32];
   pdl_wait();
@@ -188,7 +188,7 @@ extern "C" int hb_rmsnorm(int dtype, const float* x, const float* w, void* out, 
 // up columns [inter, 2*inter).  interleave == 8: blocks of 16 columns, 8 gate then 8 up.
 // out = act(gate) * up; act: silu, gelu in its tanh or erf form, or relu (HB_ACT_*).
 template <typename T>
-__global__ void swiglu_kernel(const T* __restrict__ gu, int ld, T* __restrict__ out, int ldo,
+__global__ void swiglu_kernel(const T* gu, int ld, T* __restrict__ out, int ldo,
                               int inter, int interleave, int act) {
   pdl_wait();
   pdl_launch();
@@ -220,7 +220,7 @@ __device__ __forceinline__ float glu_act(float g, int act) {
          : act == HB_ACT_RELU    ? fmaxf(g, 0.0f)
                                  : g / (1.0f + expf(-g));
 }
-__global__ void swiglu8_bf16_kernel(const bf16* __restrict__ gu, int ld, bf16* __restrict__ out, int ldo, int groups, int act) {
+__global__ void swiglu8_bf16_kernel(const bf16* gu, int ld, bf16* __restrict__ out, int ldo, int groups, int act) {
   pdl_wait();
   pdl_launch();
   const int t = blockIdx.y, grp = blockIdx.x * blockDim.x + threadIdx.x;
@@ -521,7 +521,7 @@ extern "C" int hb_qk_norm_rope_cache(int dtype, void* qkv, int ld, const float* 
 // ---------------------------------------------------------------------------------------------
 // residual[t, :] += y[t, :] (for parts that cannot fuse the sum into their last product)
 template <typename T>
-__global__ void add_residual_kernel(float* __restrict__ res, const T* __restrict__ y, int ld, int dim) {
+__global__ void add_residual_kernel(float* res, const T* y, int ld, int dim) {
   pdl_wait();
   pdl_launch();
   const int t = blockIdx.y;
@@ -543,7 +543,7 @@ extern "C" int hb_add_residual(int dtype, float* res, const void* y, int ld, int
 // Finishes a norm that a product left half done: out = xw / rms, with rms^2 = sum of the row's
 // partial sums / dim + eps (xw = x * w in bfloat16, sumsq [parts][stride]).  For consumers that
 // cannot apply the row factor themselves.
-__global__ void finish_norm_kernel(const bf16* __restrict__ xw, int ld, const float* __restrict__ sumsq, int parts,
+__global__ void finish_norm_kernel(const bf16* xw, int ld, const float* sumsq, int parts,
                                    int stride, float eps, bf16* __restrict__ out, int ldo, int dim) {
   __shared__ float red[32];
   pdl_wait();

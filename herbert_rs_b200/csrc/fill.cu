@@ -178,7 +178,7 @@ __device__ __forceinline__ float cast_in(const __half* p, long long i) { return 
 // which is what the reference does to every F32 tensor it loads.  Also used inside a step (the
 // residual stream as a sublayer's input), so it waits for the kernel before it like every step kernel.
 template <typename S, typename D>
-__global__ void cast_kernel(const S* __restrict__ in, D* __restrict__ out, long long n, int round_bf16) {
+__global__ void cast_kernel(const S* in, D* __restrict__ out, long long n, int round_bf16) {
   pdl_wait();
   pdl_launch();
   const long long stride = (long long)gridDim.x * blockDim.x;

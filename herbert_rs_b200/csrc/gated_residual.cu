@@ -125,8 +125,8 @@ extern "C" int hb_gated_norm_residual(int dtype, const float* y, int ldy, const 
 
 // ---------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void token_gate_kernel(const float* __restrict__ s, int lds, const T* __restrict__ table, int ldt, int col0,
-                                  const int* __restrict__ ids, T* __restrict__ out, int ldo, int n_tokens, int m, int vocab) {
+__global__ void token_gate_kernel(const float* s, int lds, const T* __restrict__ table, int ldt, int col0,
+                                  const int* ids, T* __restrict__ out, int ldo, int n_tokens, int m, int vocab) {
   pdl_wait();
   pdl_launch();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

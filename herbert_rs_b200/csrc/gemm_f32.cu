@@ -29,7 +29,7 @@ __device__ __forceinline__ float4 f32_load4(const float* row, int k, int end) {
 #define FR_WARPS 8
 template <int MT, int R, int EPI, int V>
 __global__ void __launch_bounds__(FR_WARPS * 32)
-gemm_f32_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* C, int ldc,
+gemm_f32_rows_kernel(const float* A, int lda, const float* __restrict__ W, int ldw, float* C, int ldc,
                      int M, int N, int K, int kw) {
   static_assert(R * MT == 32 || R * MT == 64, "the halving exchange ends with one or two sums a lane");
   constexpr int KEEP = R * MT / 32;
@@ -143,7 +143,7 @@ __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a
 
 template <int EPI, int V>
 __global__ void __launch_bounds__(FT_THREADS)
-gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* C, int ldc,
+gemm_f32_tile_kernel(const float* A, int lda, const float* __restrict__ W, int ldw, float* C, int ldc,
                      int M, int N, int K, int S, int k_per) {
   __shared__ __align__(16) float sh[FT_M * FT_N > 2 * FT_STAGE ? FT_M * FT_N : 2 * FT_STAGE];
   pdl_wait();

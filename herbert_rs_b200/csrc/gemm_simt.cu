@@ -18,7 +18,7 @@ int hb_gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int 
 
 template <typename T, int EPI>
 __global__ void __launch_bounds__(256)
-gemm_simt_kernel(const T* __restrict__ A, int lda, const T* __restrict__ W, int ldw, void* Cv, int ldc,
+gemm_simt_kernel(const T* A, int lda, const T* __restrict__ W, int ldw, void* Cv, int ldc,
                  int M, int N, int K) {
   __shared__ float As[TK][TM + 4];
   __shared__ float Ws[TK][TN + 4];

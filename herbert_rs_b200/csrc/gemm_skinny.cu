@@ -66,7 +66,7 @@ struct SkinnyNorm {
 // of 32 per batch of loads; `depth` batches (2, 3 or 6) are in flight.
 template <int NT, int RG, int UNROLL, int EPI, bool NORM>
 __global__ void __launch_bounds__(SK_THREADS, (NT * RG <= 2) ? 3 : 2)
-gemm_skinny_kernel(const bf16* __restrict__ A, int lda, const bf16* __restrict__ W, int ldw, void* Cv, int ldc,
+gemm_skinny_kernel(const bf16* A, int lda, const bf16* __restrict__ W, int ldw, void* Cv, int ldc,
                    int M, int N, int K, int units_per_cta, int depth, SkinnyNorm nm) {
   // A unit is 16 * RG weight rows.  A CTA walks units_per_cta consecutive units, so that the grid is
   // no larger than what the GPU holds at once (no partly filled last wave) and every CTA streams
@@ -146,7 +146,7 @@ gemm_skinny_kernel(const bf16* __restrict__ A, int lda, const bf16* __restrict__
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
       const int k = (warp + (b * UNROLL + u) * SK_WARPS) * 32;
-      d[u][WHOLE ? nt : 0] = m < M && k + 8 * t < K ? __ldg(reinterpret_cast<const uint4*>(row + k)) : zero;
+      d[u][WHOLE ? nt : 0] = m < M && k + 8 * t < K ? *reinterpret_cast<const uint4*>(row + k) : zero;
     }
   };
   int slot = 0;

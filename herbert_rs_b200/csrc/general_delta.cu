@@ -246,7 +246,7 @@ extern "C" int hb_channel_delta_prepare(const float* qk, int ldqk, int q_off, in
 // bits of them reach the product when its matrix holds their weights twice), the next `coarse` ones rounded once, zeros
 // up to the row's end:   out[t] = [high(fine) | low(fine) | coarse | 0].
 __global__ void __launch_bounds__(256)
-operand_parts_kernel(const float* __restrict__ x, int ld, int fine, int coarse, bf16* __restrict__ out, int ldo, long long total) {
+operand_parts_kernel(const float* x, int ld, int fine, int coarse, bf16* __restrict__ out, int ldo, long long total) {
   pdl_wait();
   pdl_launch();
   const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -22,7 +22,7 @@
 #define GD_PREFETCH_TOKENS 64      // decode steps: a prompt's CTAs share the rows anyway
 template <typename T>
 __global__ void __launch_bounds__(GD_THREADS)
-gla_decay_kernel(const float* __restrict__ low, int ld, const T* __restrict__ w2, const float* __restrict__ bias,
+gla_decay_kernel(const float* low, int ld, const T* __restrict__ w2, const float* __restrict__ bias,
                  float inv_tau, float* __restrict__ a, int n_tokens, int C, int R) {
   extern __shared__ float lows[];  // [GD_TOK][R]
   const int t0 = blockIdx.y * GD_TOK, c = blockIdx.x * GD_THREADS + threadIdx.x;
@@ -105,8 +105,8 @@ __device__ __forceinline__ void gla_copy16(float* smem, const float* gmem) {
 
 template <int RPT, int COLS>  // rows per thread: dk <= (128 / COLS) * RPT; up to 1,024 key channels with 8 columns
 __global__ void __launch_bounds__(GLA_THREADS)
-gla_scan_kernel(const float* __restrict__ proj, int ld, int q_off, int k_off, int v_off, const float* __restrict__ decay,
-                float* __restrict__ state, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
+gla_scan_kernel(const float* proj, int ld, int q_off, int k_off, int v_off, const float* decay,
+                float* state, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
                 float* __restrict__ out, int ldo, int H, int dk, int dv, float qscale, int chunk, int wide) {
   constexpr int GLA_ROWGROUPS = GLA_THREADS / COLS;
   constexpr int DKP = GLA_ROWGROUPS * RPT;  // padded row count; rows past dk hold zeros and stay zero
@@ -275,7 +275,7 @@ extern "C" int hb_gla_scan(const float* proj, int ld, int q_off, int k_off, int 
 // y[t, h, :] = o / sqrt(mean(o^2) + eps) * w * silu(g[t, h, :]).  One CTA of 128 threads per (token, head).
 template <typename T>
 __global__ void __launch_bounds__(128)
-gla_output_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ w, float eps, const float* __restrict__ gate,
+gla_output_kernel(const float* o, int ldo, const float* __restrict__ w, float eps, const float* gate,
                   int ldg, T* __restrict__ y, int ldy, int n_tokens, int H, int dv) {
   __shared__ float red[32];
   pdl_wait();

@@ -18,8 +18,8 @@
 #define GN_MAX_GROUPS 64
 template <typename T, bool RESIDUAL>
 __global__ void __launch_bounds__(256)
-group_rmsnorm_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ z, int ldz, float a, float b,
-                     const float* __restrict__ bias, const float* __restrict__ w, float* __restrict__ x, T* __restrict__ out,
+group_rmsnorm_kernel(const float* y, int ldy, const float* z, int ldz, float a, float b,
+                     const float* __restrict__ bias, const float* __restrict__ w, float* x, T* __restrict__ out,
                      const int* __restrict__ rows, int dim, int groups, float eps) {
   __shared__ float sums[GN_MAX_GROUPS];
   pdl_wait();
@@ -59,8 +59,8 @@ group_rmsnorm_kernel(const float* __restrict__ y, int ldy, const float* __restri
 // The same with the row in registers (row_norm.cuh): where groups are multiples of 128 columns and all rows start on 16 bytes.
 template <typename T, bool RESIDUAL, int V>
 __global__ void __launch_bounds__(RN_MAX_THREADS)
-group_rmsnorm_row_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ z, int ldz, float a, float b,
-                         const float* __restrict__ bias, const float* __restrict__ w, float* __restrict__ x, T* __restrict__ out,
+group_rmsnorm_row_kernel(const float* y, int ldy, const float* z, int ldz, float a, float b,
+                         const float* __restrict__ bias, const float* __restrict__ w, float* x, T* __restrict__ out,
                          const int* __restrict__ rows, int dim, int groups, float eps) {
   __shared__ float part[V * 16];
   pdl_wait();
@@ -144,7 +144,7 @@ extern "C" int hb_group_rmsnorm_residual(int dtype, const float* y, int ldy, con
 }
 
 // ---------------------------------------------------------------------------------------------
-__global__ void axpby_kernel(float* __restrict__ y, int ldy, float a, const float* __restrict__ z, int ldz, float b, int rows,
+__global__ void axpby_kernel(float* y, int ldy, float a, const float* z, int ldz, float b, int rows,
                              int cols) {
   pdl_wait();
   pdl_launch();
@@ -183,7 +183,7 @@ __device__ __forceinline__ float bias_glu_one(float g, float u, int act, float l
 // Four columns of two tokens a thread, all four loads ahead of the first use: bound by memory (2,048 tokens of 8,192 columns, 168 MB: a
 // column a thread took 70 us, 2.4 TB/s).  For rows and columns that come in whole pieces of four; the general kernel is below.
 template <typename T>
-__global__ void bias_glu4_kernel(const float* __restrict__ gu, int ld, const float* __restrict__ bias, T* __restrict__ out, int ldo,
+__global__ void bias_glu4_kernel(const float* gu, int ld, const float* __restrict__ bias, T* __restrict__ out, int ldo,
                                  int n_tokens, int inter, int interleave, int act, float limit) {
   pdl_wait();
   pdl_launch();
@@ -224,7 +224,7 @@ __global__ void bias_glu4_kernel(const float* __restrict__ gu, int ld, const flo
   }
 }
 template <typename T>
-__global__ void bias_glu_kernel(const float* __restrict__ gu, int ld, const float* __restrict__ bias, T* __restrict__ out, int ldo,
+__global__ void bias_glu_kernel(const float* gu, int ld, const float* __restrict__ bias, T* __restrict__ out, int ldo,
                                 int inter, int interleave, int act, float limit) {
   pdl_wait();
   pdl_launch();
@@ -270,7 +270,7 @@ extern "C" int hb_bias_glu(int dtype, const float* gu, int ld, const float* bias
   return 0;
 }
 
-__global__ void tanh_cap_kernel(float* __restrict__ x, int ld, float cap, int rows, int cols) {
+__global__ void tanh_cap_kernel(float* x, int ld, float cap, int rows, int cols) {
   pdl_wait();
   pdl_launch();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -23,7 +23,7 @@
 // ---------------------------------------------------------------------------------------------
 // One warp per token: c = RMSNorm(kv[:rank]) * w, r = rotate(kv[rank:]), both into the cache.
 template <typename T>
-__global__ void latent_kv_store_kernel(const float* __restrict__ kv, int ld, const float* __restrict__ nw, float eps,
+__global__ void latent_kv_store_kernel(const float* kv, int ld, const float* __restrict__ nw, float eps,
                                        const float* __restrict__ freq, float mscale, int halves, int rank, int rot,
                                        const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                                        const int* __restrict__ seq_pages, int pages_stride, T* __restrict__ cache,
@@ -82,7 +82,7 @@ extern "C" int hb_latent_kv_store(int dtype, const float* kv, int ld, const floa
 // ---------------------------------------------------------------------------------------------
 // The rotated part of every head of every token: in[t, h*in_hs + in_off + ..rot] -> out[t, h*out_hs + out_off + ..rot],
 // rotated at the token's position and multiplied by `scale`.  One thread per pair.
-__global__ void rotate_heads_kernel(const float* __restrict__ in, int ld_in, int in_hs, int in_off, float* __restrict__ out,
+__global__ void rotate_heads_kernel(const float* in, int ld_in, int in_hs, int in_off, float* __restrict__ out,
                                     int ld_out, int out_hs, int out_off, const float* __restrict__ freq, float mscale, int halves,
                                     const int* __restrict__ tok_pos, int n_tokens, int H, int rot, float scale) {
   pdl_wait();
@@ -142,8 +142,8 @@ __device__ __forceinline__ void hw_load8(const bf16* p, float* v) {
 
 template <typename TW, typename TO>
 __global__ void __launch_bounds__(HW_WARPS * 32)
-headwise_dot_kernel(const float* __restrict__ in, int ld_in, int in_hs, const TW* __restrict__ w, TO* __restrict__ out,
-                    int ld_out, int out_hs, const float* __restrict__ gate, int ld_gate, int n_tokens, int K, int N,
+headwise_dot_kernel(const float* in, int ld_in, int in_hs, const TW* __restrict__ w, TO* __restrict__ out,
+                    int ld_out, int out_hs, const float* gate, int ld_gate, int n_tokens, int K, int N,
                     float scale, int vec) {
   const int lane = threadIdx.x & 31, n = blockIdx.x * HW_WARPS + (threadIdx.x >> 5), h = blockIdx.y, t0 = blockIdx.z * HW_TT;
   const TW* wr = w + ((size_t)h * N + n) * K;
@@ -193,8 +193,8 @@ headwise_dot_kernel(const float* __restrict__ in, int ld_in, int in_hs, const TW
 #define HM_TK 32
 template <typename TO>
 __global__ void __launch_bounds__(128)
-headwise_mma_kernel(const float* __restrict__ in, int ld_in, int in_hs, const bf16* __restrict__ w, TO* __restrict__ out,
-                    int ld_out, int out_hs, const float* __restrict__ gate, int ld_gate, int n_tokens, int K, int N,
+headwise_mma_kernel(const float* in, int ld_in, int in_hs, const bf16* __restrict__ w, TO* __restrict__ out,
+                    int ld_out, int out_hs, const float* gate, int ld_gate, int n_tokens, int K, int N,
                     float scale) {
   __shared__ __align__(16) bf16 As[2][HM_TM][HM_TK + 8];
   __shared__ __align__(16) bf16 Ws[2][HM_TN][HM_TK + 8];
@@ -277,8 +277,8 @@ headwise_mma_kernel(const float* __restrict__ in, int ld_in, int in_hs, const bf
 #define HL_T 128
 template <typename TO>
 __global__ void __launch_bounds__(256, 2)
-headwise_mma_wide_kernel(const float* __restrict__ in, int ld_in, int in_hs, const bf16* __restrict__ w, TO* __restrict__ out,
-                         int ld_out, int out_hs, const float* __restrict__ gate, int ld_gate, int n_tokens, int K, int N,
+headwise_mma_wide_kernel(const float* in, int ld_in, int in_hs, const bf16* __restrict__ w, TO* __restrict__ out,
+                         int ld_out, int out_hs, const float* gate, int ld_gate, int n_tokens, int K, int N,
                          float scale, int pairs, int gate_pairs) {
   __shared__ __align__(16) bf16 As[2][HL_T][HM_TK + 8];
   __shared__ __align__(16) bf16 Ws[2][HL_T][HM_TK + 8];
@@ -450,7 +450,7 @@ extern "C" int hb_headwise_gemm(int dtype, int out_dtype, const float* in, int l
 #define LA_WARPS 4
 template <typename T, int CH>  // CH = ceil(rank / 32)
 __global__ void __launch_bounds__(LA_WARPS * 32)
-latent_attention_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, int ldo, const T* __restrict__ cache,
+latent_attention_kernel(const float* q, int ldq, float* __restrict__ out, int ldo, const T* cache,
                         const float* __restrict__ sink, const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                         const int* __restrict__ seq_pages, int pages_stride, int n_tokens, int H, int rank, int rot,
                         int page_size, int window) {
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(LM_THREADS) latent_attention_mma_kernel(Latent
 // row; its threads share the ranges' factors and take the row's columns side by side.
 #define LJ_THREADS 128
 __global__ void __launch_bounds__(LJ_THREADS)
-latent_attention_join_kernel(const float* __restrict__ part, float* __restrict__ out, int ldo, const int* __restrict__ seq_start,
+latent_attention_join_kernel(const float* part, float* __restrict__ out, int ldo, const int* __restrict__ seq_start,
                              int H, int rank, int nsplit, int row_tiles) {
   __shared__ float f[64];
   pdl_wait();

@@ -13,7 +13,7 @@
 #include "row_norm.cuh"
 
 template <typename T>
-__global__ void layernorm_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, T* __restrict__ out,
+__global__ void layernorm_kernel(const float* x, const float* __restrict__ w, const float* __restrict__ bias, T* __restrict__ out,
                                  const int* __restrict__ rows, int dim, float eps) {
   __shared__ float red[32];
   pdl_wait();
@@ -34,8 +34,8 @@ __global__ void layernorm_kernel(const float* __restrict__ x, const float* __res
 }
 
 template <typename T>
-__global__ void layernorm_residual_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ w,
-                                          const float* __restrict__ scale, float* __restrict__ x,
+__global__ void layernorm_residual_kernel(const float* y, int ldy, const float* __restrict__ w,
+                                          const float* __restrict__ scale, float* x,
                                           T* __restrict__ h, int dim, float eps) {
   __shared__ float red[32];
   pdl_wait();
@@ -65,7 +65,7 @@ __global__ void layernorm_residual_kernel(const float* __restrict__ y, int ldy, 
 // RESIDUAL: x += LN(y) (* scale), h = x; else h = LN(y[rows[r]] or y[r]) (+ bias).
 template <typename T, bool RESIDUAL, int V>
 __global__ void __launch_bounds__(RN_MAX_THREADS)
-layernorm_row_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ w, const float* __restrict__ add, float* __restrict__ x,
+layernorm_row_kernel(const float* y, int ldy, const float* __restrict__ w, const float* __restrict__ add, float* x,
                      T* __restrict__ h, const int* __restrict__ rows, int dim, float eps) {
   __shared__ float part[V * 16], part2[V * 16];
   pdl_wait();

@@ -24,7 +24,7 @@
 #include "common.cuh"
 #include "scan_rows.cuh"
 
-__global__ void silu_columns_kernel(float* __restrict__ x, int ld, int col0, int cols, int rows) {
+__global__ void silu_columns_kernel(float* x, int ld, int col0, int cols, int rows) {
   pdl_wait();
   pdl_launch();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -36,7 +36,7 @@ __global__ void silu_columns_kernel(float* __restrict__ x, int ld, int col0, int
 
 // Four columns of two rows a thread, both loads ahead of the first use, no division: bound by memory (2,048 rows of 6,144 columns, 100 MB: a
 // column a thread, two divisions each, took 52 us).
-__global__ void silu_columns4_kernel(float* __restrict__ x, int ld, int col0, int cols, int rows) {
+__global__ void silu_columns4_kernel(float* x, int ld, int col0, int cols, int rows) {
   pdl_wait();
   pdl_launch();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
@@ -72,8 +72,8 @@ extern "C" int hb_silu_columns(float* x, int ld, int col0, int cols, int rows, v
 // ---------------------------------------------------------------------------------------------
 // One warp per (token, q/k head) normalises q and k in place; the first warps of a token also turn the token's
 // per-head numbers into beta and g.  grid: (tokens), block: 32 * warps.
-__global__ void delta_prepare_kernel(float* __restrict__ qk, int ld, int q_off, int k_off, int G, int dk, float qscale,
-                                     const float* __restrict__ ab, int ldab, int b_off, int a_off, const float* __restrict__ a_log,
+__global__ void delta_prepare_kernel(float* qk, int ld, int q_off, int k_off, int G, int dk, float qscale,
+                                     const float* ab, int ldab, int b_off, int a_off, const float* __restrict__ a_log,
                                      const float* __restrict__ dt_bias, float* __restrict__ gates, int H) {
   pdl_wait();
   pdl_launch();
@@ -583,7 +583,7 @@ struct HeadDivide {
 };
 template <typename T>
 __global__ void __launch_bounds__(256)
-gated_rmsnorm_kernel(const float* __restrict__ o, int ldo, int o_stride, const float* __restrict__ w, float eps, const float* __restrict__ gate,
+gated_rmsnorm_kernel(const float* o, int ldo, int o_stride, const float* __restrict__ w, float eps, const float* gate,
                      int ldg, T* __restrict__ y, int ldy, int units, int n, int act, int w_stride, int gate_first, HeadDivide hd) {
   __shared__ float red[32];
   pdl_wait();
@@ -687,7 +687,7 @@ gated_rmsnorm_kernel(const float* __restrict__ o, int ldo, int o_stride, const f
 #define GN_PIECES 4
 template <typename T>
 __global__ void __launch_bounds__(GN_WARPS * 32)
-gated_rmsnorm_warp_kernel(const float* __restrict__ o, int ldo, int o_stride, const float* __restrict__ w, float eps, const float* __restrict__ gate,
+gated_rmsnorm_warp_kernel(const float* o, int ldo, int o_stride, const float* __restrict__ w, float eps, const float* gate,
                           int ldg, T* __restrict__ y, int ldy, int units, int n, int act, int w_stride, int gate_first, HeadDivide hd, long long total) {
   pdl_wait();
   pdl_launch();

@@ -145,7 +145,7 @@ __device__ __forceinline__ void moe_choose(float* s, float* gs, int lane, int t,
 // Any sizes.  One block per token: its warps share the experts' dot products, the first warp then takes the choice.
 template <typename T>
 __global__ void __launch_bounds__(MOE_ROUTE_WARPS * 32)
-moe_route_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr, int* __restrict__ ids, float* __restrict__ wts,
+moe_route_kernel(const T* h, int ld, const T* __restrict__ wr, int* __restrict__ ids, float* __restrict__ wts,
                  int n_tokens, int D, int E, int top, int renorm, int sigmoid, int groups, int keep, int group_top,
                  float wscale) {
   extern __shared__ float sh[];  // [E] scores, [groups] group scores
@@ -184,7 +184,7 @@ __device__ __forceinline__ void moe_widen(const uint4& u, float* v, const bf16*)
 }
 template <typename T, int TT, int W>
 __global__ void __launch_bounds__(W * 32)
-moe_route_tile_kernel(const T* __restrict__ h, int ld, const T* __restrict__ wr, int* __restrict__ ids, float* __restrict__ wts,
+moe_route_tile_kernel(const T* h, int ld, const T* __restrict__ wr, int* __restrict__ ids, float* __restrict__ wts,
                       int n_tokens, int D, int E, int top, int renorm, int sigmoid, int groups, int keep, int group_top, float wscale) {
   constexpr int VE = 16 / (int)sizeof(T), N = 2 * TT, B = 4;
   static_assert(TT <= W, "a warp per token chooses");
@@ -318,7 +318,7 @@ extern "C" int hb_moe_route(int dtype, const void* h, int ld, const void* w_rout
 // the expert's 2F rows, both products times in_w[u] if given.  One warp per output.
 template <typename T>
 __global__ void __launch_bounds__(MOE_WARPS * 32)
-moe_up_kernel(const T* __restrict__ h, int ld, const T* __restrict__ up, const int* __restrict__ ids, const float* __restrict__ in_w,
+moe_up_kernel(const T* h, int ld, const T* __restrict__ up, const int* ids, const float* in_w,
               T* __restrict__ mid, int D, int E, int F, int top, int act, int gated, float limit) {
   pdl_wait();
   pdl_launch();
@@ -343,8 +343,8 @@ moe_up_kernel(const T* __restrict__ h, int ld, const T* __restrict__ up, const i
 // y[t, d] (+)= sum_r wts[t, r] * Down_e[d, :] . mid[(t*top + r), :] (wts null: 1).  One warp per output.
 template <typename T>
 __global__ void __launch_bounds__(MOE_WARPS * 32)
-moe_down_kernel(const T* __restrict__ mid, const T* __restrict__ down, const int* __restrict__ ids, const float* __restrict__ wts,
-                float* __restrict__ y, int ldy, int D, int E, int F, int top, int accumulate) {
+moe_down_kernel(const T* mid, const T* __restrict__ down, const int* ids, const float* wts,
+                float* y, int ldy, int D, int E, int F, int top, int accumulate) {
   pdl_wait();
   pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -406,7 +406,7 @@ extern "C" int hb_moe_experts(int dtype, const void* h, int ld, const void* up, 
 #define MG_MAX_EXPERTS 1024
 
 __global__ void __launch_bounds__(1024)
-moe_group_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __restrict__ pair_off, int* __restrict__ tile_off,
+moe_group_kernel(const int* ids, int n_pairs, int E, int* __restrict__ pair_off, int* __restrict__ tile_off,
                  int* __restrict__ list) {
   __shared__ int cnt[MG_MAX_EXPERTS], off[MG_MAX_EXPERTS + 1];
   pdl_wait();
@@ -444,9 +444,9 @@ moe_group_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __restric
 // and nt + 1 (up) are the two halves of its channels.
 template <bool UP>
 __global__ void __launch_bounds__(MG_THREADS)
-moe_grouped_gemm_kernel(const bf16* __restrict__ A, int lda, const bf16* __restrict__ W, void* __restrict__ C, int ldc,
-                        const int* __restrict__ pair_off, const int* __restrict__ tile_off, const int* __restrict__ list, int E,
-                        int N, int K, int top, int act, int gated, float limit, const float* __restrict__ in_w) {
+moe_grouped_gemm_kernel(const bf16* A, int lda, const bf16* __restrict__ W, void* __restrict__ C, int ldc,
+                        const int* pair_off, const int* tile_off, const int* list, int E,
+                        int N, int K, int top, int act, int gated, float limit, const float* in_w) {
   __shared__ __align__(16) bf16 AW[2][(MG_TM + MG_TN) * (MG_TK + 8)];      // per buffer: the A tile, then the W tile
   __shared__ int rows[MG_TM];
   pdl_wait();
@@ -568,8 +568,8 @@ moe_grouped_gemm_kernel(const bf16* __restrict__ A, int lda, const bf16* __restr
 // Bound by the pairs' rows.  Measured on a B200, 3,600 tokens of 2,048 numbers, 4 pairs each, inside a step: 65 -> 36 us.
 template <int V>
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const float* __restrict__ part, const float* __restrict__ wts, float* __restrict__ y, int ldy, int D, int E, int top,
-                   int accumulate, const int* __restrict__ slot, const int* __restrict__ ids) {
+moe_combine_kernel(const float* part, const float* wts, float* y, int ldy, int D, int E, int top,
+                   int accumulate, const int* slot, const int* ids) {
   pdl_wait();
   pdl_launch();
   const int t = blockIdx.y, d = (blockIdx.x * blockDim.x + threadIdx.x) * V;
@@ -668,8 +668,8 @@ extern "C" int hb_moe_experts_grouped_bf16(const void* h, int ld, const void* up
 //   combine:  y[t] (+)= sum_r weights[t, r] * part[slot[t * top + r]]
 // Rows of padding are computed and never read.  A pair's numbers do not depend on its place.
 __global__ void __launch_bounds__(1024)
-moe_sort_padded_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __restrict__ slot, int* __restrict__ tile_expert,
-                       int* __restrict__ rows_used, int max_tiles, const float* __restrict__ wts, float* __restrict__ row_scale) {
+moe_sort_padded_kernel(const int* ids, int n_pairs, int E, int* __restrict__ slot, int* __restrict__ tile_expert,
+                       int* __restrict__ rows_used, int max_tiles, const float* wts, float* __restrict__ row_scale) {
   __shared__ int cnt[MG_MAX_EXPERTS], off[MG_MAX_EXPERTS];
   pdl_wait();
   pdl_launch();
@@ -699,7 +699,7 @@ moe_sort_padded_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __r
   }
 }
 
-__global__ void moe_gather_rows_kernel(const bf16* __restrict__ h, int ld, const int* __restrict__ slot, bf16* __restrict__ sorted,
+__global__ void moe_gather_rows_kernel(const bf16* h, int ld, const int* slot, bf16* __restrict__ sorted,
                                        int D8, int top) {
   pdl_wait();
   pdl_launch();

@@ -46,7 +46,7 @@ struct FwSorted {
 };
 
 // Every thread of the CTA; cnt: n_experts ints of shared memory.  An index outside the experts is left out.
-__device__ __forceinline__ void fw_sort(FwSorted& o, int* cnt, const int* __restrict__ ids, int n_pairs, int E, int cap) {
+__device__ __forceinline__ void fw_sort(FwSorted& o, int* cnt, const int* ids, int n_pairs, int E, int cap) {
   const int tid = threadIdx.x, lane = tid & 31;
   for (int e = tid; e < E; e += FW_THREADS) cnt[e] = 0;
   __syncthreads();
@@ -83,7 +83,7 @@ __device__ __forceinline__ void fw_sort(FwSorted& o, int* cnt, const int* __rest
 // same channels.
 template <int NT, bool GLU>
 __global__ void __launch_bounds__(FW_THREADS, 2)
-moe_few_up_kernel(const bf16* __restrict__ h, int ld, const bf16* __restrict__ up, const int* __restrict__ ids, const float* __restrict__ in_w,
+moe_few_up_kernel(const bf16* h, int ld, const bf16* __restrict__ up, const int* ids, const float* in_w,
                   bf16* __restrict__ mid, int n_pairs, int top, int E, int D, int F, int act, float limit) {
   extern __shared__ int cnt[];
   __shared__ FwSorted so;
@@ -144,7 +144,7 @@ moe_few_up_kernel(const bf16* __restrict__ h, int ld, const bf16* __restrict__ u
 #pragma unroll
         for (int u = 0; u < FW_UNROLL; ++u) {
           const int k = (ks0 + u * FW_WARPS) * 32 + 8 * t;
-          v[u] = k < D && hr[nt] != nullptr ? __ldg(reinterpret_cast<const uint4*>(hr[nt] + k)) : zero;
+          v[u] = k < D && hr[nt] != nullptr ? *reinterpret_cast<const uint4*>(hr[nt] + k) : zero;
         }
 #pragma unroll
         for (int u = 0; u < FW_UNROLL; ++u) {
@@ -190,8 +190,8 @@ moe_few_up_kernel(const bf16* __restrict__ h, int ld, const bf16* __restrict__ u
 
 template <int NT>
 __global__ void __launch_bounds__(FW_THREADS, 2)
-moe_few_down_kernel(const bf16* __restrict__ mid, const bf16* __restrict__ down, const int* __restrict__ ids, const float* __restrict__ wts,
-                    float* __restrict__ y, int ldy, int n_tokens, int top, int E, int D, int F, int accumulate) {
+moe_few_down_kernel(const bf16* mid, const bf16* __restrict__ down, const int* ids, const float* wts,
+                    float* y, int ldy, int n_tokens, int top, int E, int D, int F, int accumulate) {
   extern __shared__ int cnt[];
   __shared__ FwSorted so;
   __shared__ float ys[FW_WARPS][16][NT * 8 + 1];                          // a warp's sums per row and token
@@ -263,7 +263,7 @@ moe_few_down_kernel(const bf16* __restrict__ mid, const bf16* __restrict__ down,
 #pragma unroll
         for (int u = 0; u < FW_UNROLL; ++u) {
           const int k = (k0 + u) * 32;
-          v[u] = u < n && k + 8 * t < F && mr[nt] != nullptr ? __ldg(reinterpret_cast<const uint4*>(mr[nt] + k)) : zero;
+          v[u] = u < n && k + 8 * t < F && mr[nt] != nullptr ? *reinterpret_cast<const uint4*>(mr[nt] + k) : zero;
         }
 #pragma unroll
         for (int u = 0; u < FW_UNROLL; ++u) {

@@ -11,7 +11,7 @@
 #define RNORM_KEEP 8
 
 template <typename T>
-__global__ void scaled_residual_norm_kernel(const float* __restrict__ y, int ldy, float mult, float* __restrict__ x,
+__global__ void scaled_residual_norm_kernel(const float* y, int ldy, float mult, float* x,
                                             const float* __restrict__ w, T* __restrict__ h, int dim, float eps) {
   __shared__ float red[32];
   pdl_wait();
@@ -42,7 +42,7 @@ __global__ void scaled_residual_norm_kernel(const float* __restrict__ y, int ldy
 // The same with the row in registers and all loads ahead (row_norm.cuh): where the width is a multiple of 128 and all rows start on 16 bytes.
 template <typename T, int V>
 __global__ void __launch_bounds__(RN_MAX_THREADS)
-scaled_residual_norm_row_kernel(const float* __restrict__ y, int ldy, float mult, float* __restrict__ x, const float* __restrict__ w,
+scaled_residual_norm_row_kernel(const float* y, int ldy, float mult, float* x, const float* __restrict__ w,
                                 T* __restrict__ h, int dim, float eps) {
   __shared__ float part[V * 16];
   pdl_wait();

@@ -304,7 +304,7 @@ extern "C" int hb_qkv_rotary_cache(int dtype, const float* rows, int ld, const f
 // The angles are worked out once a token, while the kernel before ends; all heads share them.
 template <typename T>
 __global__ void __launch_bounds__(512)
-rotate_heads_back_kernel(const T* __restrict__ att, int ld, int hd, const float* __restrict__ fv, int halves,
+rotate_heads_back_kernel(const T* att, int ld, int hd, const float* __restrict__ fv, int halves,
                          const int* __restrict__ tok_pos, T* __restrict__ y, int ldy, int nh, int dv, int tabled) {
   extern __shared__ float turns[];                       // [half] sines, [half] cosines
   const int t = blockIdx.x;
@@ -354,7 +354,7 @@ extern "C" int hb_rotate_heads_back(int dtype, const void* att, int ld, int hd, 
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(128)
-head_gate_kernel(const T* __restrict__ att, int ld, int hd, const float* __restrict__ gate, int ldg, T* __restrict__ y, int ldy,
+head_gate_kernel(const T* att, int ld, int hd, const float* gate, int ldg, T* __restrict__ y, int ldy,
                  int nh, int dv) {
   pdl_wait();
   pdl_launch();
@@ -388,7 +388,7 @@ extern "C" int hb_head_gate(int dtype, const void* att, int ld, int hd, const fl
 // att holds floats, the maps of head h at heads 2h and 2h + 1 of hd channels.  One warp per (token, head).
 template <typename T>
 __global__ void __launch_bounds__(128)
-difference_heads_kernel(const float* __restrict__ att, int ld, int hd, float lambda, float factor, float eps, T* __restrict__ y,
+difference_heads_kernel(const float* att, int ld, int hd, float lambda, float factor, float eps, T* __restrict__ y,
                         int ldy, int n_tokens, int nh, int dv) {
   pdl_wait();
   pdl_launch();

@@ -26,7 +26,7 @@ __device__ __forceinline__ float key_value(unsigned int k) {       // the invers
 
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-argmax_kernel(const float* __restrict__ logits, int ld, int vocab, int* __restrict__ out) {
+argmax_kernel(const float* logits, int ld, int vocab, int* __restrict__ out) {
   __shared__ float sv[32];
   __shared__ int si[32];
   pdl_wait();
@@ -80,7 +80,7 @@ argmax_kernel(const float* __restrict__ logits, int ld, int vocab, int* __restri
 #define ARGMAX_CHUNKS 64
 
 __global__ void __launch_bounds__(256)
-argmax_partial_kernel(const float* __restrict__ logits, int ld, int vocab, float* __restrict__ pv, int* __restrict__ pi) {
+argmax_partial_kernel(const float* logits, int ld, int vocab, float* __restrict__ pv, int* __restrict__ pi) {
   __shared__ float sv[8];
   __shared__ int si[8];
   pdl_wait();
@@ -125,7 +125,7 @@ argmax_partial_kernel(const float* __restrict__ logits, int ld, int vocab, float
 }
 
 __global__ void __launch_bounds__(32)
-argmax_final_kernel(const float* __restrict__ pv, const int* __restrict__ pi, int* __restrict__ out) {
+argmax_final_kernel(const float* pv, const int* pi, int* __restrict__ out) {
   pdl_wait();
   pdl_launch();
   const int row = blockIdx.x, lane = threadIdx.x;
@@ -271,8 +271,8 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(const float* __restrict__ logits, int ld, int vocab, float temperature, int top_k,
-              float top_p, const float* __restrict__ uniforms, int* __restrict__ out, const int* __restrict__ only_rows) {
+sample_kernel(const float* logits, int ld, int vocab, float temperature, int top_k,
+              float top_p, const float* uniforms, int* __restrict__ out, const int* only_rows) {
   __shared__ SampleShared sh;
   pdl_wait();
   pdl_launch();
@@ -585,8 +585,8 @@ __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS, 1)
-sample_topk_kernel(const float* __restrict__ logits, int ld, int vocab, float temperature, int top_k,
-                   float top_p, const float* __restrict__ uniforms, int* __restrict__ out, int* __restrict__ overflow) {
+sample_topk_kernel(const float* logits, int ld, int vocab, float temperature, int top_k,
+                   float top_p, const float* uniforms, int* __restrict__ out, int* __restrict__ overflow) {
   __shared__ SampleListShared sh;
   pdl_wait();
   pdl_launch();

@@ -20,7 +20,7 @@
 // their sums); 0: any number of them.
 template <typename TO, int TAPS>
 __global__ void __launch_bounds__(SC_THREADS)
-short_conv_kernel(const float* __restrict__ in, int ld_in, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ state,
+short_conv_kernel(const float* in, int ld_in, const float* __restrict__ w, const float* __restrict__ bias, float* state,
                   const int* __restrict__ seq_slot, const int* __restrict__ seq_start, const int* __restrict__ seq_pos0,
                   TO* __restrict__ out, int ldo, int C, int taps, int add_input, int act_silu, int span) {
   pdl_wait();
@@ -123,9 +123,9 @@ extern "C" int hb_short_conv(int out_dtype, const float* in, int ld_in, const fl
 // One CTA per token.  The CTA of a sequence's first token of the step reads the id the step before left in the slot
 // and then leaves the step's last id there; no other CTA touches that int.
 template <typename T>
-__global__ void pair_embed_kernel(const T* __restrict__ table, const T* __restrict__ pair_table, const int* __restrict__ ids,
+__global__ void pair_embed_kernel(const T* __restrict__ table, const T* __restrict__ pair_table, const int* ids,
                                   const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
-                                  const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int* __restrict__ last_id,
+                                  const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int* last_id,
                                   float* __restrict__ out, int hidden, int vocab, int buckets, long long mul_prev,
                                   long long mul_cur, float scale) {
   __shared__ int prev_s;
