@@ -67,16 +67,20 @@ gemm_f32_rows_kernel(const float* A, int lda, const float* __restrict__ W, int l
     load(k + step, nw);
     if (k < K) {
 #pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        const float4 x = f32_load4<V>(ar[m], k, K);
+      for (int m0 = 0; m0 < MT; m0 += 4) {                // four rows' columns are asked for together
+        float4 x[4];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          float s = acc[r * MT + m];
-          s = fmaf(w[r].x, x.x, s);
-          s = fmaf(w[r].y, x.y, s);
-          s = fmaf(w[r].z, x.z, s);
-          acc[r * MT + m] = fmaf(w[r].w, x.w, s);
-        }
+        for (int m = 0; m < 4; ++m) x[m] = f32_load4<V>(ar[m0 + m], k, K);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            float s = acc[r * MT + m0 + m];
+            s = fmaf(w[r].x, x[m].x, s);
+            s = fmaf(w[r].y, x[m].y, s);
+            s = fmaf(w[r].z, x[m].z, s);
+            acc[r * MT + m0 + m] = fmaf(w[r].w, x[m].w, s);
+          }
       }
     }
 #pragma unroll
