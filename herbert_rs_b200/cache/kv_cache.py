@@ -185,7 +185,7 @@ class SequenceCache:
         self.lengths[s] = 0
         self._pages[s] = [[] for _ in self.kv_needs]
         self._released[s] = [0] * len(self.kv_needs)
-        if self._clearer is not None:
+        if self._clearer is not None and torch.cuda.current_device() == self._clearer.device_index:
             self._clearer.clear(s)
         else:
             for st in self.state:

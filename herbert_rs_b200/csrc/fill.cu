@@ -138,13 +138,14 @@ struct ClearRows {
 __global__ void clear_rows_kernel(ClearRows a) {
   pdl_wait();            // the step before may still read the rows (a slot handed out again)
   pdl_launch();
-  const int plane = blockIdx.y, entry = blockIdx.z;
-  if (entry >= a.entries[plane]) return;
-  char* p = a.first[plane] + entry * a.entry_bytes[plane];
+  const int plane = blockIdx.y;
   const long long n = a.row_bytes[plane], stride = (long long)gridDim.x * blockDim.x, i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long whole = ((uintptr_t)p & 15) == 0 ? n >> 4 : 0;      // pieces of 16 bytes, then what is left byte by byte
-  for (long long i = i0; i < whole; i += stride) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
-  for (long long i = (whole << 4) + i0; i < n; i += stride) p[i] = 0;
+  for (int entry = blockIdx.z; entry < a.entries[plane]; entry += gridDim.z) {
+    char* p = a.first[plane] + entry * a.entry_bytes[plane];
+    const long long whole = ((uintptr_t)p & 15) == 0 ? n >> 4 : 0;    // pieces of 16 bytes, then what is left byte by byte
+    for (long long i = i0; i < whole; i += stride) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
+    for (long long i = (whole << 4) + i0; i < n; i += stride) p[i] = 0;
+  }
 }
 
 extern "C" int hb_clear_rows(int planes, void* const* first, const long long* entry_bytes, const long long* row_bytes, const int* entries,
@@ -154,7 +155,8 @@ extern "C" int hb_clear_rows(int planes, void* const* first, const long long* en
   long long most = 0;
   int deepest = 0;
   for (int i = 0; i < planes; ++i) {
-    HB_REQUIRE(first[i] != nullptr && row_bytes[i] >= 0 && entries[i] >= 0 && entries[i] <= 65535, "clear_rows: plane %d has no rows to clear", i);
+    HB_REQUIRE(row_bytes[i] >= 0 && entries[i] >= 0, "clear_rows: plane %d has a negative size", i);
+    HB_REQUIRE(first[i] != nullptr || row_bytes[i] == 0 || entries[i] == 0, "clear_rows: plane %d has no rows to clear", i);
     a.first[i] = (char*)first[i];
     a.entry_bytes[i] = entry_bytes[i];
     a.row_bytes[i] = row_bytes[i];
@@ -164,7 +166,7 @@ extern "C" int hb_clear_rows(int planes, void* const* first, const long long* en
   }
   if (most == 0 || deepest == 0) return 0;
   const long long blocks = ceil_div_ll(most, 256 * 64);      // four pieces a thread
-  hb_launch(clear_rows_kernel, dim3((unsigned)(blocks < 128 ? blocks : 128), (unsigned)planes, (unsigned)deepest), dim3(256), 0, (cudaStream_t)stream, a);
+  hb_launch(clear_rows_kernel, dim3((unsigned)(blocks < 128 ? blocks : 128), (unsigned)planes, (unsigned)(deepest < 65535 ? deepest : 65535)), dim3(256), 0, (cudaStream_t)stream, a);
   HB_CHECK_LAUNCH("clear_rows");
   return 0;
 }

@@ -346,6 +346,7 @@ class RowClearer:
 
     def __init__(self, planes):
         self._groups = []
+        self.device_index = planes[0].device.index
         for i in range(0, len(planes), self.AT_ONCE):
             part = planes[i:i + self.AT_ONCE]
             for p in part:
@@ -353,8 +354,8 @@ class RowClearer:
                 if not p.is_contiguous():
                     raise BackendError("RowClearer: state planes must be contiguous")
             n = len(part)
-            row = [p.stride(1) * p.element_size() for p in part]
-            self._groups.append((n, part, row, (ctypes.c_longlong * n)(*[p.stride(0) * p.element_size() for p in part]),
+            row = [p[0, 0].numel() * p.element_size() if p.shape[0] else 0 for p in part]      # a plane without numbers has rows of none
+            self._groups.append((n, part, row, (ctypes.c_longlong * n)(*[r * p.shape[1] for p, r in zip(part, row)]),
                                  (ctypes.c_longlong * n)(*row), (c_int * n)(*[p.shape[0] for p in part])))
 
     def clear(self, slot: int) -> None:
