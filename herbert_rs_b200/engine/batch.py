@@ -93,7 +93,7 @@ class StepBatch:
         self.layout = StepLayout.make(self.n_tokens, self.n_seqs, self.n_want, num_kv_groups, self.pages_width,
                                       self.n_components)
         self._tokens = tokens
-        self._ids = ids                  # per sequence the same tokens as an integer array, or None
+        self._ids = ids                  # the same tokens as integer arrays, one after the other, or None
         self._positions = positions      # per sequence: [len, C] (or [len] when C == 1), or None
         self.host: Optional[np.ndarray] = None
         self.dev: Optional[torch.Tensor] = None
