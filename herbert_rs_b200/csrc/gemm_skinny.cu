@@ -24,6 +24,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "per_device.h"
 
 #define SK_WARPS 8
 #define SK_THREADS (SK_WARPS * 32)
@@ -291,19 +292,23 @@ static int skinny_launch(const bf16* A, int lda, const bf16* W, int ldw, void* C
                          int epi, cudaStream_t s, SkinnyNorm nm = SkinnyNorm{}) {
   // as many CTAs as the GPU holds at once, each with an equal run of units
   constexpr int PER_SM = NT * RG <= 2 ? 3 : 2, BATCH = SK_WARPS * UNROLL * RG * 1024;
-  static int sms = 0;
-  if (sms == 0) {
+  static HbPerDevice kept;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int sms = hb_per_device(kept, dev, [&]() {
     const void* kernels[4] = {(const void*)gemm_skinny_kernel<NT, RG, UNROLL, HB_EPI_STORE, NORM>, (const void*)gemm_skinny_kernel<NT, RG, UNROLL, HB_EPI_STORE_F32, NORM>,
                               (const void*)gemm_skinny_kernel<NT, RG, UNROLL, HB_EPI_RESIDUAL, NORM>, (const void*)gemm_skinny_kernel<NT, RG, UNROLL, HB_EPI_SWIGLU, NORM>};
     for (const void* k : kernels) {
       const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * BATCH);
-      if (e != cudaSuccess) HB_FAIL(3, "gemm_skinny: cannot reserve %d bytes of shared memory: %s", 6 * BATCH, cudaGetErrorString(e));
+      if (e != cudaSuccess) {
+        hb_set_error("gemm_skinny: cannot reserve %d bytes of shared memory: %s", 6 * BATCH, cudaGetErrorString(e));
+        return -1;
+      }
     }
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    sms = n;
-  }
+    int n = 0;
+    return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+  });
+  if (sms < 0) return 3;
   const int n_units = ceil_div(N, 16 * RG), slots = PER_SM * sms;
   // fewer than one and a half waves: one unit per CTA keeps more loads in flight than halving the grid
   const int upc = (2 * n_units > 3 * slots) ? ceil_div(n_units, slots) : 1;

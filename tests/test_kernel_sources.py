@@ -2,6 +2,7 @@
 import glob
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -57,3 +58,28 @@ def test_what_a_predecessor_writes_is_read_with_ordinary_loads(path):
         for const, name in re.findall(r"(const )?\w+\* __restrict__ (\w+)", params):
             if not const and name in WRITTEN_IN:
                 assert kernel in WRITTEN_IN[name], (kernel, name)
+
+
+def test_what_a_launcher_keeps_it_keeps_per_device(tmp_path):
+    """A number is asked for once on each device, again after a failure, and always beyond the table."""
+    src = tmp_path / "per_device.cpp"
+    src.write_text("""
+#include "per_device.h"
+#include <cstdio>
+static HbPerDevice kept;
+int main() {
+  int asked = 0;
+  auto get = [&](int dev, int answer) { return hb_per_device(kept, dev, [&]() { ++asked; return answer; }); };
+  if (get(0, 148) != 148 || get(0, 7) != 148 || asked != 1) return 1;
+  if (get(1, -1) != -1 || get(1, 132) != 132 || get(1, 5) != 132 || asked != 3) return 2;
+  if (get(HB_KEPT_DEVICES, 3) != 3 || get(HB_KEPT_DEVICES, 4) != 4 || asked != 5) return 3;
+  return get(0, 1) == 148 ? 0 : 4;
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-I", CSRC, str(src), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
+
+
+def test_the_products_of_few_rows_set_their_shared_memory_up_on_every_device():
+    code = code_of(os.path.join(CSRC, "gemm_skinny.cu"))
+    assert "static HbPerDevice" in code and not re.search(r"\n +static (int|bool)\b", code)
