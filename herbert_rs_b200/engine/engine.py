@@ -271,7 +271,7 @@ class Engine:
             _ops.set_pdl(1 if _ops.options.pdl_eager else 0)
             return self.model.forward(batch, self.cache)
         _ops.set_pdl(int(_ops.options.pdl_graph))
-        key = (batch.n_seqs, batch.n_want, batch.pages_width)
+        key = (batch.n_seqs, batch.n_want, batch.pages_width, int(_ops.options.pdl_graph))      # its launches are recorded as the option had them
         hit = self._graphs.get(key)
         if hit is not None:
             graph, logits = hit
