@@ -398,9 +398,9 @@ def test_a_kernel_that_gave_up_is_reported_and_the_counters_start_afresh(model_d
 
 @pytest.mark.gpu
 def test_decode_steps_launched_ahead_of_their_predecessor_give_the_same_bits(model_dirs, plain):
-    """Programmatic dependent launch: a product fetches its first weights, and the fused attention its
-    first keys of earlier steps, before the kernel before them has ended.  Inside recorded graphs
-    (an option, off by default) and eagerly, the logits are the bits of the plain stream order."""
+    """Programmatic dependent launch: a product fetches its first weights, and kernels work out angles and places, before
+    the kernel before them has ended.  Inside recorded graphs and eagerly, the logits are the bits of the plain stream order, and
+    near the plain implementation's."""
     from herbert_rs_b200 import ops
     rng = np.random.default_rng(43)
     lens = [150, 63, 257]
