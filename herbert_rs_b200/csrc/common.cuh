@@ -33,16 +33,20 @@ void hb_set_error(const char* fmt, ...);
   } while (0)
 
 // ---- launching ------------------------------------------------------------------------------
-// Every kernel is launched through hb_launch.  With programmatic dependent launch switched on
-// (hb_set_pdl(1); off by default) a kernel may be scheduled while its predecessor in the stream is
-// still draining; it must then call pdl_wait() before it reads anything the predecessor wrote or
-// writes anything the predecessor may still read.  pdl_launch() tells the hardware that the next
-// kernel may start its own prologue.  It is called after pdl_wait(), so that at most one kernel
-// ahead of the running one sits on the SMs, and in decode attention only when the CTA's own loads are done.  What makes
-// an early start pay or not is where the early CTAs come to stand: those of a kernel that leaves room for several on an SM
-// crowd on the SMs that are free first and keep crowded for their whole length.  The products of few rows (gemm_skinny.cu)
-// fill an SM's shared memory and trigger as soon as their own first loads are out; row kernels that trigger ahead of their wait
-// gained the recurrent designs 1 % and cost those with experts 5 to 20 %.  Both are no-ops for a kernel launched without the attribute.
+// Every kernel is launched through hb_launch.  With programmatic dependent launch (hb_set_pdl; the engine switches it on, a
+// launcher called alone runs without it) a kernel may be scheduled while kernels ahead of it in the stream still run.  What that rests on:
+//  * Every kernel calls pdl_wait(), also one that reads nothing of its predecessor's.  The wait ends when the predecessor has ended, and
+//    that one has waited for its own: so everything older has ended too.  A kernel without the wait would break the chain for the next one.
+//  * Ahead of the wait a kernel touches only weights, tables and what the host copied before the step.
+//  * What another kernel of a step writes is read with ordinary loads: no __ldg, no __restrict__ at its pointer.
+//  * pdl_launch() tells the hardware that the next kernel may start.  It does once every CTA has called it (or ended), that is, once all of
+//    them are resident: so tensor memory is taken, and whatever else an early CTA could take away, before that call.
+// Most kernels trigger right after their wait, decode attention when the CTA's own loads are done.  The products of few rows
+// (gemm_skinny.cu) trigger ahead of their wait, as soon as their own first loads are out: behind a chain of them several kernels sit on the SMs.
+// What makes an early start pay or not is where the early CTAs come to stand: those of a kernel that leaves room for several on an SM
+// crowd on the SMs that are free first and keep crowded for their whole length.  The products' CTAs leave little room on an SM; row
+// kernels that trigger ahead of their wait gained the recurrent designs 1 % and cost those with experts 5 to 20 %.  Both calls are no-ops
+// for a kernel launched without the attribute.
 int hb_pdl_enabled(void);   // 0 off, 1 every kernel, 2 only the launches that ask for it (hb_launch_pdl)
 template <typename... KArgs, typename... Args>
 static inline cudaError_t hb_launch_ex(int want_pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

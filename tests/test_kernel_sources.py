@@ -83,3 +83,15 @@ int main() {
 def test_the_products_of_few_rows_set_their_shared_memory_up_on_every_device():
     code = code_of(os.path.join(CSRC, "gemm_skinny.cu"))
     assert "static HbPerDevice" in code and not re.search(r"\n +static (int|bool)\b", code)
+
+
+@pytest.mark.parametrize("path", FILES, ids=os.path.basename)
+def test_every_kernel_waits_for_its_predecessor_and_takes_tensor_memory_before_it_lets_the_next_one_start(path):
+    """A kernel that does not wait lets its successor pass while older ones still run; tensor memory that an early CTA of the next kernel
+    could take first would never come free."""
+    for kernel, _, body in kernels_of(path):
+        assert "pdl_wait();" in body, kernel
+        depth = body[:body.index("pdl_wait();")].count("{") - body[:body.index("pdl_wait();")].count("}")
+        assert depth == 1, f"{kernel}: every thread waits"
+        if "tcgen05.alloc" in body and "pdl_launch();" in body:
+            assert body.index("tcgen05.alloc") < body.index("pdl_launch();"), kernel
