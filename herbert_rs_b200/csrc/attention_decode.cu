@@ -19,6 +19,7 @@
 #include "api.h"
 #include "common.cuh"
 #include "mma_utils.cuh"
+#include "per_device.h"
 #include "qk_norm.cuh"
 
 // exp: the hardware's fast exponential (ex2.approx, about 2 ulp in float).  The probabilities are
@@ -46,6 +47,7 @@ struct DecodeArgs {
   float softcap;       // > 0: score <- softcap * tanh(score / softcap) after the scale
   const float* gate_bias;  // [nh] or null.  Not null: no softmax; a visible key weighs sigmoid(score + gate_bias[h]) as it
                            // is.  Every running maximum then stays 0, so splits and warps simply add up (general kernel only)
+  int by_length;           // the keys-as-M kernel's rows of the grid take the sequences from the longest down
 };
 
 // What the fused variant of the keys-as-M kernel needs besides: it takes the raw q/k/v row of each
@@ -336,20 +338,22 @@ __device__ __forceinline__ void st_bf2(bf16* p, float x, float y) {
   *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y);
 }
 
-// Which sequence a CTA of row z of the grid takes.  With a key range per sequence a full server has more CTAs than the GPU holds, and
-// CTAs start in the order of their index: the longest sequences first, so that none of them is what the last wave waits for.
-// Every CTA ranks the lengths for itself (equal ones by index).  64 sequences of 210 to 2,000 tokens, 8 kv heads, inside steps: two steps of
-// eight layers 3,010 -> 2,866 us.  Up to 16 sequences their keys are cut into ranges, or the CTAs all stand on the GPU at once.
+// Which sequence a CTA of row z of the grid takes: the longest sequences first.  CTAs start in the order of their index.  Where the GPU
+// holds them all (two an SM), that gives the longest ones an SM's company of the shortest, where it does not, none of the longest is what the
+// last wave waits for.  Every CTA ranks the lengths for itself (equal ones by index), unless all are short or near the first one's:
+// then there is nothing to gain.  See decode_order for the rule.
 __device__ __forceinline__ int longest_first(const int* __restrict__ seq_len, int n, int z) {      // n <= AD_THREADS
-  __shared__ int lens[AD_THREADS], chosen;
-  const int mine = threadIdx.x < n ? seq_len[threadIdx.x] : -1;
-  lens[threadIdx.x] = mine;
-  __syncthreads();
+  __shared__ __align__(16) int keys[AD_THREADS];
+  __shared__ int chosen;
+  const int len0 = seq_len[0], len = threadIdx.x < n ? seq_len[threadIdx.x] : len0;
+  const int mine = threadIdx.x < n ? (len << 7) | (AD_THREADS - 1 - threadIdx.x) : -1;      // no two alike; lengths below 2^24
+  keys[threadIdx.x] = mine;
+  if (!__syncthreads_or(max(len, len0) > 4 * AD_TILE && abs(len - len0) > 2 * AD_TILE)) return z;
   int rank = 0;
-#pragma unroll 8
-  for (int j = 0; j < n; ++j) {
-    const int o = lens[j];
-    rank += o > mine || (o == mine && j < threadIdx.x);
+#pragma unroll 4
+  for (int j = 0; j < n; j += 4) {
+    const int4 o = *reinterpret_cast<const int4*>(keys + j);
+    rank += (o.x > mine) + (o.y > mine) + (o.z > mine) + (o.w > mine);
   }
   if (threadIdx.x < n && rank == z) chosen = threadIdx.x;
   __syncthreads();
@@ -365,8 +369,7 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_km_kernel(DecodeA
   // Before the wait on the kernel before: only what the host wrote ahead of the step (lengths, page
   // tables) and what earlier steps left in the cache.
   const int split = blockIdx.x, kvh = blockIdx.y;
-  const bool ranked = a.nsplit == 1 && gridDim.z > 16 && gridDim.z <= AD_THREADS;
-  const int b = ranked ? longest_first(a.seq_len, gridDim.z, blockIdx.z) : blockIdx.z;
+  const int b = a.by_length ? longest_first(a.seq_len, gridDim.z, blockIdx.z) : blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int G = a.nh / a.nkv;
   constexpr int row_bytes = HD * 2 + 16;
@@ -775,6 +778,23 @@ __global__ void attention_decode_difference_kernel(const float* part_o, const fl
   for (int d = threadIdx.x; d < df.dv; d += blockDim.x) out[(size_t)b * ldo + (size_t)h * df.dv + d] = __float2bfloat16_rn(row[d] * k);
 }
 
+// Longest first (keys-as-M kernel) where a sequence has one key range, there are more CTAs than SMs and a CTA's threads hold a length each.
+// Ranges of one sequence are equally long, and a CTA that has its SM to itself waits for nobody.  Measured on a B200, the fused kernel alone,
+// lengths of 200 to 2,000, us in order of the batch -> longest first: 24 x 8 key/value heads (192 CTAs) 41.7 -> 37.6, 32 x 8 42.5 -> 40.6, 37 x
+// 8 (296: all the GPU holds) 42.7 -> 42.2, 48 x 8 56.2 -> 44.8, 64 x 8 69.1 -> 52.9, 128 x 8 114 -> 105, 64 x 4 43.6 -> 40.9, 16 x 32 68.9 -> 53.5.
+// Ranking costs 1 us in 53 (64 x 8 of equal length) and 0.7 in 16 (lengths of 64 to 200), so a CTA first looks whether they differ.
+// Beyond 128 sequences they keep the order of the batch.
+static int decode_order(int n_seqs, int nkv, int nsplit) {
+  static HbPerDevice kept;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int sms = hb_per_device(kept, dev, [&]() {
+    int n = 0;
+    return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+  });
+  return nsplit == 1 && n_seqs > 1 && n_seqs <= AD_THREADS && (long long)n_seqs * nkv > sms;
+}
+
 static int decode_smem_bytes(int hd, int stages) {
   const int pipeline = stages * 2 * AD_TILE * (hd * 2 + 16);
   const int merge = (2 * AD_WARPS * 16 + AD_WARPS * 16 * hd) * 4;
@@ -816,7 +836,7 @@ extern "C" int hb_attention_decode_bf16(const void* q, int ldq, void* out, int l
   float* part_o = scratch;
   float* part_ml = scratch + (size_t)n_seqs * nh * nsplit * hd;
   DecodeArgs a{(const bf16*)q, ldq, (const bf16*)kcache, (const bf16*)vcache, seq_len, seq_pages, pages_stride,
-               part_o, part_ml, nh, nkv, hd, page_size, nsplit, scale, window, stages, softcap, gate_bias};
+               part_o, part_ml, nh, nkv, hd, page_size, nsplit, scale, window, stages, softcap, gate_bias, decode_order(n_seqs, nkv, nsplit)};
   dim3 grid(nsplit, nkv, n_seqs);
   cudaError_t e;
   if (hd <= 64) {
@@ -893,7 +913,7 @@ extern "C" int hb_attention_decode_fused_bf16(const void* qkv, int ld, void* out
   float* part_o = scratch;
   float* part_ml = scratch + (size_t)n_seqs * nh * nsplit * hd;
   DecodeArgs a{nullptr, 0, (const bf16*)kcache, (const bf16*)vcache, seq_len, seq_pages, pages_stride,
-               part_o, part_ml, nh, nkv, hd, page_size, nsplit, scale, window, stages};
+               part_o, part_ml, nh, nkv, hd, page_size, nsplit, scale, window, stages, 0.0f, nullptr, decode_order(n_seqs, nkv, nsplit)};
   DecodeFuse f{(const bf16*)qkv, ld, qw, kw, eps, cos_tab, sin_tab, table_rows, write_cache, (bf16*)kcache, (bf16*)vcache,
                counters, (bf16*)out, ldo};
   dim3 grid(nsplit, nkv, n_seqs);
