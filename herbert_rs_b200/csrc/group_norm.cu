@@ -249,9 +249,11 @@ extern "C" int hb_bias_glu(int dtype, const float* gu, int ld, const float* bias
   HB_REQUIRE(n_tokens <= 65535, "bias_glu: at most 65535 tokens per call, got %d", n_tokens);
   HB_REQUIRE(act >= HB_ACT_SILU && act <= HB_ACT_SWISH_CLAMP, "bias_glu: unknown activation %d", act);
   HB_REQUIRE(act != HB_ACT_SWISH_CLAMP || limit > 0.0f, "bias_glu: the clamped activation needs a limit > 0");
-  // few tokens keep a column a thread: four times the warps, and the step's time is one way to memory either way
+  // From half a million numbers on; below, a column a thread has eight times the warps, and the time is one way to memory either way.  A
+  // column a thread / four columns, us alone: 8,192 columns of 64 tokens 3.2 / 3.2, 96 4.2 / 3.5, 512 17.9 / 8.4; 3,072 columns of 64 tokens
+  // 2.1 / 3.0, 128 2.7 / 3.1, 192 3.5 / 3.2, 1,024 13.7 / 6.9.
   const int out_bytes = dtype == HB_F32 ? 16 : 8;
-  if (n_tokens >= 64 && inter % 4 == 0 && interleave % 4 == 0 && ld % 4 == 0 && ldo % 4 == 0 &&
+  if ((long long)n_tokens * inter >= 512 * 1024 && inter % 4 == 0 && interleave % 4 == 0 && ld % 4 == 0 && ldo % 4 == 0 &&
       (((uintptr_t)gu | (uintptr_t)bias) & 15) == 0 && ((uintptr_t)out & (out_bytes - 1)) == 0) {
     const dim3 grid4(ceil_div(inter, 1024), ceil_div(n_tokens, 2));
     if (dtype == HB_F32)

@@ -42,3 +42,17 @@ def test_silu_columns(rows, col0, cols):
     ops.silu_columns(b, col0, cols)
     assert torch.equal(torch.nan_to_num(a, nan=12345.0), torch.nan_to_num(b, nan=12345.0))
     assert torch.equal(a[:, :col0], x[:, :col0]) and torch.equal(a[:, col0 + cols:], x[:, col0 + cols:])
+
+
+@pytest.mark.parametrize("extra", [0, 1, 138])
+@pytest.mark.parametrize("inter,interleave", [(12, 0), (1028, 0), (2048, 8), (48, 4), (8192, 0)])
+@pytest.mark.parametrize("act", ["silu", "swish_clamp"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_bias_glu_from_half_a_million_numbers_on(extra, inter, interleave, act, dtype):
+    test_bias_glu(-(-512 * 1024 // inter) + extra, inter, interleave, act, dtype)
+
+
+@pytest.mark.parametrize("extra", [0, 1, 138])
+@pytest.mark.parametrize("col0,cols", [(0, 4), (8, 1028), (4, 2048), (0, 6144)])
+def test_silu_columns_from_half_a_million_numbers_on(extra, col0, cols):
+    test_silu_columns(-(-512 * 1024 // cols) + extra, col0, cols)
