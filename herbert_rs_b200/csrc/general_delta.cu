@@ -51,10 +51,6 @@ __global__ void __launch_bounds__(GP_MAX_THREADS) general_delta_prepare_kernel(G
   __shared__ float red[GP_TOK][GP_MAX_THREADS / 32];
   __shared__ float inv[GP_TOK];
   const int t0 = blockIdx.x * GP_TOK, h = blockIdx.y;
-  if (a.n_tokens <= 64) {      // a decode step: the head's rows of w2, one piece of memory, come while the kernel before ends
-    const size_t bytes = (size_t)a.dk * a.rank * sizeof(T), part = (bytes / (blockDim.x >> 5) + 127) & ~(size_t)127, from = (threadIdx.x >> 5) * part;
-    if (from < bytes) warp_prefetch_l2((const char*)a.w2 + (size_t)h * bytes + from, bytes - from < part ? bytes - from : part);
-  }
   pdl_wait();
   pdl_launch();
   const int nt = a.n_tokens - t0 < GP_TOK ? a.n_tokens - t0 : GP_TOK;
@@ -95,7 +91,8 @@ __global__ void __launch_bounds__(GP_MAX_THREADS) general_delta_prepare_kernel(G
     const float z0 = a.w0[c], a0 = a.a0[c];
 #pragma unroll
     for (int tt = 0; tt < GP_TOK; ++tt) z[tt] = z0;
-    // sixteen weights at a time where rows are whole pieces of 16 bytes: a weight at a time is a way to L1 each
+    // sixteen weights at a time where rows are whole pieces of 16 bytes: a weight at a time is a way to L1 each (16 heads of 128, rank 128, us
+    // alone: 1 token 15.1 -> 7.6, 2,048 tokens 324 -> 115)
     constexpr int VE = 16 / (int)sizeof(T);
     int j = 0;
     if (a.rank % VE == 0 && ((uintptr_t)w2 & 15) == 0)

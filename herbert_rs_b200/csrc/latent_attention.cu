@@ -147,7 +147,6 @@ headwise_dot_kernel(const float* in, int ld_in, int in_hs, const TW* __restrict_
                     float scale, int vec) {
   const int lane = threadIdx.x & 31, n = blockIdx.x * HW_WARPS + (threadIdx.x >> 5), h = blockIdx.y, t0 = blockIdx.z * HW_TT;
   const TW* wr = w + ((size_t)h * N + n) * K;
-  if (n < N) warp_prefetch_l2(wr, (size_t)K * sizeof(TW));      // while the kernel before ends
   pdl_wait();
   pdl_launch();
   if (n >= N) return;
