@@ -8,15 +8,19 @@
 // warps share K, and every lane fetches 16 contiguous bytes of a weight row straight from global
 // memory into the registers mma.sync.m16n8k16 wants.  The k index inside one instruction is
 // permuted the same way for both operands (a lane's 8 consecutive elements serve k-slots
-// {2t,2t+1,2t+8,2t+9} of two instructions), which leaves the dot products unchanged.  Between memory and registers a lane's
-// pieces wait in shared memory of its own (cp.async, read back by the lane that asked: no barrier), so that what a CTA has under
-// way is not bound by its registers but fills the SM: six batches where the grid gives an SM one CTA, three with two CTAs, two
-// with three.  What an SM has under way is its rate: with two batches in registers (32 KB a CTA) the products of 2,048 rows, one CTA
-// an SM, ran at 2.7 TB/s.  And with the SM's shared memory taken, the next kernel's CTAs (they start early, see common.cuh) find
-// one place where one of these has left, so they spread over the SMs; kernels without that crowded on the SMs that were done
-// first, which made early starts slower than none.  Measured on a B200 with both (before -> now, us a pass): the 0.6B-sized decoder's two
-// steps of one sequence 1,806 -> 1,505, four steps of eight sequences on eight 8B-sized layers 4,067 -> 3,907, turns of the designs 1.03 to 1.08
-// times faster; the ring without early starts 1,690 and 4,141, early starts without the ring 1,992 and 6,015.
+// {2t,2t+1,2t+8,2t+9} of two instructions), which leaves the dot products unchanged.  Up to 32 rows a lane's pieces wait between memory and
+// registers in shared memory of its own (cp.async, read back by the lane that asked: no barrier), so that what a CTA has under
+// way is not bound by its registers: six batches where the grid gives an SM one CTA, three where it gives two and a batch and the sums
+// leave room, else two (see `depth` below; a batch is 32 KB, from 17 rows on 16 KB).  What an SM has under way is its rate: with two batches
+// in registers (32 KB a CTA) the products of 2,048 rows, one CTA an SM, ran at 2.7 TB/s.  And with the SM's shared memory taken, the next
+// kernel's CTAs (they start early, see common.cuh) find one place where one of these has left, so they spread over the SMs; kernels
+// without that crowded on the SMs that were done first, which made early starts slower than none.  Measured on a B200 with both (before -> now, us
+// a pass): the 0.6B-sized decoder's two steps of one sequence 1,806 -> 1,505, four steps of eight sequences on eight 8B-sized layers 4,142 -> 3,994,
+// four of 17 and 32 on the 0.6B-sized one 4,744 -> 3,970 and 4,980 -> 4,395, turns of the designs 1.03 to 1.08 times faster; the ring without early
+// starts 1,690 and 4,141, early starts without the ring 1,992 and 6,015.
+// From 33 rows on every CTA reads so many activations that what the ring takes from L1 costs more than it gives (64 x 3,072 on 1,024 rows
+// alone 13.4 us without, 13.9 with it; four 0.6B-sized steps of 63 sequences 7,500 without early starts, 8,210 with ring and early starts,
+// 7,000 as it is now): there a batch waits in registers, and the next kernel is let start when a CTA's last weights are in.
 // The activation rows (at most 64 x K) come through L1/L2.  Partial sums of the 8 warps meet in
 // shared memory; the epilogue stores, adds into the float residual stream, or applies SwiGLU to
 // rows stored as 8 gate rows followed by the 8 up rows of the same channels.
@@ -29,6 +33,7 @@
 #define SK_WARPS 8
 #define SK_THREADS (SK_WARPS * 32)
 #define SK_NORM_ROWS 16
+#define SK_RING(NT) ((NT) < 8)      // up to 32 rows; see above
 
 __device__ __forceinline__ void sk_copy16(unsigned dst, const void* src, bool there) {      // zeros where there is nothing
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
@@ -36,6 +41,11 @@ __device__ __forceinline__ void sk_copy16(unsigned dst, const void* src, bool th
 __device__ __forceinline__ uint4 sk_read16(unsigned src) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 ld_stream16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ void mma_bf16_16816(float* d, unsigned a0, unsigned a1, unsigned a2, unsigned a3,
@@ -78,6 +88,7 @@ gemm_skinny_kernel(const bf16* A, int lda, const bf16* __restrict__ W, int ldw, 
   const int g = lane >> 2, t = lane & 3;
   const int n_units = (N + 16 * RG - 1) / (16 * RG);
   int unit = blockIdx.x * units_per_cta;
+  constexpr bool RING = SK_RING(NT);
   const int ksteps = (K + 31) >> 5, batches = ksteps > warp ? (ksteps - warp + SK_WARPS * UNROLL - 1) / (SK_WARPS * UNROLL) : 0;
   const uint4 zero = make_uint4(0, 0, 0, 0);
   // The ring: `depth` batches of UNROLL steps, of every step 2 RG pieces of 16 bytes a lane.  The next batch to ask for is batch
@@ -120,12 +131,24 @@ gemm_skinny_kernel(const bf16* A, int lda, const bf16* __restrict__ W, int ldw, 
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (++aslot == depth) aslot = 0;
   };
-  // Weights never depend on the previous kernel: the first batches are asked for before the wait on it.  The next kernel
+  // Without a ring: a batch in registers and the next one on its way into others.
+  uint4 wa[RING ? 1 : UNROLL][2 * RG], wb[RING ? 1 : UNROLL][2 * RG];
+  auto fetch = [&](int b, uint4 (&d)[RING ? 1 : UNROLL][2 * RG]) {      // batch b of unit au
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const int k = (warp + (b * UNROLL + u) * SK_WARPS) * 32;
+#pragma unroll
+      for (int i = 0; i < 2 * RG; ++i) d[RING ? 0 : u][i] = k + 8 * t < K && ((w_ok >> i) & 1u) ? ld_stream16(w_at + (size_t)(8 * i) * ldw + k) : zero;
+    }
+  };
+  // Weights never depend on the previous kernel: the first batches are asked for before the wait on it.  With the ring the next kernel
   // may start as soon as that is done; it finds room on an SM when one of this kernel's CTAs has left (see `depth` below), so
   // its CTAs come to stand where there is one free place, not several on the SMs that are done first.
   ask_unit();
-  for (int i = 0; i < depth; ++i) ask();
-  pdl_launch();
+  if constexpr (RING) {
+    for (int i = 0; i < depth; ++i) ask();
+    pdl_launch();
+  } else fetch(0, wa);
   pdl_wait();
   if (NORM) {
     // 1 / rms of the activation rows from the producer's partial sums: warp w sums rows w and w + 8
@@ -206,7 +229,41 @@ gemm_skinny_kernel(const bf16* A, int lda, const bf16* __restrict__ W, int ldw, 
       ask();                               // into the slot just read: behind the instructions that took its values
       if (++slot == depth) slot = 0;
     };
-    if constexpr (AHEAD) {
+    if constexpr (!RING) {
+      for (int b = 0; b < batches; ++b) {
+        fetch(b + 1, wb);
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+          const int k = (warp + (b * UNROLL + u) * SK_WARPS) * 32 + 8 * t;
+#pragma unroll
+          for (int n0 = 0; n0 < NT; n0 += 4) {             // four groups of rows are asked for together
+            uint4 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int m = (n0 + j) * 8 + g;
+              x[j] = m < M && k < K ? *reinterpret_cast<const uint4*>(A + (size_t)m * lda + k) : zero;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+              for (int rg = 0; rg < RG; ++rg) {
+                const uint4 lo = wa[RING ? 0 : u][2 * rg], hi = wa[RING ? 0 : u][2 * rg + 1];
+                mma_bf16_16816(acc[rg][n0 + j], lo.x, hi.x, lo.y, hi.y, x[j].x, x[j].y);
+                mma_bf16_16816(acc[rg][n0 + j], lo.z, hi.z, lo.w, hi.w, x[j].z, x[j].w);
+              }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u)
+#pragma unroll
+          for (int i = 0; i < 2 * RG; ++i) wa[RING ? 0 : u][i] = wb[RING ? 0 : u][i];
+      }
+      if (unit + 1 < unit_end) {           // the next unit's first batch, under this unit's sums
+        ++au;
+        ask_unit();
+        fetch(0, wa);
+      } else pdl_launch();
+    } else if constexpr (AHEAD) {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) load_x(0, nt, xs[0]);
       for (int b = 0; b < batches; b += 2) {
@@ -315,7 +372,7 @@ static int skinny_launch(const bf16* A, int lda, const bf16* W, int ldw, void* C
   const unsigned grid = (unsigned)ceil_div(n_units, upc);
   // What an SM's CTAs have under way together fills its shared memory.  (Three batches where the grid gives an SM one CTA, so that the
   // next product's first batches fit beside them: 0.6B-sized steps 1,551 instead of 1,505 us, the 2,048-wide designs 1 to 2 % slower.)
-  const int depth = (int)grid <= sms ? 6 : (int)grid <= 2 * sms && NT * RG <= 2 ? 3 : 2;
+  const int depth = !SK_RING(NT) ? 0 : (int)grid <= sms ? 6 : (int)grid <= 2 * sms && NT * RG <= 2 ? 3 : 2;
   const size_t smem = (size_t)depth * BATCH;
   switch (epi) {
     case HB_EPI_STORE: hb_launch_pdl(gemm_skinny_kernel<NT, RG, UNROLL, HB_EPI_STORE, NORM>, dim3(grid), dim3(SK_THREADS), smem, s, A, lda, W, ldw, C, ldc, M, N, K, upc, depth, nm); break;

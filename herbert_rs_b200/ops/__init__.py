@@ -1388,12 +1388,12 @@ def _tcgen05_ok(a, w) -> bool:
 
 
 def _decode_gemm(a, w):
-    """Which kernel multiplies at most 64 activation rows.  Measured (microseconds at 17 / 32 / 64
-    rows; mma.sync kernel, streaming tcgen05 kernel, prefill kernel) at Qwen3-8B shapes: q/k/v
-    19 / 21 / 31, 23 / 23 / 28, 14 / 15 / 16; o 12 / 12 / 18, 27 / 30 / 42, 13 / 14 / 14; gate/up
-    58 / 65 / 93, 46 / 49 / 57, 41 / 41 / 42; down 28 / 29 / 42, 53 / 59 / 76, 26 / 26 / 26; at 32B shapes
-    the prefill kernel wins all four from 32 rows on, at 0.6B shapes (at most 6 M elements) the
-    mma.sync kernel wins all four.
+    """Which kernel multiplies at most 64 activation rows.  Measured alone (microseconds at 17 / 32 / 33 / 64 rows; mma.sync kernel,
+    streaming tcgen05 kernel, prefill kernel) at Qwen3-8B shapes: q/k/v 20 / 22 / 31 / 34, 23 / 24 / 26 / 30, 15 / 16 / 16 / 18; o 13 /
+    14 / 18 / 20, 28 / 32 / 34 / 45, 13 / 14 / 14 / 14; gate/up 53 / 59 / 94 / 106, 48 / 48 / 49 / 52, 43 / 42 / 42 / 43; down 29 / 31 /
+    43 / 47, 54 / 59 / 62 / 77, 26 / 27 / 27 / 28.  At 32B shapes the prefill kernel wins (10,240 x 5,120 25 to 28; 5,120 x 8,192 24 to
+    25, also at 17 and 32 rows, which the rule leaves to the mma.sync kernel with 35 and 38).  At 0.6B shapes (at most 6 M elements) the
+    mma.sync kernel wins, but for gate/up beyond 32 rows (13.6 / 14.6 against 10.4 / 11.7).
     Up to 16 rows the mma.sync kernel streams the weights at the memory's rate; beyond that every CTA
     of 16 weight rows reads the whole activation matrix again, and the prefill kernel (K cut over a
     cluster of CTAs where the matrix has few tiles) wins wherever the matrix is large enough to pay
