@@ -366,8 +366,8 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_km_kernel(DecodeA
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(16) bf16 sm_q[FUSED ? 8 * NH * HD : 8];
   __shared__ int s_last;
-  // Before the wait on the kernel before: only what the host wrote ahead of the step (lengths, page
-  // tables) and what earlier steps left in the cache.
+  // Before the wait on the kernel before: only what the host wrote ahead of the step (lengths, page tables).  The keys of earlier
+  // steps are asked for after it (ahead of it: 8B sizes 1 % faster, 0.6B sizes 1 % slower).
   const int split = blockIdx.x, kvh = blockIdx.y;
   const int b = a.by_length ? longest_first(a.seq_len, gridDim.z, blockIdx.z) : blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;

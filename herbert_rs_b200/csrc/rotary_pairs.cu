@@ -287,7 +287,8 @@ extern "C" int hb_qkv_rotary_cache(int dtype, const float* rows, int ld, const f
   const bool v4 = ((dk | dv | hd | ld | ldq) & 3) == 0 && (in_ptrs & 15) == 0 && (out_ptrs & 15) == 0 && rot % (halves ? 8 : 4) == 0 &&
                   (fv == nullptr || dv % (halves ? 8 : 4) == 0);
   cudaStream_t s = (cudaStream_t)stream;
-  // a decode step's few CTAs take sixteen warps each, so that a warp's heads do not follow one another
+  // A decode step's few CTAs (at most one an SM) take sixteen warps each, so that a warp's heads do not follow one another.  Eight warps /
+  // sixteen, 16 + 16 heads of 128, us alone: 1 token 5.5 / 4.4, 128 tokens 5.8 / 4.7, 256 6.4 / 5.9, 512 8.5 / 9.9.
   const int threads = n_tokens <= 128 ? 512 : 256;
   if (dtype == HB_F32) {
     if (v4) hb_launch(qkv_rotary_cache_kernel<float, true>, dim3(n_tokens), dim3(threads), smem, s, a);
@@ -338,6 +339,7 @@ extern "C" int hb_rotate_heads_back(int dtype, const void* att, int ld, int hd, 
                                     void* y, int ldy, int n_tokens, int nh, int dv, void* stream) {
   HB_REQUIRE(n_tokens > 0 && nh > 0 && dv > 0 && hd >= dv, "rotate_heads_back: sizes must be positive and heads wide enough");
   HB_REQUIRE(dv % 2 == 0, "rotate_heads_back: values of %d channels have no pairs", dv);
+  // at most one CTA an SM: four warps / sixteen, 16 heads of 128, us alone: 1 token 3.4 / 2.2, 128 tokens 3.9 / 2.6, 1,024 5.1 / 5.2
   const int threads = n_tokens <= 128 ? 512 : 128;
   const int tabled = (size_t)dv * sizeof(float) <= 48 * 1024;
   const size_t smem = tabled ? (size_t)dv * sizeof(float) : 0;

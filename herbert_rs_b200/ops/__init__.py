@@ -1006,12 +1006,13 @@ def moe_tc_ok(h, up, top, gated, act) -> bool:
 
 
 def moe_few_pays(tokens, top, experts, D, F, gated) -> bool:
-    """Whether a step of few tokens gains by reading every chosen expert once for all its tokens.  The kernels that do so sort the
-    step's pairs first, about 5 us, and then stream at the better rate, more so the more tokens share an expert: they pay from
-    about 36 MB of matrices on, counted once per pair.  Measured inside recorded decode steps, us a layer that they take less
-    than a warp per output number (4 of 32 experts of 1,408 over 2,048, then 2 of 16 of 768 over 1,024): plain experts at 1, 2, 4, 8 tokens
-    +11, +8, +13, +18 and -2, -4, -2, +3 (6 tokens: -0.3), gated ones +4, +5, +10, +16 and -1, -1, +1, +5; one of 4 of 128 over 256, alone, at
-    1 and 31 tokens -5, -10."""
+    """Whether a step of few tokens reads every chosen expert once for all its tokens.  The kernels that do so sort the
+    step's pairs first, about 5 us, and then stream at the better rate, more so the more tokens share an expert.  The line, 36 MB of
+    matrices counted once per pair, was drawn in recorded steps without early starts.  Measured with them, us a layer that they take less
+    than a warp per output number (4 of 32 experts of 1,408 over 2,048): plain experts at 1, 2, 3, 4, 8 tokens -1, -4, -2, +3, +5, gated
+    ones -1 to +1, -2, -1 to +1, +3, +8; 2 of 16 of 768 over 1,024, below the line, at 1, 2, 4, 6 tokens plain -1, -2, -3, -2, gated -2, -3, -3,
+    -2, above it, gated at 8 and 13 tokens +1, +1.  Two and three tokens of the wider ones would gain 1 to 2 % of a step on the other side;
+    the line stays, since the other kernel adds in another order."""
     return tokens * top * (3 if gated else 2) * D * F * 2 >= 36e6
 
 
