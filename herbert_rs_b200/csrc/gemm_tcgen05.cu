@@ -30,6 +30,11 @@ struct TgSmem {
 };
 
 #define HB_EPI_QKV 4
+// The q/k/v product whose epilogue also does what follows it in an attention layer with heads of
+// 128 (crates/backends/backend_common/src/generic_attention/prefill/mod.rs:115-232): per-head RMSNorm
+// of q and k (one weight vector each, or none), rotation of the pairs (j, j + 64) at the token's
+// position, q (bfloat16) into the output, k and v into the paged cache.  A half tile of 128 columns
+// is one head: a lane reads its row's head out of tensor memory and adds the norm's squares, eight lanes then share a head (tg_turn_in).
 struct TgQkv {
   const float* qw;         // norm weights [128], both or neither
   const float* kw;

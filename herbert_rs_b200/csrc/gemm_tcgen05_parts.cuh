@@ -40,11 +40,6 @@ struct TgNorm {
   int act;                 // HB_EPI_ACT: the activation (HB_ACT_SILU, HB_ACT_GELU, HB_ACT_GELU_TANH)
 };
 
-// The q/k/v product whose epilogue also does what follows it in an attention layer with heads of
-// 128 (crates/backends/backend_common/src/generic_attention/prefill/mod.rs:115-232): per-head RMSNorm
-// of q and k (one weight vector each, or none), rotation of the pairs (j, j + 64) at the token's
-// position, q (bfloat16) into the output, k and v into the paged cache.  A half tile of 128 columns
-// is one head, so an epilogue thread (one row, one half tile) holds a whole head of one token.
 // The epilogue of 32 consecutive output columns (n ..) of row m, whose float results are in r:
 // scale by 1/rms, then store / store as float / add into the residual stream (and begin the next
 // norm: x * w in bfloat16, sum of x^2 into sq) / SwiGLU.  Rows beyond M and columns beyond N are skipped.
@@ -173,7 +168,8 @@ __device__ __forceinline__ void tg_epilogue32(unsigned (&r)[32], int m, int n, i
 // unit that takes a line a cycle was what a tile's epilogue waited for (256 x 256 tiles of the residual epilogue with a norm: 20,000
 // line accesses, 10 us; the products of K = 2,048 have 12 us of tensor work a tile, and after the last tile nothing hides it).
 // Here the warp turns its 32 x 32 block round in shared memory (4 KB of its own, 16-byte pieces swizzled by the row: no bank
-// conflicts either way) and eight lanes then share a row of 128 bytes: an eighth of the line accesses.  Measured on a B200 alone (us, before
+// conflicts either way) and eight lanes then share a row of 128 bytes: an eighth of the line accesses.  A row's sum of squares stays its own
+// lane's, in the order of the columns: eight lanes' shares would save nothing (5,083 x 1,024 x 2,048, cold L2: 53.4 us with them, 53.6 so).  Measured on a B200 alone (us, before
 // -> now): 5,083 x 1,024 x 2,048 residual with a norm 46.0 -> 31.9, stored as float 32.3 -> 27.7, as bfloat16 27.8 -> 26.6; 2,048 x 4,096 x
 // 4,096 residual with a norm 65.3 -> 62.3; 2,673 x 2,048 x 8,192 stored as float 117.0 -> 89.2.
 #define TG_TURN_BYTES 4096      // shared memory per epilogue warp

@@ -30,3 +30,10 @@ def test_every_depth_and_every_edge(M, N, K):
     ops.gemm_skinny(a, w, c, ops.EPI_STORE_F32)
     assert torch.isnan(c[0]).all() and torch.isnan(c[:, N - 1]).all()
     assert M == 1 or ((c[1:, :N - 1].double() - ref[1:, :N - 1]).abs() <= bound[1:, :N - 1]).all()
+
+
+@pytest.mark.parametrize("M", [17, 32, 33, 40, 57])
+@pytest.mark.parametrize("N,K", [(24, 8), (48, 264), (2376, 1032), (4744, 520), (8200, 264)])
+def test_the_edges_of_the_ring_and_of_the_products_without_it(M, N, K):
+    """17 to 32 rows with the ring, 33 to 64 with a batch in registers: one unit a CTA and several."""
+    test_every_depth_and_every_edge(M, N, K)
